@@ -21,9 +21,9 @@
 //
 // Lattice tiles go further: delta_p = i s_row + j s_col, so u . delta_p and W . delta_p are
 // sums of a row and a column term.  The records carry the two terms per pulse (the phase
-// ones split exactly as above), each thread forms them once per pulse at a reference pixel,
-// and its four pixels, m rows apart, step from there: per pixel-pulse only the eps term,
-// the window gather and the rotation remain.
+// ones split exactly as above), each thread forms range and phase once per pulse at the middle
+// of a run of eight rows and steps along the run by their Taylor series: per pixel-pulse
+// only two short polynomials, the window gather and the rotation remain.
 //
 // Range interpolation: for each (tile, pulse) the chunk stages the range bins
 // the tile can touch as Horner coefficients of the reference's four-point
@@ -34,6 +34,8 @@
 // outside the precision envelope, runs through a two-float per-sample fallback instead.
 #include <limits.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -75,11 +77,19 @@ constexpr double kDirectEnvelope = 8.0;
 
 struct Rec {
     float4 a;  // W_hi.x, W_hi.y, W_lo.x, W_lo.y   (lattice: B_row hi, lo, B_col hi, lo)
-    float4 b;  // u.x, u.y, 2R, frac(Q) - 1/2       (lattice: u.s_row, u.s_col, 2R, frac(Q) - 1/2)
+    float4 b;  // u.x, u.y, 2R, frac(Q) - 1/2       (lattice: u.s_row, u.s_col, 2R (forward: R), frac(Q) - 1/2)
     float4 c;  // Phi, window bias bits, window offset bits, window count - 1 bits
-    float4 d;  // u.z, W_hi.z, W_lo.z                (lattice: 2 pi frac(m B_row), m u.s_row or u.x, u.y, u.z)
-    float4 e;  // lattice forward: the pairs (2R, 2R), (frac(Q) - 1/2, frac(Q) - 1/2) of packed-FP32 operands
+               // (lattice forward: Phi', window byte base, 2 pi frac(B_row), 12.5 e4: see lattice_runs)
+    float4 d;  // u.z, W_hi.z, W_lo.z                (lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z)
+    float4 e;  // lattice adjoint: the pairs (2R, 2R), (frac(Q) - 1/2, frac(Q) - 1/2) of packed-FP32 operands;
+               // lattice forward: (-, window bias bits, window offset bits, window count - 1 bits)
 };
+
+// Where the chunk driver keeps a pulse's window placement: c, or e in the lattice forward records.
+template <int MODE>
+__device__ __forceinline__ float4& rec_window(Rec& r) { return MODE == 1 ? r.e : r.c; }
+template <int MODE>
+__device__ __forceinline__ const float4& rec_window(const Rec& r) { return MODE == 1 ? r.e : r.c; }
 
 struct Pix {
     float dx, dy, dz;
@@ -492,15 +502,13 @@ __device__ void setup_lattice(const Job& J, TileShared& S, Pix px[kPX]) {
     }
 }
 
-// Lattice tile set-up for the separable pulse loop: the tile centre, bounds and quantum as
-// setup_lattice, the steps as two-float, and per pixel only |delta|^2 (FP32).  Thread t holds
-// pixels (row (t >> lc) + k m, column t & (cols - 1)), k = 0..3, m = kThreads >> lc.
-__device__ void setup_lattice_sep(const Job& J, TileShared& S, float d2[kPX]) {
+// Lattice tile set-up for the separable pulse loops: the tile centre, bounds and quantum as
+// setup_lattice, and the steps as two-float.
+__device__ void setup_lattice_tile(const Job& J, TileShared& S) {
     const sarbp_lattice& L = J.lat;
-    const int tid = threadIdx.x;
     const int cols_t = 1 << J.lc, rows_t = kSplitTilePixels >> J.lc;
     const int hr = rows_t >> 1, hc = cols_t >> 1;
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         const double i0 = (double)(J.tile_r + hr), j0 = (double)(J.tile_u + hc);
         S.cx = L.origin[0] + i0 * L.step_row[0] + j0 * L.step_col[0];
         S.cy = L.origin[1] + i0 * L.step_row[1] + j0 * L.step_col[1];
@@ -518,6 +526,15 @@ __device__ void setup_lattice_sep(const Job& J, TileShared& S, float d2[kPX]) {
         S.row_step = kThreads >> J.lc;
     }
     __syncthreads();
+}
+
+// setup_lattice_tile plus, per pixel, |delta|^2 (FP32).  Thread t holds pixels (row (t >> lc) + k m,
+// column t & (cols - 1)), k = 0..3, m = kThreads >> lc (the adjoint's assignment).
+__device__ void setup_lattice_sep(const Job& J, TileShared& S, float d2[kPX]) {
+    setup_lattice_tile(J, S);
+    const int tid = threadIdx.x;
+    const int cols_t = 1 << J.lc, rows_t = kSplitTilePixels >> J.lc;
+    const int hr = rows_t >> 1, hc = cols_t >> 1;
     const float dj = (float)((tid & (cols_t - 1)) - hc);
 #pragma unroll
     for (int k = 0; k < kPX; ++k) {
@@ -776,11 +793,12 @@ struct SlowRec {
     float4 b;  // w.z hi, w.z lo, phase / 2pi reduced to [-1/2, 1/2], weight
 };
 
-// Sum over pulses [c0, c0 + n) of one pixel's contributions in two-float geometry.  Out of
+// Sum over pulses c0 + first, c0 + first + step, ... below c0 + n of one pixel's contributions in two-float geometry.  Out of
 // line (and the pixel by value) so that the rarely taken fallback does not add registers
 // to the kernels' fast path.
-__device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int n, int c0, float dxh,
-                                          float dxl, float dyh, float dyl, float dzh, float dzl, float psi);
+__device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int first, int n, int step,
+                                          int c0, float dxh, float dxl, float dyh, float dyl, float dzh, float dzl,
+                                          float psi);
 
 // Dynamic shared memory of the chunk kernels: [records | windows]; the two-float records of
 // a chunk that stages no window live at the start of the window space.
@@ -915,20 +933,38 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         r.a.y = (Br.h - r.a.x) + Br.l;
         r.a.z = rintf(Bc.h * iq) * q;
         r.a.w = (Bc.h - r.a.z) + Bc.l;
-        // Phase and range steps between a thread's successive pixels (m = kThreads >> lc rows).
-        const float m = (float)S.row_step;
+        // Phase and range steps between a thread's successive pixels: one row (forward), or
+        // m = kThreads >> lc rows (adjoint).
+        const float m = MODE == 1 ? 1.0f : (float)S.row_step;
         const float mh = m * Br.h;  // exact: m is a power of two
-        float sp = (mh - rintf(mh)) + m * Br.l;
-        sp -= rintf(sp);
+        float turns = rintf(mh), sp = (mh - turns) + m * Br.l;
+        const float more = rintf(sp);
+        sp -= more;
+        turns += more;
         const float Ar = fmaf(uxf, S.sth[0], fmaf(uyf, S.sth[1], uzf * S.sth[2]));
         const float Ac = fmaf(uxf, S.sth[3], fmaf(uyf, S.sth[4], uzf * S.sth[5]));
-        r.b = make_float4(Ar, Ac, 2.0f * Rf, Fm);
-        // The phase step in radians; the range step (forward) or u (adjoint).
-        // The forward holds its per-pulse operands as float2 pairs: (phase step, phase step),
-        // (-range step, -range step) in d and (2R, 2R), (Fm, Fm) in e.
-        const float spr = sp * kTwoPiF, nstep = -(m * Ar);
-        r.d = MODE == 1 ? make_float4(spr, spr, nstep, nstep) : make_float4(spr, uxf, uyf, uzf);
-        r.e = make_float4(2.0f * Rf, 2.0f * Rf, Fm, Fm);
+        const float spr = sp * kTwoPiF;  // the phase step in radians
+        if (MODE == 1) {
+            r.b = make_float4(Ar, Ac, Rf, Fm);
+            // Fourth-order range term of a run of rows, e4 k^4 with k^4 ~ 12.5 k^2 - 21.0625 (lattice_runs).
+            const float s2 = S.sth[0] * S.sth[0] + S.sth[1] * S.sth[1] + S.sth[2] * S.sth[2];
+            const float iRf = 1.0f / Rf;
+            const float e4 = 0.125f * (s2 - Ar * Ar) * (5.0f * Ar * Ar - s2) * iRf * iRf * iRf;
+            r.c = make_float4(fmaf(-21.0625f * P.Kf, e4, t1), 0.0f, 0.0f, 12.5f * e4);
+            // The phase step reduced modulo half a turn, which keeps the angles along a run small: the step is
+            // spT + N / 2 with |spT| <= 1/4, and pixel k = 2 g - 3.5 + c adds k N / 2 = (g - 2) N + (2 c + 1) N / 4
+            // turns: N / 4 for the even pixels of the run (c = 0) and half of N more for the odd ones.
+            const float n2 = rintf(2.0f * sp);
+            const float even = 0.25f * (n2 + 2.0f * turns);
+            r.c.z = (sp - 0.5f * n2) * kTwoPiF;
+            r.c.x += even - rintf(even);
+            const float odd = 0.5f * n2;
+            r.d = make_float4(odd - rintf(odd), 0.0f, 0.0f, 0.0f);
+        } else {
+            r.b = make_float4(Ar, Ac, 2.0f * Rf, Fm);
+            r.d = make_float4(spr, uxf, uyf, uzf);
+            r.e = make_float4(2.0f * Rf, 2.0f * Rf, Fm, Fm);
+        }
     } else {
         const float sw = (float)P.scale_w, isw = (float)P.inv_scale_w;  // powers of two: exact
         r.a.x = rintf(Wx.h * isw) * sw;
@@ -942,17 +978,20 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         r.d.w = 0.0f;
         r.e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    r.c.x = t1;
-    r.c.y = __int_as_float(kMagicBits + bo);
+    if (MODE != 1) r.c.x = t1;
+    float4& rw = rec_window<MODE>(r);
+    rw.y = __int_as_float(kMagicBits + bo);
     const int count = ok ? (int)(hi - lo) + 1 : P.cap + 1;
-    r.c.z = 0.0f;
-    r.c.w = __int_as_float(count - 1);
+    rw.z = 0.0f;
+    rw.w = __int_as_float(count - 1);
+    if (MODE == 1) rw.x = 0.0f;
     rec[lane] = r;
     return count;
 }
 
-__device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int n, int c0, float dxh,
-                                          float dxl, float dyh, float dyl, float dzh, float dzl, float psi) {
+__device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int first, int n, int step,
+                                          int c0, float dxh, float dxl, float dyh, float dyl, float dzh, float dzl,
+                                          float psi) {
     Pix q;
     q.dxh = dxh;
     q.dxl = dxl;
@@ -961,7 +1000,7 @@ __device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* s
     q.dzh = dzh;
     q.dzl = dzl;
     float ar = 0.0f, ai = 0.0f;
-    for (int j = 0; j < n; ++j) {
+    for (int j = first; j < n; j += step) {
         const SlowRec sr = srec[j];
         SlowSample o;
         if (!slow_sample<false>(P, sr, P.in.data + (size_t)(c0 + j) * P.in.samples, q, psi, o)) continue;
@@ -1019,6 +1058,7 @@ __device__ __forceinline__ bool bulk_wait(unsigned bar, unsigned phase) {
 // on 16-byte boundaries of the data array, so the copied range is widened to even elements.
 // Returns false (the same in every thread) if the copies did not arrive within the bounded wait;
 // the caller then stops staging and waits once more before leaving.
+template <int MODE>
 __device__ __forceinline__ bool bulk_stage_windows(const SplitParams& P, TileShared& S, const Rec* rec, float4* win,
                                                    float2* raw, unsigned long long& mbar, unsigned phase, int c0,
                                                    int nfit, bool weighted) {
@@ -1037,7 +1077,7 @@ __device__ __forceinline__ bool bulk_stage_windows(const SplitParams& P, TileSha
             if (nl < nfit) {
                 const long long row0 = (long long)(c0 + nl) * in.samples;
                 const long long b0 = S.base[nl];
-                const int cnt = __float_as_int(rec[nl].c.w) + 1;
+                const int cnt = __float_as_int(rec_window<MODE>(rec[nl]).w) + 1;
                 // [g0, g1) within the row; rows start on even elements (samples is even), so
                 // widening to even bounds stays inside the row.
                 const long long g0 = min(max(b0 - 1, 0ll), (long long)in.samples);
@@ -1088,8 +1128,8 @@ __device__ __forceinline__ bool bulk_stage_windows(const SplitParams& P, TileSha
         return false;
     }
     for (int nl = warp; nl < nfit; nl += kThreads / 32) {
-        const int woff = __float_as_int(rec[nl].c.z);
-        const int cnt = __float_as_int(rec[nl].c.w) + 1;
+        const int woff = __float_as_int(rec_window<MODE>(rec[nl]).z);
+        const int cnt = __float_as_int(rec_window<MODE>(rec[nl]).w) + 1;
         const long long b0 = S.base[nl];
         const float a = weighted ? S.wt[nl] : 1.0f;
         const float2* r = raw + S.roff[nl] + ((long long)(c0 + nl) * in.samples - S.raw0[nl]);  // row-relative
@@ -1180,7 +1220,14 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
             if (warp == 1) inc += S.wsum;
             // Counts are >= 1, so the pulses that fit form a prefix of the chunk.
             const unsigned fits = __ballot_sync(0xffffffffu, idx < want && inc <= P.cap);
-            if (idx < want) rec[idx].c.z = __int_as_float(inc - count);
+            if (idx < want) {
+                float4& rw = rec_window<Body::kRecMode>(rec[idx]);
+                rw.z = __int_as_float(inc - count);
+                // Byte offset in the windows of the entry that index bits 0 would address: bits * 32 plus
+                // this wraps to the entry's own offset.
+                if (Body::kRecMode == 1)
+                    rec[idx].c.y = __int_as_float((int)(32u * ((unsigned)(inc - count) - (unsigned)__float_as_int(rw.y))));
+            }
             if (lane == 0) S.nfit_w[warp] = __popc(fits);
         }
         __syncthreads();
@@ -1188,7 +1235,7 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
         if (nfit > 0) {
 #if SARBP_BULK_WINDOWS
             if (bulk) {
-                if (!bulk_stage_windows(P, S, rec, win, raw, mbar, phase, c0, nfit, weighted)) {
+                if (!bulk_stage_windows<Body::kRecMode>(P, S, rec, win, raw, mbar, phase, c0, nfit, weighted)) {
                     // The copies did not arrive: the tile's image is invalid (g_wait_timeouts counts it).
                     // Wait once more, bounded, for the copies still in flight, then leave.
                     bulk_wait((unsigned)__cvta_generic_to_shared(&mbar), phase);
@@ -1198,8 +1245,9 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
             } else
 #endif
             for (int nl = warp; nl < nfit; nl += kThreads / 32) {
-                const int off = __float_as_int(rec[nl].c.z);
-                const int cnt = __float_as_int(rec[nl].c.w) + 1;
+                const float4& rw = rec_window<Body::kRecMode>(rec[nl]);
+                const int off = __float_as_int(rw.z);
+                const int cnt = __float_as_int(rw.w) + 1;
                 const long long b0 = S.base[nl];
                 const float a = weighted ? S.wt[nl] : 1.0f;
                 const float2* row = in.data + (size_t)(c0 + nl) * in.samples;
@@ -1227,7 +1275,8 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
             if (warp < 2) {
                 const int idx = 32 * warp + lane;
                 const unsigned misses =
-                    __ballot_sync(0xffffffffu, idx < want && __float_as_int(rec[idx].c.w) + 1 > P.cap);
+                    __ballot_sync(0xffffffffu,
+                                  idx < want && __float_as_int(rec_window<Body::kRecMode>(rec[idx]).w) + 1 > P.cap);
                 if (lane == 0) S.miss_w[warp] = misses;
             }
             __syncthreads();
@@ -1265,7 +1314,7 @@ struct ForwardBody {
 #pragma unroll
         for (int k = 0; k < kPX; ++k) {
             const Pix& q = px[k];
-            const float2 v = slow_pixel(P, srec, nslow, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
+            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
                                         DEMOD ? q.psi : 0.0f);
             px[k].ar += v.x;
             px[k].ai += v.y;
@@ -1279,70 +1328,85 @@ __device__ void pulse_loop(const SplitParams& P, const Job& J, TileShared& S, ch
     chunk_loop(P, J, S, smem, true, body);
 }
 
-// ---- lattice tiles: separable pulse loop ------------------------------------------------
+// ---- lattice tiles: runs of eight rows ---------------------------------------------------
 //
 // On a lattice the pixel offset is delta = i s_row + j s_col, so u . delta and W . delta
-// split into row and column terms.  Per (thread, pulse) the record gives the terms at the
-// thread's reference pixel (row (t >> lc) + 2m, its column): L0 = u . delta, and the phase
-// r0 = frac(Phi + W . delta) from the exact hi products; its other pixels are kc = -2..1
-// steps of m rows away, L = L0 + kc (m u . s_row) and phase r0 + kc frac(m W . s_row).
-// Per pixel-pulse this leaves the eps term, the window gather and the rotation.
+// split into row and column terms.  A thread holds a run of eight pixels, rows i0 + k of one
+// column, k = -3.5 .. 3.5 about the run's middle.  Per pulse it forms the range D and the
+// reduced phase at the middle from the record's terms, with the exact hi products, and then
+// steps along the run with the Taylor series of d(k) = |V + k s_row| (V: antenna to middle):
+//   d(k) = D + a k + e2 k^2 + e3 k^3 + e4 k^4,   a = V . s_row / D,
+//   e2 = (s^2 - a^2) / 2D,  e3 = -a e2 / D,  e4 = (s^2 - a^2)(5 a^2 - s^2) / 8 D^3.
+// a = u . s_row + e1 with e1 = (delta . s_row - (D - R) u . s_row) / D small, so the large
+// linear phase K k u . s_row stays in the record's exactly reduced step and only K (e1 k +
+// e2 k^2 + e3 k^3) is FP32.  e4 is a per-record constant (it varies by 1% over a tile and is
+// below 1e-10 m at a kilometre); over the run's four |k| it is folded into the constant and
+// the e2 term (k^4 ~ 12.5 k^2 - 21.0625 within 18).  The envelope bounds the rest: K rho^2 <= 8 R
+// leaves a residual below 0.004 / (K R) rad.
+//
+// Per pixel-pulse that leaves five packed operations per pixel pair for the range and the
+// phase, the window gather, the cubic and the rotation; the run's own set-up (about 60
+// instructions) is shared by eight pixels.
+//
+// What bounds the loop: the register file feeds two operands a cycle to the FMA pipe (a fused
+// multiply-add of three registers takes 1.5 cycles, a packed one 3), so issue sits at 71% with the
+// FMA pipe, the shared-memory pipe and issue all at 60-70%, and every instruction removed shows in
+// the time.  4096 pulses onto 2048 x 2048: 17.2 ms (998 Gpixel-pulses/s; 29.4 instructions per
+// pixel-pulse), 19.6 ms (876; 31.3) with four pixels per thread and the root-free range chain of the
+// adjoint per pixel.  Measured and not kept: runs of 16 (24 warps per SM instead of 32: 16.7 ms, but a larger
+// error on small scenes), even and odd parts of the polynomials with constant multipliers (17.2), scalar
+// cubic (17.5), staging two bins per lane (17.15) and three blocks per SM (17.7).
+constexpr int kRun = 8;                               // pixels per run
+constexpr int kRunThreads = kSplitTilePixels / kRun;  // threads per pulse group
 
-// The forward's per-pixel geometry runs on packed FP32 (f32x2): pixels k = 2h and 2h + 1 of
-// a thread form one float2 lane pair through the range, fraction, index and angle steps, so
-// one instruction issues both pixels' operation.  Each half rounds exactly like the scalar
-// operation, and the chain is carried with the sign of L, q2, e0 and eps flipped (negation
-// is exact, so every value equals the scalar formulation's bit for bit):
-//   -L = kc (-m u.s_row) + (-L0),  -q2 = (-L)^2 - d2,  2L + 2R = -2 (-L) + 2R,
-//   -e0 = -q2 B,  -eps = (-e0)^2 B + (-e0),  qp = ((-L) + (-eps)) (-1/dr) + Fm,
-//   s = qp - (tq - M) = (tq - M) (-1) + qp,  ang = (-kr) (-eps) + (kc sp + r0).
-// The complex cubic evaluates (re, im) as one pair; the accumulation stays scalar.
-__device__ __forceinline__ void lattice_chunk(const SplitParams& P, const Rec* __restrict__ rec,
-                                              const float4* __restrict__ win, int chn, int lc, const float d2[kPX],
-                                              float ar[kPX], float ai[kPX]) {
-    static_assert(kPX == 4, "two pixel pairs per thread");
+// Forward on lattice tiles.  The block's two halves take alternate pulses of the tile (by the
+// parity of the pulse's distance from the range's first, so that the image does not depend on
+// the chunks) and their images are added once at the end.
+__device__ __forceinline__ void lattice_runs(const SplitParams& P, const Rec* __restrict__ rec,
+                                             const char* __restrict__ win, int first, int chn, float di, float dj,
+                                             float d2, float ds, float s2, float ar[kRun], float ai[kRun]) {
     const float inv_dr = P.inv_drf, kr = P.Kf * kTwoPiF;
-    const int m = kThreads >> lc, hr = (kSplitTilePixels >> lc) >> 1, cols_t = 1 << lc;
-    const int tid = threadIdx.x;
-    const float di = (float)((tid >> lc) + 2 * m - hr);
-    const float dj = (float)((tid & (cols_t - 1)) - (cols_t >> 1));
-    const float2 nd2[2] = {make_float2(-d2[0], -d2[1]), make_float2(-d2[2], -d2[3])};
-    const float2 kcs[2] = {make_float2(-2.0f, -1.0f), make_float2(0.0f, 1.0f)};
-    const float2 ninv = pair(-inv_dr), nkr = pair(-kr), magic = pair(kMagic), nmagic = pair(-kMagic);
-    const float2 mone = pair(-1.0f), mtwo = pair(-2.0f);
+    const float2 magic = pair(kMagic), nmagic = pair(-kMagic), mone = pair(-1.0f);
 #pragma unroll 1
-    for (int nl = 0; nl < chn; ++nl) {
-        const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c, rd = rec[nl].d, re = rec[nl].e;
-        const int bias = __float_as_int(rc.y);
-        const unsigned last = (unsigned)__float_as_int(rc.w);
-        const float4* wrow = win + 2 * __float_as_int(rc.z);
-        const float nL0 = fmaf(-dj, rb.y, -di * rb.x);  // -L0, exactly
-        const float t = fmaf(dj, ra.z, di * ra.x);       // exact
-        const float r0 = ((t - round_magic(t)) + fmaf(dj, ra.w, fmaf(di, ra.y, rc.x))) * kTwoPiF;  // radians
-        const float2 sp = make_float2(rd.x, rd.y), nstep = make_float2(rd.z, rd.w);
-        const float2 twoR = make_float2(re.x, re.y), fm = make_float2(re.z, re.w);
-        const float2 nL02 = pair(nL0), r02 = pair(r0);
+    for (int nl = first; nl < chn; nl += 2) {
+        const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c;
+        const unsigned wbase = (unsigned)__float_as_int(rc.y);
+        const float L = fmaf(dj, rb.y, di * rb.x);
+        const float t = fmaf(dj, ra.z, di * ra.x);  // exact
+        const float ph = (t - round_magic(t)) + fmaf(dj, ra.w, fmaf(di, ra.y, rc.x));  // turns
+        const float q2 = fmaf(-L, L, d2);
+        const float h = rb.z + L;
+        const float B = rcp_approx(h + h);
+        const float e0 = q2 * B;
+        const float eps = fmaf(-e0 * e0, B, e0);
+        const float iD = rcp_approx(h + eps);
+        const float Le = L + eps;
+        const float e1 = fmaf(-Le, rb.x, ds) * iD;
+        const float a = rb.x + e1;
+        const float e2 = fmaf(fmaf(-a, a, s2), 0.5f * iD, rc.w);
+        const float e3 = -a * e2 * iD;
+        float P0 = fmaf(P.Kf, eps, ph);
+        P0 -= round_magic(P0);
+        const float2 p0 = __fmul2_rn(make_float2(P0, P0 + rec[nl].d.x), pair(kTwoPiF));
+        const float2 p1 = pair(fmaf(kr, e1, rc.z));
+        const float2 p2 = pair(kr * e2), p3 = pair(kr * e3);
+        const float2 q0 = pair(fmaf(Le, inv_dr, rb.w)), q1 = pair(a * inv_dr), q2k = pair(e2 * inv_dr);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float2 nL = __ffma2_rn(kcs[h], nstep, nL02);
-            const float2 nq2 = __ffma2_rn(nL, nL, nd2[h]);
-            const float2 den = __ffma2_rn(mtwo, nL, twoR);
-            const float2 B = make_float2(rcp_approx(den.x), rcp_approx(den.y));
-            const float2 ne0 = __fmul2_rn(nq2, B);
-            const float2 neps = __ffma2_rn(__fmul2_rn(ne0, ne0), B, ne0);
-            const float2 qp = __ffma2_rn(__fadd2_rn(nL, neps), ninv, fm);
+        for (int g = 0; g < kRun / 2; ++g) {
+            const float2 kk = make_float2(2.0f * g - 3.5f, 2.0f * g - 2.5f);
+            const float2 ang = __ffma2_rn(__ffma2_rn(__ffma2_rn(p3, kk, p2), kk, p1), kk, p0);
+            const float2 qp = __ffma2_rn(__ffma2_rn(q2k, kk, q1), kk, q0);
             const float2 tq = __fadd2_rn(qp, magic);
             const float2 s = __ffma2_rn(__fadd2_rn(tq, nmagic), mone, qp);
-            // |r0| <= 1/2 + small, |kc frac| <= 1 and K eps <= envelope / 2 turns: the angle
-            // stays within +-40 rad, which the hardware sin/cos reduce themselves.
-            const float2 ang = __ffma2_rn(nkr, neps, __ffma2_rn(kcs[h], sp, r02));
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const int k = 2 * h + c;
-                const float tqc = c ? tq.y : tq.x, sc = c ? s.y : s.x;
-                const unsigned j = min((unsigned)(__float_as_int(tqc) - bias), last);
-                const float4 c01 = wrow[2 * j], c23 = wrow[2 * j + 1];
-                const float2 ss = pair(sc);
+                const int k = 2 * g + c;
+                // The record's window holds every bin a pixel of the tile can round to, with half a bin to
+                // spare, so the index needs no clamp.
+                const float4* w = reinterpret_cast<const float4*>(
+                    win + (32u * (unsigned)__float_as_int(c ? tq.y : tq.x) + wbase));
+                const float4 c01 = w[0], c23 = w[1];
+                const float2 ss = pair(c ? s.y : s.x);
                 const float2 v = __ffma2_rn(
                     __ffma2_rn(__ffma2_rn(make_float2(c23.z, c23.w), ss, make_float2(c23.x, c23.y)), ss,
                                make_float2(c01.z, c01.w)),
@@ -1358,32 +1422,42 @@ __device__ __forceinline__ void lattice_chunk(const SplitParams& P, const Rec* _
     }
 }
 
+// Pulses the fast path cannot stage, every second one from `first`, on the run's pixels: offsets in
+// two-float from FP64 (rare, and out of line so that it costs the fast path no registers).
+__device__ __noinline__ void lattice_run_slow(const SplitParams& P, const TileShared& S, const sarbp_lattice& L, float di,
+                                              float dj, int first, int nslow, int c0, const SlowRec* srec,
+                                              float2* more) {
+#pragma unroll 1
+    for (int k = 0; k < kRun; ++k) {
+        const double i = (double)(di - 3.5f) + (double)k, j = (double)dj;
+        Pix q;
+        pixel_from_offsets(S, i * L.step_row[0] + j * L.step_col[0], i * L.step_row[1] + j * L.step_col[1],
+                           i * L.step_row[2] + j * L.step_col[2], q);
+        more[k] = slow_pixel(P, srec, first, nslow, 2, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, 0.0f);
+    }
+}
+
 struct LatticeBody {
     static constexpr int kRecMode = 1;
     static constexpr bool kShflWindows = false;
     const SplitParams& P;
     const TileShared& S;
     const Job& J;
-    const float* d2;
+    float di, dj, d2, ds, s2;  // the run's middle: offsets (rows, columns), |delta|^2, delta . s_row; |s_row|^2
     float* ar;
     float* ai;
-    __device__ void fast(const Rec* rec, const float4* win, int nfit, int) {
-        lattice_chunk(P, rec, win, nfit, J.lc, d2, ar, ai);
+    __device__ int group() const { return threadIdx.x / kRunThreads; }
+    __device__ void fast(const Rec* rec, const float4* win, int nfit, int c0) {
+        lattice_runs(P, rec, reinterpret_cast<const char*>(win), (c0 - J.p0 + group()) & 1, nfit, di, dj, d2, ds, s2, ar,
+                     ai);
     }
-    // Pulses the fast path cannot stage: the pixel offsets in two-float from FP64 (rare).
     __device__ void slow(int c0, int nslow, const SlowRec* srec) {
-        const sarbp_lattice& L = J.lat;
-        const int tid = threadIdx.x, cols_t = 1 << J.lc, hr = (kSplitTilePixels >> J.lc) >> 1;
-        const double dj = (double)((tid & (cols_t - 1)) - (cols_t >> 1));
-#pragma unroll 1
-        for (int k = 0; k < kPX; ++k) {
-            const double di = (double)(((tid + kThreads * k) >> J.lc) - hr);
-            Pix q;
-            pixel_from_offsets(S, di * L.step_row[0] + dj * L.step_col[0], di * L.step_row[1] + dj * L.step_col[1],
-                               di * L.step_row[2] + dj * L.step_col[2], q);
-            const float2 v = slow_pixel(P, srec, nslow, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, 0.0f);
-            ar[k] += v.x;
-            ai[k] += v.y;
+        float2 more[kRun];
+        lattice_run_slow(P, S, J.lat, di, dj, (c0 - J.p0 + group()) & 1, nslow, c0, srec, more);
+#pragma unroll
+        for (int k = 0; k < kRun; ++k) {
+            ar[k] += more[k].x;
+            ai[k] += more[k].y;
         }
     }
 };
@@ -1755,18 +1829,39 @@ __device__ __forceinline__ void lattice_tile(const SplitParams& P, const sarbp_l
     J.tile_u = tile_u;
     J.p0 = p0;
     J.p1 = p1;
-    float d2[kPX], ar[kPX], ai[kPX];
-    setup_lattice_sep(J, S, d2);
+    setup_lattice_tile(J, S);
+    const int cols_t = 1 << lc, hr = (kSplitTilePixels >> lc) >> 1;
+    const int slot = threadIdx.x & (kRunThreads - 1), col = slot & (cols_t - 1), row0 = kRun * (slot >> lc);
+    const float di = (float)(row0 - hr) + 3.5f, dj = (float)(col - (cols_t >> 1));
+    float d2 = 0.0f, ds = 0.0f, s2 = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) ar[k] = ai[k] = 0.0f;
-    LatticeBody body{P, S, J, d2, ar, ai};
+    for (int c = 0; c < 3; ++c) {
+        const float x = fmaf(di, S.sth[c], dj * S.sth[3 + c]);
+        d2 = fmaf(x, x, d2);
+        ds = fmaf(x, S.sth[c], ds);
+        s2 = fmaf(S.sth[c], S.sth[c], s2);
+    }
+    float ar[kRun], ai[kRun];
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) ar[k] = ai[k] = 0.0f;
+    LatticeBody body{P, S, J, di, dj, d2, ds, s2, ar, ai};
     chunk_loop(P, J, S, smem, true, body);
-    const int cols_t = 1 << lc;
+    // Add the two halves' images: each half passes on four rows of every run and finishes the other four.
+    __syncthreads();  // the last chunk's windows are consumed
+    const int half = body.group();
+    float2* ex = reinterpret_cast<float2*>(smem + window_offset());
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) {
-        const int p = threadIdx.x + kThreads * k;
-        const int wr = tile_r + (p >> lc), wu = tile_u + (p & (cols_t - 1));
-        if (wr < lat.rows && wu < lat.cols) out[(long long)wr * lat.cols + wu] = make_float2(ar[k], ai[k]);
+    for (int k = 0; k < kRun / 2; ++k)
+        ex[(kRun / 2 * half + k) * kRunThreads + slot] =
+            half ? make_float2(ar[k], ai[k]) : make_float2(ar[k + kRun / 2], ai[k + kRun / 2]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRun / 2; ++k) {
+        const float2 o = ex[(kRun / 2 * (1 - half) + k) * kRunThreads + slot];
+        const float2 v = half ? make_float2(o.x + ar[k + kRun / 2], o.y + ai[k + kRun / 2])
+                              : make_float2(ar[k] + o.x, ai[k] + o.y);
+        const int wr = tile_r + row0 + kRun / 2 * half + k, wu = tile_u + col;
+        if (wr < lat.rows && wu < lat.cols) out[(long long)wr * lat.cols + wu] = v;
     }
 }
 
@@ -2983,6 +3078,12 @@ int capacity_for(int chunk, int window_bins, int budget_bytes = kWindowBudget) {
     return (int)(cap > budget ? budget : cap);
 }
 
+// Lattice tiles: at least room for the block halves' exchange of their images (half a tile's pixels each).
+int lattice_capacity(int chunk, int window_bins) {
+    return std::max(capacity_for(chunk, window_bins, kLatticeWindowBudget),
+                    kSplitTilePixels * (int)sizeof(float2) / 32);
+}
+
 // Leaf window entries: the windows share the CTA's shared memory with the chunk's pulse and
 // (pulse, column) records, within the same per-CTA total as the direct kernels' windows.
 int leaf_capacity(int chunk, int window_bins) {
@@ -3071,7 +3172,7 @@ int split_lattice_auto_split(const sarbp_lattice& lat, int pulses) {
 
 int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pulse_split, int chunk, int window_bins,
                          float2* out, long long split_stride, cudaStream_t s) {
-    SplitParams P = make_params(in, chunk, capacity_for(chunk, window_bins, kLatticeWindowBudget), pulse_split);
+    SplitParams P = make_params(in, chunk, lattice_capacity(chunk, window_bins), pulse_split);
     P.out = out;
     P.split_stride = split_stride;
     const int lc = 5;
@@ -3405,7 +3506,7 @@ size_t split_batch_scene_bytes() { return sizeof(BatchScene); }
 size_t split_batch_pack_scene(const BatchSceneDesc& d, void* dst) {
     BatchScene b{};
     b.P = make_params(d.in, d.chunk,
-                      d.kind == 0 ? capacity_for(d.chunk, d.window_bins, kLatticeWindowBudget)
+                      d.kind == 0 ? lattice_capacity(d.chunk, d.window_bins)
                                   : leaf_capacity(d.chunk, d.window_bins),
                       1);
     b.P.out = d.out;
