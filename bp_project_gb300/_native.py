@@ -101,6 +101,9 @@ SIGNATURES = {
     "sarbp_batch_execute": ([_P, _P], _I),
     "sarbp_batch_set_trace": ([_P, _P], _I),
     "sarbp_batch_set_concurrent": ([_P, _I], _I),
+    "sarbp_rc_block_points": ([], _I),
+    "sarbp_rc_blocks_fit": ([_I, _I], _I),
+    "sarbp_rc_blocks": ([_P, _I, _I, _I, _P, _P, _P], _I),
     "sarbp_rc_prepare": ([_P, _I, _I, _I, _P, _P], _I),
     "sarbp_decode_iq": ([_P, _I, _I64, _I, _I, _P, _P], _I),
     "sarbp_rc_filter": ([_P, _P, _I, _I, _I, _P, _P], _I),

@@ -471,6 +471,21 @@ int sarbp_rc_crop(const float* corr, int pulses, int length, int offset, int sam
                           reinterpret_cast<float2*>(out), (cudaStream_t)stream);
 }
 
+int sarbp_rc_block_points(void) { return rc_blocks_points(); }
+int sarbp_rc_blocks_fit(int samples, int taps) { return rc_blocks_fit(samples, taps) ? 1 : 0; }
+
+int sarbp_rc_blocks(const float* raw, int pulses, int samples, int taps, const float* response, float* out,
+                    void* stream) {
+    if (!raw || !response || !out) return fail(SARBP_ERR_TYPE, "raw, response and out must be device pointers");
+    if (((uintptr_t)raw & 7) || ((uintptr_t)response & 7) || ((uintptr_t)out & 7))
+        return fail(SARBP_ERR_TYPE, "arrays must be 8-byte aligned");
+    if (pulses < 1 || !rc_blocks_fit(samples, taps))
+        return fail(SARBP_ERR_VALUE, "pulses must be positive and %d samples x %d taps must fit a block", samples, taps);
+    return launch_rc_blocks(reinterpret_cast<const float2*>(raw), pulses, samples, taps,
+                            reinterpret_cast<const float2*>(response), reinterpret_cast<float2*>(out),
+                            (cudaStream_t)stream);
+}
+
 int sarbp_decode_iq(const void* frames, int n, long long frame_size, int iq_offset, int nr, float* out,
                     void* stream) {
     if (!frames || !out) return fail(SARBP_ERR_TYPE, "frames and out must be device pointers");

@@ -246,6 +246,11 @@ int launch_rc_filter(const float2* spec, const float2* response, int pulses, int
                      cudaStream_t s);
 int launch_rc_crop(const float2* corr, int pulses, int length, int offset, int samples, float scale, float2* out,
                    cudaStream_t s);
+// The whole filter without oversampling in one launch; `response`: rc_blocks_points() values.
+int rc_blocks_points();
+bool rc_blocks_fit(int samples, int taps);
+int launch_rc_blocks(const float2* raw, int pulses, int samples, int taps, const float2* response, float2* out,
+                     cudaStream_t s);
 int launch_decode_iq(const unsigned char* frames, int n, long long frame_size, int iq_offset, int nr, float2* out,
                      cudaStream_t s);
 

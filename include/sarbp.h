@@ -266,6 +266,16 @@ int sarbp_rc_filter(const float* spectrum, const float* response, int pulses, in
 int sarbp_rc_crop(const float* corr, int pulses, int length, int offset, int samples, float scale, float* out,
                   void* stream);
 
+/* The same without oversampling (length = nfft), in one launch: the linear correlation by overlap-save
+ * blocks of sarbp_rc_block_points() samples in shared memory.  `response`: the transform of the `taps`
+ * filter values h, zero-padded to sarbp_rc_block_points() points and divided by that number.
+ * sarbp_rc_blocks_fit: 1 if the kernel takes pulses of `samples` samples and this many taps, else 0 (use
+ * the steps above). */
+int sarbp_rc_block_points(void);
+int sarbp_rc_blocks_fit(int samples, int taps);
+int sarbp_rc_blocks(const float* raw, int pulses, int samples, int taps, const float* response, float* out,
+                    void* stream);
+
 /* Raw capture frames -> complex64 pulses (sar_io.Capture.read, sar_io.py:79-81):
  * out [n, nr] = I + jQ from the little-endian int16 pairs that start iq_offset bytes
  * into each of n consecutive frames of frame_size bytes (device memory).  frames,
