@@ -104,10 +104,13 @@ struct PolarDesc {
     // box_u columns (then rounded down to an even column) before the stencil bin of the parent
     // tile's centre pixel and is box_h x box_w elements; box_w == 0: not staged.
     int box_r, box_u, box_h, box_w;
+    double inv_dr, inv_du;  // 1 / dr, 1 / du
 };
 
-// Fills PolarDesc::tf from the FP64 fields (host).
+// Fills PolarDesc::tf and the reciprocals from the FP64 fields (host).
 inline void split_geometry(PolarDesc& d) {
+    d.inv_dr = 1.0 / d.dr;
+    d.inv_du = 1.0 / d.du;
     const double v[9] = {d.ox, d.oy, d.oz, d.r0, d.dr, d.u0, d.du, 1.0 / d.dr, 1.0 / d.du};
     for (int i = 0; i < 9; ++i) {
         const float h = (float)v[i];

@@ -5,6 +5,7 @@
 // points (sample1/sample2 weights, per-child complex64 rounding in merges) and
 // are the "plain FP64-phase" baseline the split-precision kernels are
 // measured against.
+#include <limits.h>
 #include <math.h>
 
 #include "common.cuh"
@@ -88,6 +89,63 @@ __device__ __forceinline__ void sample2(const float2* __restrict__ img, int nr, 
     }
 }
 
+// ---- the mixed policy's FP64 steps ---------------------------------------------------------
+//
+// An FP64 instruction holds a GB300 sub-partition's FP64 unit for 64 cycles whatever the warp does
+// with it, so the mixed policy's kernels are bound by their number.  FP64 carries what needs it,
+// positions, ranges, coordinates and the unreduced phase; where the policy rounds to FP32 anyway (interpolation
+// weights, sine and cosine), only the reduced argument is formed in FP64.  Per pixel and pulse that is 18
+// FP64 operations instead of 58: direct BP of 256 pulses onto
+// the 257 x 257 scene's polar sector takes 0.70 ms instead of 2.10, with the same error against FP64 (2.9e-7), and a
+// polar image at 160,000 terrain points 19 us instead of 35 (0.9e-7 instead of 1.0e-7).
+
+// sqrt(x), x >= 0: an FP32 reciprocal root of the truncated value and two FP64 Newton steps (relative
+// error 2^-22, 2^-44, then the last bit).  The bit moves replace FP64 <-> FP32 conversions, which
+// run at the FP64 rate.  Values outside the FP32 range, and no numbers, take the library's root.
+// yh: 0.5 / sqrt(x) to FP32 precision (0 for 0).
+__device__ __forceinline__ double fast_sqrt(double x, double& yh) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    if ((unsigned)(hi - (897 << 20)) >= (unsigned)(253 << 20)) {
+        const double g = sqrt(x);
+        yh = g > 0.0 ? 0.5 / g : 0.0;
+        return g;
+    }
+    const float xf = __int_as_float(((hi - ((1023 - 127) << 20)) << 3) | ((unsigned)lo >> 29));
+    const int h = __float_as_int(0.5f * rsqrtf(xf));
+    yh = __hiloint2double((h >> 3) + ((1023 - 127) << 20), h << 29);
+    const double g0 = x * (yh + yh);
+    const double g1 = fma(fma(-g0, g0, x), yh, g0);
+    return fma(fma(-g1, g1, x), yh, g1);
+}
+
+// Bins 1 <= floor(q) <= n - 3 (the support of a four-point stencil in n samples): the bin and the
+// fraction less 1/2.  One FP64 addition: at 1.5 2^20 the last mantissa bit is worth 2^-32, so rounding
+// down leaves floor(q) in the high word and the fraction's 32 bits in the low one.
+__device__ __forceinline__ bool fast_bin(double q, int n, int& i, float& s) {
+    const double m = __dadd_rd(q, 1572864.0);
+    i = (__double2hiint(m) & 0x000fffff) - 0x80000;
+    s = (float)(__double2loint(m) ^ INT_MIN) * 2.3283064365386963e-10f;
+    if ((__double2hiint(m) >> 20) == 0x413 && i < 0x7fff0) return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
+    if (!(q >= 1.0 && q < (double)(n - 2))) return false;  // rows of half a million samples and more, or no number
+    i = (int)floor(q);
+    s = (float)(q - ((double)i + 0.5));
+    return true;
+}
+
+// sin and cos (FP32) of an angle in quarter turns: reduced in FP64 to +-1/2 quarter turn.
+__device__ __forceinline__ void quarter_sincos(double y, float* s, float* c) {
+    const double big = 6755399441055744.0;  // 1.5 2^52
+    const double m = y + big;
+    float s0, c0;
+    sincospif(0.5f * (float)(y - (m - big)), &s0, &c0);
+    const int n = __double2loint(m);
+    const float a = n & 1 ? c0 : s0, b = n & 1 ? s0 : c0;
+    *s = n & 2 ? -a : a;
+    *c = (n + 1) & 2 ? -b : b;
+}
+
+constexpr double kQuarters = 0.63661977236758134308;  // quarter turns per radian
+
 // Per-pulse inputs converted to the policy's types and staged in shared memory.
 template <int M>
 struct PulseStage {
@@ -107,6 +165,53 @@ __device__ __forceinline__ void stage_pulses(PulseStage<M>& st, const PulseInput
         st.pos[3 * t + 2] = (G)in.pos[3 * n + 2];
         st.w[t] = (W)in.weight[n];
         st.ph[t] = (G)in.phase[n];
+    }
+}
+
+// accumulate for the mixed policy; FLAT: the point lies at z = 0 and the pulses' z^2 is staged instead of z.
+template <bool FLAT>
+__device__ __forceinline__ void accumulate_mixed(PulseStage<SARBP_MIXED>& st, const PulseInputs& in, int p0, int p1,
+                                                 bool active, double x, double y, double z, double r_demod,
+                                                 float& accr, float& acci) {
+    const double inv = 1.0 / in.data_dr, k4 = in.k * kQuarters;
+    for (int c0 = p0; c0 < p1; c0 += kChunk) {
+        const int count = min(kChunk, p1 - c0);
+        __syncthreads();
+        for (int t = threadIdx.x; t < count; t += blockDim.x) {
+            const int n = c0 + t;
+            const double pz = in.pos[3 * n + 2];
+            st.pos[3 * t] = in.pos[3 * n];
+            st.pos[3 * t + 1] = in.pos[3 * n + 1];
+            st.pos[3 * t + 2] = FLAT ? pz * pz : pz;
+            st.w[t] = (float)in.weight[n];
+            st.ph[t] = in.phase[n] * kQuarters;
+        }
+        __syncthreads();
+        if (!active) continue;
+        for (int t = 0; t < count; ++t) {
+            const double dx = x - st.pos[3 * t], dy = y - st.pos[3 * t + 1];
+            const double dz = FLAT ? 0.0 : z - st.pos[3 * t + 2];
+            const double zz = FLAT ? st.pos[3 * t + 2] : dz * dz;
+            double yh;
+            const double d = fast_sqrt(fma(dx, dx, fma(dy, dy, zz)), yh);
+            float vr = 0.0f, vi = 0.0f, f, sn, cs;
+            int i;
+            if (fast_bin((d - in.range_start) * inv, in.samples, i, f)) {
+                float w[4];
+                lagrange_centred(f, w);
+                const float2* row = in.data + (size_t)(c0 + t) * in.samples + i - 1;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const float2 v = __ldg(row + a);
+                    vr += w[a] * v.x;
+                    vi += w[a] * v.y;
+                }
+            }
+            quarter_sincos(fma(k4, d - r_demod, st.ph[t]), &sn, &cs);
+            const float a = st.w[t];
+            accr += a * (vr * cs - vi * sn);
+            acci += a * (vr * sn + vi * cs);
+        }
     }
 }
 
@@ -173,7 +278,10 @@ __global__ void __launch_bounds__(kThreads) plain_polar_kernel(PulseInputs in, P
     G x, y, r;
     polar_point<G>(g, g.win_r0 + wr, g.win_u0 + wu, x, y, r);
     A accr = A(0), acci = A(0);
-    accumulate<M>(st, in, p0, p1, active, x, y, G(0), r, accr, acci);
+    if constexpr (M == SARBP_MIXED)
+        accumulate_mixed<true>(st, in, p0, p1, active, x, y, 0.0, r, accr, acci);
+    else
+        accumulate<M>(st, in, p0, p1, active, x, y, G(0), r, accr, acci);
     if (active) out[(long long)wr * out_stride + wu] = to_c64(accr, acci);
 }
 
@@ -188,7 +296,10 @@ __global__ void __launch_bounds__(kThreads) plain_points_kernel(PulseInputs in, 
     const int q = active ? p : 0;
     const G x = (G)xyz[3 * q], y = (G)xyz[3 * q + 1], z = (G)xyz[3 * q + 2];
     A accr = A(0), acci = A(0);
-    accumulate<M>(st, in, 0, in.pulses, active, x, y, z, G(0), accr, acci);
+    if constexpr (M == SARBP_MIXED)
+        accumulate_mixed<false>(st, in, 0, in.pulses, active, x, y, z, 0.0, accr, acci);
+    else
+        accumulate<M>(st, in, 0, in.pulses, active, x, y, z, G(0), accr, acci);
     if (active) out[p] = to_c64(accr, acci);
 }
 
@@ -207,7 +318,10 @@ __global__ void __launch_bounds__(kThreads) plain_lattice_kernel(PulseInputs in,
     const G y = (G)(lat.origin[1] + i * lat.step_row[1] + j * lat.step_col[1]);
     const G z = (G)(lat.origin[2] + i * lat.step_row[2] + j * lat.step_col[2]);
     A accr = A(0), acci = A(0);
-    accumulate<M>(st, in, 0, in.pulses, active, x, y, z, G(0), accr, acci);
+    if constexpr (M == SARBP_MIXED)
+        accumulate_mixed<false>(st, in, 0, in.pulses, active, x, y, z, 0.0, accr, acci);
+    else
+        accumulate<M>(st, in, 0, in.pulses, active, x, y, z, G(0), accr, acci);
     if (active) out[p] = to_c64(accr, acci);
 }
 
@@ -231,6 +345,55 @@ __device__ __forceinline__ float2 regrid_pixel(const float2* __restrict__ img, c
     sin_cos((G)k * (rr - r), &sg, &cg);
     const A s = (A)sg, c = (A)cg;
     return to_c64(vr * c - vi * s, vr * s + vi * c);
+}
+
+// A polar image at the ground point (dx, dy) from its origin (mixed policy): the 4x4 stencil, and the
+// point's range rr to the origin; false (and no value) at the origin itself.
+__device__ __forceinline__ bool image_at_mixed(const float2* __restrict__ img, const PolarDesc& src, double dx, double dy,
+                                               double& rr, float& vr, float& vi) {
+    const double g2 = fma(dx, dx, dy * dy);
+    double yh, unused;
+    const double g = fast_sqrt(g2, yh);
+    rr = fast_sqrt(fma(src.oz, src.oz, g2), unused);
+    vr = vi = 0.0f;
+    // uu = dy / g: the reciprocal to 2^-44, then one correction of the quotient.
+    const double y0 = yh + yh, y1 = fma(fma(-g, y0, 1.0), y0, y0);
+    const double u0 = dy * y1, uu = fma(fma(-u0, g, dy), y1, u0);
+    int ir, iu;
+    float tr, tu;
+    if (fast_bin((rr - src.r0) * src.inv_dr, src.nr, ir, tr) && fast_bin((uu - src.u0) * src.inv_du, src.nu, iu, tu)) {
+        float wr[4], wu[4];
+        lagrange_centred(tr, wr);
+        lagrange_centred(tu, wu);
+        const float2* base = img + (size_t)(ir - 1) * src.nu + iu - 1;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            float rr4 = 0.0f, ri4 = 0.0f;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float2 v = __ldg(base + (size_t)a * src.nu + b);
+                rr4 = fmaf(wu[b], v.x, rr4);
+                ri4 = fmaf(wu[b], v.y, ri4);
+            }
+            vr = fmaf(wr[a], rr4, vr);
+            vi = fmaf(wr[a], ri4, vi);
+        }
+    }
+    return g2 != 0.0;
+}
+
+template <>
+__device__ __forceinline__ float2 regrid_pixel<SARBP_MIXED>(const float2* __restrict__ img, const PolarDesc& src,
+                                                            const PolarDesc& dst, double k, int ir, int iu) {
+    const double r = fma((double)ir, dst.dr, dst.r0), u = fma((double)iu, dst.du, dst.u0);
+    double unused, rr;
+    const double ground = fast_sqrt(fmax(0.0, fma(r, r, -dst.oz * dst.oz)), unused);
+    const double x = dst.ox + dst.side * ground * fast_sqrt(fmax(0.0, fma(-u, u, 1.0)), unused);
+    float vr, vi, s, c;
+    if (!image_at_mixed(img, src, x - src.ox, fma(ground, u, dst.oy) - src.oy, rr, vr, vi))
+        return make_float2(0.0f, 0.0f);
+    quarter_sincos(k * kQuarters * (rr - r), &s, &c);
+    return make_float2(vr * c - vi * s, vr * s + vi * c);
 }
 
 template <int M>
@@ -273,7 +436,10 @@ __global__ void __launch_bounds__(kThreads) plain_ffbp_leaf_kernel(PulseInputs i
     G x, y, r;
     polar_point<G>(g, g.win_r0 + wr, g.win_u0 + wu, x, y, r);
     A accr = A(0), acci = A(0);
-    accumulate<M>(st, in, g.a, g.b, active, x, y, G(0), r, accr, acci);
+    if constexpr (M == SARBP_MIXED)
+        accumulate_mixed<true>(st, in, g.a, g.b, active, x, y, 0.0, r, accr, acci);
+    else
+        accumulate<M>(st, in, g.a, g.b, active, x, y, G(0), r, accr, acci);
     if (active) arena[g.out_offset + (long long)wr * g.out_stride + wu] = to_c64(accr, acci);
 }
 
@@ -301,16 +467,11 @@ __global__ void __launch_bounds__(kThreads) evaluate_kernel(const float2* __rest
     const int p = blockIdx.x * kThreads + threadIdx.x;
     if (p >= npts) return;
     // ffbp.py:192-197: the points' z is not used.
-    const double dx = xyz[3 * p] - g.ox, dy = xyz[3 * p + 1] - g.oy;
-    const double gd = sqrt(dx * dx + dy * dy);
-    const double r = sqrt(gd * gd + g.oz * g.oz);
-    const double u = dy / gd;
-    float vr, vi;
-    sample2<SARBP_MIXED>(img, g.nr, g.nu, (r - g.r0) / g.dr, (u - g.u0) / g.du, vr, vi);
-    double sd, cd;
-    sincos(k * r, &sd, &cd);
-    const float s = (float)sd, c = (float)cd;
-    out[p] = make_float2(vr * c - vi * s, vr * s + vi * c);
+    double r;
+    float vr, vi, s, c;
+    const bool off = image_at_mixed(img, g, xyz[3 * p] - g.ox, xyz[3 * p + 1] - g.oy, r, vr, vi);
+    quarter_sincos(k * kQuarters * r, &s, &c);
+    out[p] = off ? make_float2(vr * c - vi * s, vr * s + vi * c) : make_float2(0.0f, 0.0f);
 }
 
 __global__ void __launch_bounds__(kThreads) target_contrib_kernel(PulseInputs in, const double* __restrict__ xyz,
