@@ -345,10 +345,24 @@ int sarbp_direct_polar(const float* data, int pulses, int samples, const double*
     return st;
 }
 
+namespace {
+
+// Split-mode point lists longer than one tile: the spatial order's buffers, then the partial images of
+// the pulse split (the automatic one where the caller asks for one pass).  Points of a list longer than a
+// tile need neither, but both pay: see points_order.cu.
+size_t points_order_space(int npts) { return (points_order_bytes(npts) + 255) / 256 * 256; }
+constexpr int kMaxAutoSplit = 8;
+
+size_t points_parts(int npts, int pulse_split) {
+    return pulse_split > 1 && npts > 0 ? (size_t)pulse_split * (size_t)npts * sizeof(float2) : 0;
+}
+
+}  // namespace
+
 size_t sarbp_backproject_points_workspace(int mode, int npts, int pulse_split) {
-    (void)mode;
-    if (pulse_split <= 1 || npts <= 0) return 0;
-    return (size_t)pulse_split * (size_t)npts * sizeof(float2);
+    if (mode != SARBP_SPLIT || npts <= kPointTile) return points_parts(npts, pulse_split);
+    if (pulse_split <= 1) pulse_split = split_points_auto_split(npts, kMaxAutoSplit);
+    return points_order_space(npts) + points_parts(npts, pulse_split);
 }
 
 int sarbp_backproject_points(const float* data, int pulses, int samples, const double* pos, const double* weight,
@@ -361,18 +375,34 @@ int sarbp_backproject_points(const float* data, int pulses, int samples, const d
     if (npts <= 0) return fail(SARBP_ERR_VALUE, "at least one point is required");
     if (pulse_split < 1 || pulse_split > pulses) return fail(SARBP_ERR_VALUE, "pulse_split must be in [1, pulses]");
     if (mode != SARBP_SPLIT && pulse_split != 1) return fail(SARBP_ERR_VALUE, "pulse_split applies to split mode only");
-    const size_t need = sarbp_backproject_points_workspace(mode, npts, pulse_split);
+    size_t need = points_parts(npts, pulse_split);
     if (need && (!workspace || workspace_bytes < need))
         return fail(SARBP_ERR_WORKSPACE, "backproject_points needs %zu workspace bytes", need);
     cudaStream_t s = (cudaStream_t)stream;
     const PulseInputs in = inputs_of(data, pulses, samples, pos, weight, phase, range_start, data_dr, k);
     float2* dst = reinterpret_cast<float2*>(out);
     if (mode != SARBP_SPLIT) return launch_plain_points(mode, in, xyz, npts, 0, dst, s);
-    float2* parts = pulse_split > 1 ? reinterpret_cast<float2*>(workspace) : dst;
+    // With the workspace that the query asks for, the list is taken in spatial order and one pass over the
+    // pulses becomes the split that fills the GPU; with less (partial images only, or none) the list is
+    // taken as it is, in the split that was asked for.
+    const PointOrder* order = nullptr;
+    const int* index = nullptr;
+    char* ws = static_cast<char*>(workspace);
+    int split = pulse_split;
+    if (npts > kPointTile && workspace && ((uintptr_t)workspace & 255) == 0) {
+        if (pulse_split == 1) split = split_points_auto_split(npts, std::min(pulses, kMaxAutoSplit));
+        if (workspace_bytes >= points_order_space(npts) + points_parts(npts, split)) {
+            if (int st = launch_points_order(xyz, npts, ws, &order, &index, s)) return st;
+            ws += points_order_space(npts);
+        } else {
+            split = pulse_split;
+        }
+    }
+    float2* parts = split > 1 ? reinterpret_cast<float2*>(ws) : dst;
     const int wb = split_window_bins(kPointRadius, data_dr);
     const int ch = split_chunk_for(wb, 64);
-    int st = launch_split_points(in, xyz, npts, pulse_split, ch, wb, parts, npts, s);
-    if (st == SARBP_OK && pulse_split > 1) st = launch_sum_parts(parts, pulse_split, npts, npts, dst, s);
+    int st = launch_split_points(in, xyz, npts, order, index, split, ch, wb, parts, npts, s);
+    if (st == SARBP_OK && split > 1) st = launch_sum_parts(parts, split, npts, npts, dst, s);
     return st;
 }
 

@@ -201,8 +201,23 @@ int launch_split_polar(const PulseInputs& in, const PolarDesc& g, int pulse_spli
                        float2* out, long long out_stride, long long split_stride, cudaStream_t s);
 int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pulse_split, int chunk,
                          int window_bins, float2* out, long long split_stride, cudaStream_t s);
-int launch_split_points(const PulseInputs& in, const double* xyz, int npts, int pulse_split, int chunk,
-                        int window_bins, float2* out, long long split_stride, cudaStream_t s);
+// Points per tile of the points kernel.
+constexpr int kPointTile = 512;
+// Spatial order of a point list (points_order.cu): the bounding box as ordered integers, and whether every
+// tile of the list is narrow as it is (then the index is not written and not used).
+struct PointOrder {
+    unsigned low[2], high[2];  // min x, y and ~max x, y
+    unsigned narrow;
+};
+size_t points_order_bytes(int npts);
+int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder** order, const int** index,
+                        cudaStream_t s);
+// The pulse split that fills the GPU for this many points.
+int split_points_auto_split(int npts, int pulses);
+// order: NULL, or the order in which the kernel takes the points (index: point of each place).
+int launch_split_points(const PulseInputs& in, const double* xyz, int npts, const PointOrder* order, const int* index,
+                        int pulse_split, int chunk, int window_bins, float2* out, long long split_stride,
+                        cudaStream_t s);
 // Adjoint of split-precision lattice BP: per-pulse gradients of a real image loss
 // (grad = dl/dRe I + i dl/dIm I) with respect to position, phase and weight.
 size_t split_adjoint_workspace(const sarbp_lattice& lat, int pulses);

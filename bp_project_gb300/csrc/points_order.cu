@@ -1,0 +1,247 @@
+// Spatial order of a point list for split-precision direct BP.
+//
+// The points kernel forms tiles of 1024 consecutive points; its fast path needs tiles of at most
+// about 20 m radius, while a raster of terrain points puts a tile on a strip of hundreds of metres
+// and every pulse on the two-float fallback.  These kernels order a list by the Hilbert curve of a 256 x 256
+// raster over its bounding square: two stable 8-bit counting passes, so the order (and with it the
+// image) is the same on every run.  Nothing is ordered when no tile is wide: the kernels
+// then return at once, and the points kernel takes the list as it is.
+// 192,384 terrain points in raster order (501 to a row, half a metre apart), 1024 pulses: 2.50 ms as they
+// come, 0.64 ms ordered, of which the ordering is about 0.05; error against FP64 2.8e-7 either way.
+#include "common.cuh"
+
+namespace sarbp {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kKeys = 4096;            // keys per block of a counting pass
+constexpr int kTilePoints = kPointTile;  // points per tile of the points kernel
+constexpr float kWideRadius = 16.0f;   // tiles above this radius (m) are worth ordering
+constexpr int kDigits = 256;
+
+// FP32 as an unsigned of the same order.
+__device__ __forceinline__ unsigned ordered(float v) {
+    const unsigned b = __float_as_uint(v);
+    return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float unordered(unsigned u) {
+    return __uint_as_float(u & 0x80000000u ? u ^ 0x80000000u : ~u);
+}
+
+// Bounds of each tile: the list's bounding box, and whether any tile is wide.  One block per tile.
+__global__ void __launch_bounds__(kThreads) points_extent_kernel(const double* __restrict__ xyz, int npts,
+                                                                 PointOrder* __restrict__ h) {
+    const float inf = __int_as_float(0x7f800000);
+    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+    const int end = min(npts, (blockIdx.x + 1) * kTilePoints);
+    for (int i = blockIdx.x * kTilePoints + threadIdx.x; i < end; i += kThreads)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float v = (float)xyz[3LL * i + c];
+            lo[c] = fminf(lo[c], v);
+            hi[c] = fmaxf(hi[c], v);
+        }
+    __shared__ float part[kThreads / 32][6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+            hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+        }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            part[threadIdx.x >> 5][c] = lo[c];
+            part[threadIdx.x >> 5][3 + c] = hi[c];
+        }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < kThreads / 32; ++w)
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = fminf(lo[c], part[w][c]);
+            hi[c] = fmaxf(hi[c], part[w][3 + c]);
+        }
+    float d2 = 0.0f;
+    for (int c = 0; c < 3; ++c) d2 += (hi[c] - lo[c]) * (hi[c] - lo[c]);
+    for (int c = 0; c < 2; ++c) {
+        atomicMin(&h->low[c], ordered(lo[c]));
+        atomicMin(&h->high[c], ~ordered(hi[c]));
+    }
+    atomicMin(&h->narrow, d2 <= 4.0f * kWideRadius * kWideRadius ? 1u : 0u);
+}
+
+// Place of cell (x, y) along the Hilbert curve of a 256 x 256 raster: level by level from the top, the
+// quadrant's two bits, then the quadrant's own orientation (swap, and mirror in the fourth).  Its steps
+// go to neighbouring cells, so any stretch of it is compact (the Z-curve's jumps left a third of the tiles
+// wide).
+__device__ __forceinline__ unsigned hilbert(unsigned x, unsigned y) {
+    unsigned key = 0;
+#pragma unroll
+    for (unsigned bit = 128; bit; bit >>= 1) {
+        const unsigned rx = (x & bit) ? 1u : 0u, ry = (y & bit) ? 1u : 0u;
+        key = 4 * key + ((3u * rx) ^ ry);
+        if (!ry) {
+            if (rx) {
+                x = 255u - x;
+                y = 255u - y;
+            }
+            const unsigned t = x;
+            x = y;
+            y = t;
+        }
+    }
+    return key;
+}
+
+// Counts of each digit in each block's keys, digit-major: counts[digit * blocks + block].  FIRST: the keys
+// are made from the points.
+template <bool FIRST>
+__global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __restrict__ xyz, int npts,
+                                                                const PointOrder* __restrict__ h,
+                                                                unsigned short* __restrict__ keys,
+                                                                int* __restrict__ counts) {
+    if (h->narrow) return;
+    __shared__ int hist[kDigits];
+    hist[threadIdx.x] = 0;
+    __syncthreads();
+    const float x0 = unordered(h->low[0]), y0 = unordered(h->low[1]);
+    const float span = fmaxf(unordered(~h->high[0]) - x0, unordered(~h->high[1]) - y0);
+    const float scale = 255.99f / fmaxf(span, 1e-6f);
+    const int end = min(npts, (int)(blockIdx.x + 1) * kKeys);
+    for (int i = blockIdx.x * kKeys + threadIdx.x; i < end; i += kThreads) {
+        unsigned key;
+        if (FIRST) {
+            // Cells outside 0 .. 255 (no numbers, overflow) go to the edge cells.
+            const unsigned qx = (unsigned)fminf(fmaxf(((float)xyz[3LL * i] - x0) * scale, 0.0f), 255.0f);
+            const unsigned qy = (unsigned)fminf(fmaxf(((float)xyz[3LL * i + 1] - y0) * scale, 0.0f), 255.0f);
+            key = hilbert(qx, qy);
+            keys[i] = (unsigned short)key;
+        } else {
+            key = keys[i];
+        }
+        atomicAdd(&hist[FIRST ? key & 255u : key >> 8], 1);
+    }
+    __syncthreads();
+    counts[threadIdx.x * gridDim.x + blockIdx.x] = hist[threadIdx.x];
+}
+
+// Exclusive prefix sum of n counts in place (one block).
+__global__ void __launch_bounds__(1024) points_scan_kernel(const PointOrder* __restrict__ h, int* __restrict__ counts,
+                                                           int n) {
+    if (h->narrow) return;
+    __shared__ int warps[32];
+    const int per = (n + 1023) / 1024, b = min(n, (int)threadIdx.x * per), e = min(n, b + per);
+    int sum = 0;
+    for (int i = b; i < e; ++i) sum += counts[i];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) warps[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        int w = warps[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += v;
+        }
+        warps[lane] = w;
+    }
+    __syncthreads();
+    int at = inc - sum + (warp ? warps[warp - 1] : 0);
+    for (int i = b; i < e; ++i) {
+        const int v = counts[i];
+        counts[i] = at;
+        at += v;
+    }
+}
+
+// Stable scatter of one pass: a round of 256 keys at a time, ranked by warp (lanes with the same digit) and
+// over the warps.  FIRST: the payload is the point's index.
+template <bool FIRST>
+__global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, const PointOrder* __restrict__ h,
+                                                                  const unsigned short* __restrict__ keys,
+                                                                  const int* __restrict__ index,
+                                                                  const int* __restrict__ counts,
+                                                                  unsigned short* __restrict__ keys_out,
+                                                                  int* __restrict__ index_out) {
+    if (h->narrow) return;
+    __shared__ int base[kDigits];
+    __shared__ int seen[kThreads / 32][kDigits];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    base[threadIdx.x] = counts[threadIdx.x * gridDim.x + blockIdx.x];
+    const int begin = blockIdx.x * kKeys, end = min(npts, begin + kKeys);
+    for (int r = begin; r < end; r += kThreads) {
+        for (int w = 0; w < kThreads / 32; ++w) seen[w][threadIdx.x] = 0;
+        __syncthreads();
+        const int i = r + threadIdx.x;
+        const unsigned key = i < end ? keys[i] : 0u;
+        const unsigned digit = i < end ? (FIRST ? key & 255u : key >> 8) : kDigits;
+        const unsigned same = __match_any_sync(0xffffffffu, digit);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        if (i < end && rank == 0) seen[warp][digit] = __popc(same);
+        __syncthreads();
+        int at = base[threadIdx.x];  // thread t: digit t
+        for (int w = 0; w < kThreads / 32; ++w) {
+            const int v = seen[w][threadIdx.x];
+            seen[w][threadIdx.x] = at;
+            at += v;
+        }
+        base[threadIdx.x] = at;
+        __syncthreads();
+        if (i < end) {
+            const int to = seen[warp][digit] + rank;
+            index_out[to] = FIRST ? i : index[i];
+            if (FIRST) keys_out[to] = (unsigned short)key;
+        }
+        __syncthreads();
+    }
+}
+
+size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
+int order_blocks(int npts) { return (npts + kKeys - 1) / kKeys; }
+
+}  // namespace
+
+size_t points_order_bytes(int npts) {
+    return align_up(sizeof(PointOrder)) + 2 * align_up(sizeof(unsigned short) * (size_t)npts) +
+           2 * align_up(sizeof(int) * (size_t)npts) + align_up(sizeof(int) * (size_t)kDigits * order_blocks(npts));
+}
+
+// Orders the list in `ws` (points_order_bytes, 256-byte aligned); *order, *index: what the points kernel takes.
+int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder** order, const int** index,
+                        cudaStream_t s) {
+    char* p = static_cast<char*>(ws);
+    const auto take = [&p](size_t bytes) {
+        char* at = p;
+        p += align_up(bytes);
+        return at;
+    };
+    auto* h = reinterpret_cast<PointOrder*>(take(sizeof(PointOrder)));
+    auto* keys = reinterpret_cast<unsigned short*>(take(sizeof(unsigned short) * (size_t)npts));
+    auto* keys1 = reinterpret_cast<unsigned short*>(take(sizeof(unsigned short) * (size_t)npts));
+    auto* index1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)npts));
+    auto* index2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)npts));
+    const int blocks = order_blocks(npts);
+    auto* counts = reinterpret_cast<int*>(take(sizeof(int) * (size_t)kDigits * blocks));
+    const cudaError_t e = cudaMemsetAsync(h, 0xff, sizeof(PointOrder), s);
+    if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "points order: %s", cudaGetErrorString(e));
+    points_extent_kernel<<<(npts + kTilePoints - 1) / kTilePoints, kThreads, 0, s>>>(xyz, npts, h);
+    points_count_kernel<true><<<blocks, kThreads, 0, s>>>(xyz, npts, h, keys, counts);
+    points_scan_kernel<<<1, 1024, 0, s>>>(h, counts, kDigits * blocks);
+    points_scatter_kernel<true><<<blocks, kThreads, 0, s>>>(npts, h, keys, nullptr, counts, keys1, index1);
+    points_count_kernel<false><<<blocks, kThreads, 0, s>>>(xyz, npts, h, keys1, counts);
+    points_scan_kernel<<<1, 1024, 0, s>>>(h, counts, kDigits * blocks);
+    points_scatter_kernel<false><<<blocks, kThreads, 0, s>>>(npts, h, keys1, index1, counts, nullptr, index2);
+    note_launches(7);
+    *order = h;
+    *index = index2;
+    return check_launch("points_order");
+}
+
+}  // namespace sarbp

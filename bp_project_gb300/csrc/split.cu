@@ -44,6 +44,7 @@ namespace {
 
 constexpr int kThreads = kSplitThreads;
 constexpr int kPX = 4;
+constexpr int kPointPX = kPointTile / kThreads;  // pixels per thread of the points kernel
 // Threads of the single-scene merge kernel: four column pairs of parent pixels per thread (more
 // gathers in flight per warp than two pairs at 256 threads).
 constexpr int kMergeThreads = 128;
@@ -79,7 +80,10 @@ struct Rec {
     float4 a;  // W_hi.x, W_hi.y, W_lo.x, W_lo.y   (lattice: B_row hi, lo, B_col hi, lo)
     float4 b;  // u.x, u.y, 2R, frac(Q) - 1/2       (lattice: u.s_row, u.s_col, 2R (forward: R), frac(Q) - 1/2)
     float4 c;  // Phi, window bias bits, window offset bits, window count - 1 bits
-               // (lattice forward: Phi', window byte base, 2 pi frac(B_row), 12.5 e4: see lattice_runs)
+               // (lattice forward: Phi', window byte base, 2 pi frac(B_row), 12.5 e4: see lattice_runs;
+               // points: a = W in 2^-16 turns/m and Phi in 2^-32 turns, e = u / dr in 2^-12 bins/m and c.x the
+               // middle's place in the window in 2^-28 bins (integers); b = u, 2R; c.y that place, FP32;
+               // d = rest of W, rest of u.x / dr; e.w rest of u.y / dr)
     float4 d;  // u.z, W_hi.z, W_lo.z                (lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z)
     float4 e;  // lattice adjoint: the pairs (2R, 2R), (frac(Q) - 1/2, frac(Q) - 1/2) of packed-FP32 operands;
                // lattice forward: (-, window bias bits, window offset bits, window count - 1 bits)
@@ -99,6 +103,17 @@ struct Pix {
     float ar, ai;
 };
 
+// A point's offset from the tile centre: FP32 plus rest (the fallback's two-float), and as a whole number of
+// 2^-16 m plus rest for the phase.
+struct PointPix {
+    float dx, dy, dz;     // FP32
+    float lx, ly, lz;     // offset - dx
+    int ix, iy, iz;       // rint(2^16 dx)
+    float rx, ry, rz;     // offset - 2^-16 ix
+    float d2;
+    float ar, ai;
+};
+
 struct TileShared {
     double cx, cy, cz;
     float ch[3], cl[3];         // the centre as two-float (hi + lo), for the FP32 records
@@ -111,6 +126,7 @@ struct TileShared {
     float red[8][8];
     int base[kMaxChunk];        // global bin of window entry 0, per pulse of the chunk
     float wt[kMaxChunk];
+    float rest[kMaxChunk];      // points: the z part of the range scale's rest (see points_chunk)
     int nfit;
     int nfit_w[2];              // fitting pulses among each record warp's 32
     unsigned miss_w[2];         // pulses of each record warp that cannot be staged (bit per lane)
@@ -154,7 +170,8 @@ struct Job {
     PolarDesc g;          // polar grids
     sarbp_lattice lat;    // lattices
     const double* xyz;    // point lists
-    int npts;
+    const int* index;     // the point at each place of the list's spatial order, or NULL
+    int p_begin, p_end;   // the points of the tile (or of a stretch of it)
     int tile_r, tile_u, lc;
     int p0, p1;
 };
@@ -549,18 +566,20 @@ __device__ void setup_lattice_sep(const Job& J, TileShared& S, float d2[kPX]) {
     }
 }
 
-__device__ void setup_points(const Job& J, TileShared& S, Pix px[kPX]) {
+// Points [J.p_begin, J.p_end) of the list; the tile's other places repeat the first of them.
+__device__ void setup_points(const Job& J, TileShared& S, PointPix px[kPointPX]) {
     const int tid = threadIdx.x;
-    double p3[kPX][3];
+    double p3[kPointPX][3];
     double v[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) {
+    for (int k = 0; k < kPointPX; ++k) {
         const int idx = J.tile_r + tid + kThreads * k;
-        const bool ok = idx < J.npts;
-        const int q = ok ? idx : J.tile_r;
-        p3[k][0] = J.xyz[3 * q];
-        p3[k][1] = J.xyz[3 * q + 1];
-        p3[k][2] = J.xyz[3 * q + 2];
+        const bool ok = idx >= J.p_begin && idx < J.p_end;
+        int q = ok ? idx : J.p_begin;
+        if (J.index) q = J.index[q];
+        p3[k][0] = J.xyz[3LL * q];
+        p3[k][1] = J.xyz[3LL * q + 1];
+        p3[k][2] = J.xyz[3LL * q + 2];
         if (ok) {
             v[0] += p3[k][0];
             v[1] += p3[k][1];
@@ -572,7 +591,7 @@ __device__ void setup_points(const Job& J, TileShared& S, Pix px[kPX]) {
     const double cx = v[0] / v[3], cy = v[1] / v[3], cz = v[2] / v[3];
     float m[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) {
+    for (int k = 0; k < kPointPX; ++k) {
         m[0] = fmaxf(m[0], (float)fabs(p3[k][0] - cx));
         m[1] = fmaxf(m[1], (float)fabs(p3[k][1] - cy));
         m[2] = fmaxf(m[2], (float)fabs(p3[k][2] - cz));
@@ -587,80 +606,93 @@ __device__ void setup_points(const Job& J, TileShared& S, Pix px[kPX]) {
         S.bnd[0] = (float)b0;
         S.bnd[1] = (float)b1;
         S.bnd[2] = (float)b2;
-        set_quantum(S, (float)fmax(b0, fmax(b1, b2)), 11);
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) {
-        Pix& q = px[k];
-        pixel_from_offsets(S, p3[k][0] - cx, p3[k][1] - cy, p3[k][2] - cz, q);
-        q.psi = 0.0f;
+    for (int k = 0; k < kPointPX; ++k) {
+        PointPix& q = px[k];
+        const auto part = [](double o, float& h, float& l, int& n, float& r) {
+            split2(o, h, l);
+            n = __float2int_rn(h * 65536.0f);
+            r = (h - (float)n * (1.0f / 65536.0f)) + l;  // exact difference within 256 m
+        };
+        part(p3[k][0] - cx, q.dx, q.lx, q.ix, q.rx);
+        part(p3[k][1] - cy, q.dy, q.ly, q.iy, q.ry);
+        part(p3[k][2] - cz, q.dz, q.lz, q.iz, q.rz);
+        q.d2 = q.dx * q.dx + q.dy * q.dy + q.dz * q.dz;
         q.ar = q.ai = 0.0f;
     }
 }
 
 // ---- the pulse loop ---------------------------------------------------------------
-template <bool HAS_Z, bool DEMOD>
-__device__ __forceinline__ void fast_chunk(const SplitParams& P, const Rec* __restrict__ rec,
-                                           const float4* __restrict__ win, int chn, Pix px[kPX]) {
+// Points: offsets in three dimensions, no demodulation.  The large linear terms of the phase and of
+// the range, W . delta and u . delta / dr, are formed in 32-bit integers: with W in whole 2^-16
+// turns/m, u / dr in whole 2^-12 bins/m and delta in whole 2^-16 m, the wrapping products and their sums are exact
+// modulo one turn (2^-32 turns) and modulo 16 bins (2^-28 bins); taking the nearest bin off leaves
+// a fraction of a bin.  What the roundings leave (rests of W, u / dr and delta, below 1e-3 turns or bins) is FP32.
+// An FP32 range of ten bins alone would put 3e-7 on the fraction, and through it on the image.  Tiles hold
+// 512 points (the range correction, FP32, grows with the square of the tile).  192,384 points, 1024
+// pulses: 0.64 ms; with FP32 products of 10- and 11-bit parts 0.58 ms and an error of 3.6e-7 instead of 2.8e-7.
+__device__ __forceinline__ void points_chunk(const SplitParams& P, const Rec* __restrict__ rec,
+                                             const float4* __restrict__ win, const float* __restrict__ rest, int chn,
+                                             PointPix px[kPointPX]) {
     const float inv_dr = P.inv_drf, Kf = P.Kf;
+    // The chunk's sum goes to the image at the end: shorter FP32 sums.
+    float ar[kPointPX], ai[kPointPX];
+#pragma unroll
+    for (int k = 0; k < kPointPX; ++k) ar[k] = ai[k] = 0.0f;
 #pragma unroll 1
     for (int nl = 0; nl < chn; ++nl) {
-        const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c;
-        float4 rd = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (HAS_Z) rd = rec[nl].d;
-        const int bias = __float_as_int(rc.y);
-        const unsigned last = (unsigned)__float_as_int(rc.w);
+        const float4 rb = rec[nl].b, rc = rec[nl].c, rd = rec[nl].d;
+        const int4 ri = *reinterpret_cast<const int4*>(&rec[nl].a), re = *reinterpret_cast<const int4*>(&rec[nl].e);
+        const float uly = __int_as_float(re.w), ulz = rest[nl];
         const float4* wrow = win + 2 * __float_as_int(rc.z);
 #pragma unroll
-        for (int k = 0; k < kPX; ++k) {
-            Pix& q = px[k];
-            float L = fmaf(rb.x, q.dx, rb.y * q.dy);
-            if (HAS_Z) L = fmaf(rd.x, q.dz, L);
+        for (int k = 0; k < kPointPX; ++k) {
+            const PointPix& q = px[k];
+            const float L = fmaf(rb.z, q.dz, fmaf(rb.x, q.dx, rb.y * q.dy));
             const float q2 = fmaf(-L, L, q.d2);
-            const float B = rcp_approx(fmaf(2.0f, L, rb.z));
+            const float B = rcp_approx(fmaf(2.0f, L, rb.w));
             const float e0 = q2 * B;
             const float eps = fmaf(-e0 * e0, B, e0);
-            const float qp = fmaf(L + eps, inv_dr, rb.w);
-            const float tq = qp + kMagic;
-            const float s = qp - (tq - kMagic);
-            const unsigned j = min((unsigned)(__float_as_int(tq) - bias), last);
+            // Nearest bin of the window (see lattice_runs for why it is inside).
+            const float tq = fmaf(L + eps, inv_dr, rc.y) + kMagic;
+            const unsigned j = (unsigned)(__float_as_int(tq) - kMagicBits);
             const float4 c01 = wrow[2 * j], c23 = wrow[2 * j + 1];
+            // u . (rest of delta), in metres, with eps: small terms of the range and of the phase.
+            const float er = eps + fmaf(rb.z, q.rz, fmaf(rb.x, q.rx, rb.y * q.ry));
+            const int bins = (int)((unsigned)__float_as_int(rc.x) - ((unsigned)__float_as_int(tq) << 28) +
+                                   (unsigned)re.x * (unsigned)q.ix + (unsigned)re.y * (unsigned)q.iy +
+                                   (unsigned)re.z * (unsigned)q.iz);
+            const float s = fmaf(inv_dr, er, fmaf((float)bins, 3.7252902984619141e-09f,
+                                                  fmaf(ulz, q.dz, fmaf(uly, q.dy, rd.w * q.dx))));
             const float vr = fmaf(fmaf(fmaf(c23.z, s, c23.x), s, c01.z), s, c01.x);
             const float vi = fmaf(fmaf(fmaf(c23.w, s, c23.y), s, c01.w), s, c01.y);
-            float tb = ra.y * q.dyh;
-            if (HAS_Z) tb = fmaf(rd.y, q.dzh, tb);
-            tb = fmaf(ra.x, q.dxh, tb);
-            float sm = fmaf(Kf, eps, rc.x);
-            sm = fmaf(ra.x, q.dxl, sm);
-            sm = fmaf(ra.y, q.dyl, sm);
-            sm = fmaf(ra.z, q.dx, sm);
-            sm = fmaf(ra.w, q.dy, sm);
-            if (HAS_Z) {
-                sm = fmaf(rd.y, q.dzl, sm);
-                sm = fmaf(rd.z, q.dz, sm);
-            }
-            if (DEMOD) sm += q.psi;
-            // The reduced large term is in [-1/2, 1/2] turn and |sm| <= 1 + K eps <= 1 + envelope / 2
-            // turns (5 turns for direct tiles), so the angle stays within +-40 rad: the hardware
-            // sin/cos reduce it themselves with an absolute error below 3e-6 rad, and a second
-            // reduction in turns is not needed.
-            const float ang = ((tb - round_magic(tb)) + sm) * kTwoPiF;
+            const int turns = (int)((unsigned)ri.w + (unsigned)ri.x * (unsigned)q.ix + (unsigned)ri.y * (unsigned)q.iy +
+                                    (unsigned)ri.z * (unsigned)q.iz);
+            const float tot = fmaf(Kf, er, fmaf((float)turns, 2.3283064365386963e-10f,
+                                                fmaf(rd.z, q.dz, fmaf(rd.y, q.dy, rd.x * q.dx))));
+            // K eps goes to a few turns, beyond which the hardware sine and cosine lose accuracy.
+            const float ang = (tot - round_magic(tot)) * kTwoPiF;
             float sn, cs;
             __sincosf(ang, &sn, &cs);
-            q.ar = fmaf(vr, cs, q.ar);
-            q.ar = fmaf(-vi, sn, q.ar);
-            q.ai = fmaf(vr, sn, q.ai);
-            q.ai = fmaf(vi, cs, q.ai);
+            ar[k] = fmaf(vr, cs, ar[k]);
+            ar[k] = fmaf(-vi, sn, ar[k]);
+            ai[k] = fmaf(vr, sn, ai[k]);
+            ai[k] = fmaf(vi, cs, ai[k]);
         }
+    }
+#pragma unroll
+    for (int k = 0; k < kPointPX; ++k) {
+        px[k].ar += ar[k];
+        px[k].ai += ai[k];
     }
 }
 
-// fast_chunk for 2-D demodulated tiles (polar grids) with the thread's pixels k = 2h, 2h + 1
-// as packed FP32 (f32x2) pairs through the range, fraction, window-index and phase steps; the
-// complex cubic evaluates (re, im) as one pair and the accumulation stays scalar.  Every half
-// rounds like fast_chunk's scalar operation, and the chain carries -L, -q2, -e0 and -eps
-// (negation is exact), so the image is fast_chunk<false, true>'s bit for bit:
+// 2-D demodulated tiles (polar grids) with the thread's pixels k = 2h, 2h + 1 as packed FP32
+// (f32x2) pairs through the range, fraction, window-index and phase steps; the complex cubic
+// evaluates (re, im) as one pair and the accumulation stays scalar.  The chain carries -L, -q2,
+// -e0 and -eps (negation is exact):
 //   -L = (-u) . delta,  -q2 = (-L)^2 - d2,  2L + 2R = -2 (-L) + 2R,  -e0 = -q2 B,
 //   -eps = (-e0)^2 B + (-e0),  qp = ((-L) + (-eps)) (-1/dr) + Fm,  sm = -K (-eps) + Phi + ...
 __device__ __forceinline__ void polar_chunk(const SplitParams& P, const Rec* __restrict__ rec,
@@ -873,7 +905,7 @@ __device__ __noinline__ void slow_record(const SplitParams& P, const TileShared&
 // arithmetic (about 44 bits; GB300's FP64 rate would make these records the barrier-bound
 // part of every chunk).  Returns the number of window entries the pulse needs (cap + 1 if
 // it cannot be staged).
-// MODE 0: per-pixel offsets (polar, points); 1: lattice tiles; 2: lattice tiles, adjoint.
+// MODE 0: per-pixel offsets (polar); 1: lattice tiles; 2: lattice tiles, adjoint; 3: points.
 template <int MODE>
 __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, Rec* rec, int lane, int n) {
     const PulseInputs& in = P.in;
@@ -919,7 +951,25 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
     S.wt[lane] = (float)in.weight[n];
     Rec r;
     const FF Wx = ff_mul(Kk, ux), Wy = ff_mul(Kk, uy), Wz = ff_mul(Kk, uz);
-    if (MODE != 0) {
+    if (MODE == 3) {
+        const auto whole = [](FF w, float scale, float inv, float& rest) {
+            const int n = __float2int_rn(w.h * scale);
+            rest = (w.h - (float)n * inv) + w.l;  // exact difference (n has 24 bits or fewer)
+            return __int_as_float(n);
+        };
+        const FF idr{P.idrh, P.idrl};
+        r.a.x = whole(Wx, 65536.0f, 1.0f / 65536.0f, r.d.x);
+        r.a.y = whole(Wy, 65536.0f, 1.0f / 65536.0f, r.d.y);
+        r.a.z = whole(Wz, 65536.0f, 1.0f / 65536.0f, r.d.z);
+        r.a.w = __int_as_float(__float2int_rn(t1 * 4294967296.0f));  // |t1| <= 1/2 (saturates at 1/2)
+        r.b = make_float4(uxf, uyf, uzf, 2.0f * Rf);
+        r.e.x = whole(ff_mul(ux, idr), 4096.0f, 1.0f / 4096.0f, r.d.w);
+        r.e.y = whole(ff_mul(uy, idr), 4096.0f, 1.0f / 4096.0f, r.e.w);
+        r.e.z = whole(ff_mul(uz, idr), 4096.0f, 1.0f / 4096.0f, S.rest[lane]);
+        const int mid = __float2int_rn(Fm * 268435456.0f);  // |Fm| <= 1/2
+        r.c.x = __int_as_float((int)((unsigned)mid - ((unsigned)bo << 28)));
+        r.c.y = Fm - (float)bo;
+    } else if (MODE != 0) {
         // Lattice tile: the linear phase W . delta of pixel (i, j) is i B_row + j B_col with
         // B = W . step.  Both are split on one power-of-two quantum with <= 10 significant
         // bits, so i B_row_hi + j B_col_hi is exact in FP32 for |i|, |j| < 2^12.
@@ -978,9 +1028,9 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         r.d.w = 0.0f;
         r.e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    if (MODE != 1) r.c.x = t1;
+    if (MODE == 0 || MODE == 2) r.c.x = t1;
     float4& rw = rec_window<MODE>(r);
-    rw.y = __int_as_float(kMagicBits + bo);
+    if (MODE != 3) rw.y = __int_as_float(kMagicBits + bo);
     const int count = ok ? (int)(hi - lo) + 1 : P.cap + 1;
     rw.z = 0.0f;
     rw.w = __int_as_float(count - 1);
@@ -1295,38 +1345,44 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
 #endif
 }
 
-template <bool HAS_Z, bool DEMOD>
-struct ForwardBody {
+struct PolarBody {
     static constexpr int kRecMode = 0;
     // Polar grids stage their windows with one load per lane and shuffled neighbours (751 against
     // 744 Gpixel-pulses/s on the 4096-pulse root grid); the lattice loop measured 0.5% slower with it.
-    static constexpr bool kShflWindows = !HAS_Z && DEMOD;
+    static constexpr bool kShflWindows = true;
     const SplitParams& P;
-    const TileShared& S;
     Pix* px;
-    __device__ void fast(const Rec* rec, const float4* win, int nfit, int) {
-        if (!HAS_Z && DEMOD)
-            polar_chunk(P, rec, win, nfit, px);
-        else
-            fast_chunk<HAS_Z, DEMOD>(P, rec, win, nfit, px);
-    }
+    __device__ void fast(const Rec* rec, const float4* win, int nfit, int) { polar_chunk(P, rec, win, nfit, px); }
     __device__ void slow(int c0, int nslow, const SlowRec* srec) {
 #pragma unroll
         for (int k = 0; k < kPX; ++k) {
             const Pix& q = px[k];
-            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
-                                        DEMOD ? q.psi : 0.0f);
+            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, q.psi);
             px[k].ar += v.x;
             px[k].ai += v.y;
         }
     }
 };
 
-template <bool HAS_Z, bool DEMOD>
-__device__ void pulse_loop(const SplitParams& P, const Job& J, TileShared& S, char* smem, Pix px[kPX]) {
-    ForwardBody<HAS_Z, DEMOD> body{P, S, px};
-    chunk_loop(P, J, S, smem, true, body);
-}
+struct PointsBody {
+    static constexpr int kRecMode = 3;
+    static constexpr bool kShflWindows = false;
+    const SplitParams& P;
+    const TileShared& S;
+    PointPix* px;
+    __device__ void fast(const Rec* rec, const float4* win, int nfit, int) {
+        points_chunk(P, rec, win, S.rest, nfit, px);
+    }
+    __device__ void slow(int c0, int nslow, const SlowRec* srec) {
+#pragma unroll
+        for (int k = 0; k < kPointPX; ++k) {
+            const PointPix& q = px[k];
+            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dx, q.lx, q.dy, q.ly, q.dz, q.lz, 0.0f);
+            px[k].ar += v.x;
+            px[k].ai += v.y;
+        }
+    }
+};
 
 // ---- lattice tiles: runs of eight rows ---------------------------------------------------
 //
@@ -1814,7 +1870,8 @@ __global__ void __launch_bounds__(kThreads, 3) split_polar_kernel(SplitParams P,
     Pix px[kPX];
     PolarTables& T = *reinterpret_cast<PolarTables*>(smem + window_offset());
     setup_polar(P, J, S, T, px, true);
-    pulse_loop<false, true>(P, J, S, smem, px);
+    PolarBody body{P, px};
+    chunk_loop(P, J, S, smem, true, body);
     store_window(J, g.win_nr, g.win_nu, px, P.out + blockIdx.y * P.split_stride, P.out_stride);
 }
 
@@ -1875,24 +1932,61 @@ __global__ void __launch_bounds__(kThreads, 4) split_lattice_kernel(SplitParams 
 }
 
 __global__ void __launch_bounds__(kThreads, 3) split_points_kernel(SplitParams P, const double* __restrict__ xyz,
-                                                                   int npts) {
+                                                                   int npts, const PointOrder* __restrict__ order,
+                                                                   const int* __restrict__ index) {
     extern __shared__ __align__(16) char smem[];
     __shared__ TileShared S;
     Job J;
     J.xyz = xyz;
-    J.npts = npts;
+    J.index = order && !order->narrow ? index : nullptr;
     J.lc = 0;
-    J.tile_r = blockIdx.x * kSplitTilePixels;
+    J.tile_r = blockIdx.x * kPointTile;
     J.tile_u = 0;
     split_range(0, P.in.pulses, P.pulse_split, blockIdx.y, J.p0, J.p1);
-    Pix px[kPX];
-    setup_points(J, S, px);
-    pulse_loop<true, false>(P, J, S, smem, px);
-    float2* out = P.out + blockIdx.y * P.split_stride;
+    const int end = min(npts, J.tile_r + kPointTile);
+    // A tile whose list jumps (a spatial order leaves and re-enters the points' outline, targets follow each
+    // other) is formed stretch by stretch: one wide tile on the two-float fallback would take as long as seven
+    // others and hold up the launch's end.  Lists that jump all the time stay whole.
+    __shared__ unsigned jumps[kPointTile / 32];
+    constexpr float kJump2 = 16.0f * 16.0f;
 #pragma unroll
-    for (int k = 0; k < kPX; ++k) {
-        const int idx = J.tile_r + threadIdx.x + kThreads * k;
-        if (idx < npts) out[idx] = make_float2(px[k].ar, px[k].ai);
+    for (int k = 0; k < kPointPX; ++k) {
+        const int at = J.tile_r + threadIdx.x + kThreads * k;
+        bool jump = false;
+        if (at > J.tile_r && at < end) {
+            const double* a = xyz + 3LL * (J.index ? J.index[at] : at);
+            const double* b = xyz + 3LL * (J.index ? J.index[at - 1] : at - 1);
+            const float dx = (float)a[0] - (float)b[0], dy = (float)a[1] - (float)b[1], dz = (float)a[2] - (float)b[2];
+            jump = dx * dx + dy * dy + dz * dz > kJump2;
+        }
+        const unsigned w = __ballot_sync(0xffffffffu, jump);
+        if ((threadIdx.x & 31) == 0) jumps[(threadIdx.x + kThreads * k) >> 5] = w;
+    }
+    __syncthreads();
+    int njumps = 0;
+    for (int w = 0; w < kPointTile / 32; ++w) njumps += __popc(jumps[w]);
+    float2* out = P.out + blockIdx.y * P.split_stride;
+    for (J.p_begin = J.tile_r; J.p_begin < end; J.p_begin = J.p_end) {
+        J.p_end = end;
+        if (njumps <= 4)
+            for (int w = (J.p_begin + 1 - J.tile_r) >> 5, from = (J.p_begin + 1 - J.tile_r) & 31; w < kPointTile / 32;
+                 ++w, from = 0) {
+                const unsigned rest = jumps[w] & (0xffffffffu << from);
+                if (rest) {
+                    J.p_end = J.tile_r + 32 * w + __ffs(rest) - 1;
+                    break;
+                }
+            }
+        PointPix px[kPointPX];
+        setup_points(J, S, px);
+        PointsBody body{P, S, px};
+        chunk_loop(P, J, S, smem, true, body);
+#pragma unroll
+        for (int k = 0; k < kPointPX; ++k) {
+            const int idx = J.tile_r + threadIdx.x + kThreads * k;
+            if (idx >= J.p_begin && idx < J.p_end) out[J.index ? J.index[idx] : idx] = make_float2(px[k].ar, px[k].ai);
+        }
+        __syncthreads();  // the next stretch's set-up
     }
 }
 
@@ -3041,10 +3135,10 @@ int prepare(K kernel, size_t smem) {
 // s <= 8 (and <= pulses), ties to the smaller split.  A tile's pulse ranges are independent
 // work, so a small image with few tiles still keeps every SM busy to the end.
 template <class K>
-int best_pulse_split(K kernel, size_t smem, long long tiles, int pulses) {
+int best_pulse_split(K kernel, int threads, size_t smem, long long tiles, int pulses) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) != cudaSuccess || per_sm <= 0 ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm <= 0 ||
         sms <= 0 || tiles <= 0) {
         cudaGetLastError();
         return 1;
@@ -3167,7 +3261,7 @@ int split_wait_timeouts(int* count) {
 int split_lattice_auto_split(const sarbp_lattice& lat, int pulses) {
     const size_t smem = dynamic_smem(capacity_for(kMaxChunk, 1 << 20, kLatticeWindowBudget), false);
     if (prepare(split_lattice_kernel, smem) != SARBP_OK) return 1;
-    return best_pulse_split(split_lattice_kernel, smem, tiles_of(lat.rows, lat.cols, 5), pulses);
+    return best_pulse_split(split_lattice_kernel, kThreads, smem, tiles_of(lat.rows, lat.cols, 5), pulses);
 }
 
 int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pulse_split, int chunk, int window_bins,
@@ -3184,15 +3278,22 @@ int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pu
     return check_launch("split_lattice");
 }
 
-int launch_split_points(const PulseInputs& in, const double* xyz, int npts, int pulse_split, int chunk,
-                        int window_bins, float2* out, long long split_stride, cudaStream_t s) {
+int split_points_auto_split(int npts, int pulses) {
+    const size_t smem = dynamic_smem(capacity_for(kMaxChunk, 1 << 20), false);
+    if (prepare(split_points_kernel, smem) != SARBP_OK) return 1;
+    return best_pulse_split(split_points_kernel, kThreads, smem, (npts + kPointTile - 1) / kPointTile, pulses);
+}
+
+int launch_split_points(const PulseInputs& in, const double* xyz, int npts, const PointOrder* order, const int* index,
+                        int pulse_split, int chunk, int window_bins, float2* out, long long split_stride,
+                        cudaStream_t s) {
     SplitParams P = make_params(in, chunk, capacity_for(chunk, window_bins), pulse_split);
     P.out = out;
     P.split_stride = split_stride;
     const size_t smem = dynamic_smem(P.cap, false);
     if (int st = prepare(split_points_kernel, smem)) return st;
-    dim3 grid((npts + kSplitTilePixels - 1) / kSplitTilePixels, pulse_split);
-    split_points_kernel<<<grid, kThreads, smem, s>>>(P, xyz, npts);
+    dim3 grid((npts + kPointTile - 1) / kPointTile, pulse_split);
+    split_points_kernel<<<grid, kThreads, smem, s>>>(P, xyz, npts, order, index);
     note_launches(1);
     return check_launch("split_points");
 }
@@ -3209,7 +3310,7 @@ int launch_split_lattice_adjoint(const PulseInputs& in, const sarbp_lattice& lat
     const size_t smem = dynamic_smem(P.cap, false);
     const int ntiles = tiles_of(lat.rows, lat.cols, lc);
     if (int st = prepare(split_lattice_adjoint_kernel, smem)) return st;
-    const dim3 grid(ntiles, best_pulse_split(split_lattice_adjoint_kernel, smem, ntiles, in.pulses));
+    const dim3 grid(ntiles, best_pulse_split(split_lattice_adjoint_kernel, kThreads, smem, ntiles, in.pulses));
     split_lattice_adjoint_kernel<<<grid, kThreads, smem, s>>>(P, lat, lc, grad, partials);
     note_launches(1);
     if (int st = check_launch("split_lattice_adjoint")) return st;
