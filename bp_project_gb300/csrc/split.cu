@@ -77,10 +77,11 @@ __host__ __device__ constexpr int raw_bytes_for(int cap, int chunk) {
 constexpr double kDirectEnvelope = 8.0;
 
 struct Rec {
-    float4 a;  // W_hi.x, W_hi.y, W_lo.x, W_lo.y   (lattice: B_row hi, lo, B_col hi, lo)
+    float4 a;  // W_hi.x, W_hi.y, W_lo.x, W_lo.y   (lattice adjoint: B_row hi, lo, B_col hi, lo;
+               // lattice forward: B_row / 2 and B_col modulo one turn in 2^-32 turns, integers)
     float4 b;  // u.x, u.y, 2R, frac(Q) - 1/2       (lattice: u.s_row, u.s_col, 2R (forward: R), frac(Q) - 1/2)
     float4 c;  // Phi, window bias bits, window offset bits, window count - 1 bits
-               // (lattice forward: Phi', window byte base, 2 pi frac(B_row), 12.5 e4: see lattice_runs;
+               // (lattice forward: Phi' in 2^-32 turns, window byte base, 2 pi frac(B_row), 12.5 e4: see lattice_runs;
                // points: a = W in 2^-16 turns/m and Phi in 2^-32 turns, e = u / dr in 2^-12 bins/m and c.x the
                // middle's place in the window in 2^-28 bins (integers); b = u, 2R; c.y that place, FP32;
                // d = rest of W, rest of u.x / dr; e.w rest of u.y / dr)
@@ -995,6 +996,15 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         const float Ac = fmaf(uxf, S.sth[3], fmaf(uyf, S.sth[4], uzf * S.sth[5]));
         const float spr = sp * kTwoPiF;  // the phase step in radians
         if (MODE == 1) {
+            // The linear phase per half row and per column, modulo one turn, in 2^-32 turns: the middle of a
+            // run is a whole number of half rows and of columns away, so wrapping products are exact.
+            const auto wrap = [](FF v) {
+                const float n = rintf(v.h);
+                return (int)((unsigned)__float2int_rn((v.h - n) * 4294967296.0f) +
+                             (unsigned)__float2int_rn(v.l * 4294967296.0f));
+            };
+            r.a.x = __int_as_float(wrap(FF{0.5f * Br.h, 0.5f * Br.l}));
+            r.a.y = __int_as_float(wrap(Bc));
             r.b = make_float4(Ar, Ac, Rf, Fm);
             // Fourth-order range term of a run of rows, e4 k^4 with k^4 ~ 12.5 k^2 - 21.0625 (lattice_runs).
             const float s2 = S.sth[0] * S.sth[0] + S.sth[1] * S.sth[1] + S.sth[2] * S.sth[2];
@@ -1009,7 +1019,9 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
             r.c.z = (sp - 0.5f * n2) * kTwoPiF;
             r.c.x += even - rintf(even);
             const float odd = 0.5f * n2;
-            r.d = make_float4(odd - rintf(odd), 0.0f, 0.0f, 0.0f);
+            r.d.x = odd - rintf(odd);
+            r.d.y = r.d.z = r.d.w = 0.0f;
+            r.c.x = __int_as_float(wrap(FF{r.c.x, 0.0f}));
         } else {
             r.b = make_float4(Ar, Ac, 2.0f * Rf, Fm);
             r.d = make_float4(spr, uxf, uyf, uzf);
@@ -1407,11 +1419,12 @@ struct PointsBody {
 // What bounds the loop: the register file feeds two operands a cycle to the FMA pipe (a fused
 // multiply-add of three registers takes 1.5 cycles, a packed one 3), so issue sits at 71% with the
 // FMA pipe, the shared-memory pipe and issue all at 60-70%, and every instruction removed shows in
-// the time.  4096 pulses onto 2048 x 2048: 17.2 ms (998 Gpixel-pulses/s; 29.4 instructions per
+// the time.  4096 pulses onto 2048 x 2048: 17.1 ms (1006 Gpixel-pulses/s; 28.9 instructions per
 // pixel-pulse), 19.6 ms (876; 31.3) with four pixels per thread and the root-free range chain of the
 // adjoint per pixel.  Measured and not kept: runs of 16 (24 warps per SM instead of 32: 16.7 ms, but a larger
-// error on small scenes), even and odd parts of the polynomials with constant multipliers (17.2), scalar
-// cubic (17.5), staging two bins per lane (17.15) and three blocks per SM (17.7).
+// error on small scenes), the range to the middle in integers too (18.3; error 0.68e-6 instead of 0.80), even
+// and odd parts of the polynomials with constant multipliers (17.2), scalar cubic (17.5), staging two bins per
+// lane (17.15) and three blocks per SM (17.7).
 constexpr int kRun = 8;                               // pixels per run
 constexpr int kRunThreads = kSplitTilePixels / kRun;  // threads per pulse group
 
@@ -1420,16 +1433,17 @@ constexpr int kRunThreads = kSplitTilePixels / kRun;  // threads per pulse group
 // the chunks) and their images are added once at the end.
 __device__ __forceinline__ void lattice_runs(const SplitParams& P, const Rec* __restrict__ rec,
                                              const char* __restrict__ win, int first, int chn, float di, float dj,
-                                             float d2, float ds, float s2, float ar[kRun], float ai[kRun]) {
+                                             int hi2, int ji, float d2, float ds, float s2, float ar[kRun], float ai[kRun]) {
     const float inv_dr = P.inv_drf, kr = P.Kf * kTwoPiF;
     const float2 magic = pair(kMagic), nmagic = pair(-kMagic), mone = pair(-1.0f);
 #pragma unroll 1
     for (int nl = first; nl < chn; nl += 2) {
-        const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c;
+        const int4 ra = *reinterpret_cast<const int4*>(&rec[nl].a);
+        const float4 rb = rec[nl].b, rc = rec[nl].c;
+        const float2 rd = *reinterpret_cast<const float2*>(&rec[nl].d);
         const unsigned wbase = (unsigned)__float_as_int(rc.y);
         const float L = fmaf(dj, rb.y, di * rb.x);
-        const float t = fmaf(dj, ra.z, di * ra.x);  // exact
-        const float ph = (t - round_magic(t)) + fmaf(dj, ra.w, fmaf(di, ra.y, rc.x));  // turns
+        const int turns = (int)((unsigned)__float_as_int(rc.x) + (unsigned)ra.x * (unsigned)hi2 + (unsigned)ra.y * (unsigned)ji);
         const float q2 = fmaf(-L, L, d2);
         const float h = rb.z + L;
         const float B = rcp_approx(h + h);
@@ -1441,9 +1455,9 @@ __device__ __forceinline__ void lattice_runs(const SplitParams& P, const Rec* __
         const float a = rb.x + e1;
         const float e2 = fmaf(fmaf(-a, a, s2), 0.5f * iD, rc.w);
         const float e3 = -a * e2 * iD;
-        float P0 = fmaf(P.Kf, eps, ph);
+        float P0 = fmaf(P.Kf, eps, (float)turns * 2.3283064365386963e-10f);
         P0 -= round_magic(P0);
-        const float2 p0 = __fmul2_rn(make_float2(P0, P0 + rec[nl].d.x), pair(kTwoPiF));
+        const float2 p0 = __fmul2_rn(make_float2(P0, P0 + rd.x), pair(kTwoPiF));
         const float2 p1 = pair(fmaf(kr, e1, rc.z));
         const float2 p2 = pair(kr * e2), p3 = pair(kr * e3);
         const float2 q0 = pair(fmaf(Le, inv_dr, rb.w)), q1 = pair(a * inv_dr), q2k = pair(e2 * inv_dr);
@@ -1504,8 +1518,8 @@ struct LatticeBody {
     float* ai;
     __device__ int group() const { return threadIdx.x / kRunThreads; }
     __device__ void fast(const Rec* rec, const float4* win, int nfit, int c0) {
-        lattice_runs(P, rec, reinterpret_cast<const char*>(win), (c0 - J.p0 + group()) & 1, nfit, di, dj, d2, ds, s2, ar,
-                     ai);
+        lattice_runs(P, rec, reinterpret_cast<const char*>(win), (c0 - J.p0 + group()) & 1, nfit, di, dj,
+                     (int)(2.0f * di), (int)dj, d2, ds, s2, ar, ai);
     }
     __device__ void slow(int c0, int nslow, const SlowRec* srec) {
         float2 more[kRun];
