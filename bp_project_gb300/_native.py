@@ -101,6 +101,9 @@ SIGNATURES = {
     "sarbp_batch_execute": ([_P, _P], _I),
     "sarbp_batch_set_trace": ([_P, _P], _I),
     "sarbp_batch_set_concurrent": ([_P, _I], _I),
+    "sarbp_pga_max_targets": ([], _I),
+    "sarbp_pga_update_workspace": ([_I, _I], _Z),
+    "sarbp_pga_update": ([_P, _I, _I, _P, _P, _D, _P, _P, _P, _I, _P, _P, _P, _Z, _P], _I),
     "sarbp_rc_block_points": ([], _I),
     "sarbp_rc_blocks_fit": ([_I, _I], _I),
     "sarbp_rc_blocks": ([_P, _I, _I, _I, _P, _P, _P], _I),

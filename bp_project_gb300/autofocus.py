@@ -7,8 +7,8 @@ Two estimators of per-pulse navigation errors, both device-resident:
   Target contributions come from the ``sarbp_target_contributions`` kernel,
   the Butterworth smoothing of each target's pulse history from the
   ``sarbp_sosfiltfilt`` kernel, and the robust weighted least squares, the
-  detrend and the Savitzky-Golay smoothing run as FP64 torch operations on
-  the device.  scipy designs the filters (coefficients only).
+  detrend and the Savitzky-Golay smoothing from ``sarbp_pga_update`` (FP64; torch
+  operations for more than 1024 targets).  scipy designs the filters (coefficients only).
 * ``entropy_autofocus``: minimises the image entropy of a split-precision
   lattice image over per-pulse phase and position corrections, with the
   gradient from the adjoint kernel (``bp_project_gb300.autograd``) and L-BFGS.
@@ -110,19 +110,24 @@ def _projection(window: int, polyorder: int) -> np.ndarray:
 _SAVGOL_CACHE: dict = {}
 
 
+def _savgol_rows(n: int, window: int, polyorder: int, device):
+    """The projection's middle row and its first and last window // 2 rows, on ``device`` (cached)."""
+    if window % 2 != 1 or window > n or polyorder >= window:
+        raise ValueError("window must be odd, <= the signal length and > polyorder")
+    key = (window, polyorder, device)
+    if key not in _SAVGOL_CACHE:
+        h = _projection(window, polyorder)
+        half = window // 2
+        _SAVGOL_CACHE[key] = tuple(torch.from_numpy(np.ascontiguousarray(m)).to(device)
+                                   for m in (h[half], h[:half], h[window - half:]))
+    return _SAVGOL_CACHE[key]
+
+
 def savgol_smooth(x: torch.Tensor, window: int, polyorder: int) -> torch.Tensor:
     """Savitzky-Golay smoothing along dim 0 of [n, c] with polynomial fits at the edges
     (scipy.signal.savgol_filter, deriv 0, mode 'interp')."""
     n = x.shape[0]
-    if window % 2 != 1 or window > n or polyorder >= window:
-        raise ValueError("window must be odd, <= the signal length and > polyorder")
-    key = (window, polyorder, x.device)
-    if key not in _SAVGOL_CACHE:
-        h = _projection(window, polyorder)
-        half = window // 2
-        _SAVGOL_CACHE[key] = tuple(torch.from_numpy(np.ascontiguousarray(m)).to(x.device)
-                                   for m in (h[half], h[:half], h[window - half:]))
-    centre, left, right = _SAVGOL_CACHE[key]
+    centre, left, right = _savgol_rows(n, window, polyorder, x.device)
     half = window // 2
     out = torch.empty_like(x)
     out[half:n - half] = torch.einsum("icw,w->ic", x.unfold(0, window, 1), centre)
@@ -176,6 +181,22 @@ def estimate_update(data, pos, points, r_start, dr, k, prf, cutoff):
     n = p.shape[0]
     xi = core.target_contributions(d, p, pts, r_start, dr, k)
     smooth = sosfiltfilt(xi, butter_lowpass(cutoff, prf))
+    lib = nat.load()
+    if pts.shape[0] <= lib.sarbp_pga_max_targets():
+        t = int(pts.shape[0])
+        window = min(501, n // 2 * 2 - 1)
+        rows = _savgol_rows(n, window, 3, dev)
+        delta = torch.empty((n, 3), dtype=torch.float64, device=dev)
+        out = torch.empty((7,), dtype=torch.float64, device=dev)
+        nbytes = int(lib.sarbp_pga_update_workspace(t, n))
+        ws = torch.empty((nbytes,), dtype=torch.uint8, device=dev)
+        nat.check(lib.sarbp_pga_update(core._ptr(smooth), t, n, core._ptr(p), core._ptr(pts), float(k),
+                                       *(core._ptr(r) for r in rows), window, core._ptr(delta), core._ptr(out),
+                                       core._ptr(ws), nbytes, core.stream_handle()), "pga_update")
+        v = out.tolist()
+        return delta, dict(targets=t, cutoff_hz=cutoff, median_gradient_coherence=v[0], delta_rms_m=v[1:4],
+                           delta_max_m=v[4:])
+    # More targets than a block has threads: the same steps as tensor operations.
     cross = smooth[:, 1:] * smooth[:, :-1].conj()
     gradient = torch.angle(cross)
     amp = cross.abs()

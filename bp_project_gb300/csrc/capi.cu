@@ -551,6 +551,30 @@ int sarbp_sosfiltfilt(const float* x, int rows, int n, const double* sos, const 
                               (cudaStream_t)stream);
 }
 
+int sarbp_pga_max_targets(void) { return pga_max_targets(); }
+
+size_t sarbp_pga_update_workspace(int targets, int pulses) {
+    return targets > 0 && pulses > 0 ? pga_update_workspace(targets, pulses) : 0;
+}
+
+int sarbp_pga_update(const double* smooth, int targets, int pulses, const double* pos, const double* xyz, double k,
+                     const double* centre, const double* left, const double* right, int window, double* delta,
+                     double* stats, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!smooth || !pos || !xyz || !centre || !left || !right || !delta || !stats)
+        return fail(SARBP_ERR_TYPE, "arrays must be device pointers");
+    if (((uintptr_t)smooth & 15) || ((uintptr_t)workspace & 15))
+        return fail(SARBP_ERR_TYPE, "smooth and workspace must be 16-byte aligned");
+    if (targets < 1 || targets > pga_max_targets() || pulses < 2)
+        return fail(SARBP_ERR_VALUE, "1 to %d targets and at least two pulses are required", pga_max_targets());
+    if (window < 1 || window % 2 != 1 || window > pulses)
+        return fail(SARBP_ERR_VALUE, "window must be odd and at most the pulse count (got %d)", window);
+    if (!is_finite_value(k) || k == 0.0) return fail(SARBP_ERR_VALUE, "k must be finite and non-zero");
+    const size_t need = pga_update_workspace(targets, pulses);
+    if (!workspace || workspace_bytes < need) return fail(SARBP_ERR_WORKSPACE, "pga_update needs %zu workspace bytes", need);
+    return launch_pga_update(reinterpret_cast<const double2*>(smooth), targets, pulses, pos, xyz, k, centre, left, right,
+                             window, delta, stats, workspace, (cudaStream_t)stream);
+}
+
 int sarbp_tile_argmax(const float* magnitude, int nr, int nu, int nr_tiles, int nu_tiles, float* tile_max,
                       long long* tile_index, void* stream) {
     if (!magnitude || !tile_max || !tile_index) return fail(SARBP_ERR_TYPE, "magnitude, tile_max and tile_index must be device pointers");

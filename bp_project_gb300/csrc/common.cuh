@@ -272,6 +272,13 @@ int launch_rc_blocks(const float2* raw, int pulses, int samples, int taps, const
 int launch_decode_iq(const unsigned char* frames, int n, long long frame_size, int iq_offset, int nr, float2* out,
                      cudaStream_t s);
 
+// Trajectory update of the phase-gradient autofocus (trajectory.cu).
+int pga_max_targets();
+size_t pga_update_workspace(int targets, int pulses);
+int launch_pga_update(const double2* smooth, int targets, int pulses, const double* pos, const double* xyz, double k,
+                      const double* centre, const double* left, const double* right, int window, double* delta,
+                      double* stats, void* ws, cudaStream_t s);
+
 // Zero-phase IIR smoothing along rows (autofocus phase-history filter).
 size_t sosfiltfilt_workspace(int rows, int n, int padlen);
 int launch_tile_argmax(const float* a, int nr, int nu, int nr_tiles, int nu_tiles, float* tmax, long long* first,

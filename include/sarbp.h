@@ -300,6 +300,17 @@ int sarbp_sosfiltfilt(const float* x, int rows, int n, const double* sos, const 
                       const double* sos_host, int padlen, double* y, void* workspace, size_t workspace_bytes,
                       void* stream);
 
+/* Trajectory update of the phase-gradient autofocus (fast_bp/autofocus.py:40-79) from the smoothed target
+ * histories smooth (complex128 [targets, pulses]): delta float64 [pulses, 3] and stats float64 [7] (median
+ * gradient coherence, root mean square of delta's x, y, z, largest |x|, |y|, |z|).  centre [window], left
+ * and right [window / 2, window]: the rows of the Savitzky-Golay projection matrix.  1 <= targets <=
+ * sarbp_pga_max_targets(); window odd and <= pulses, pulses >= 2; workspace 16-byte aligned. */
+int sarbp_pga_max_targets(void);
+size_t sarbp_pga_update_workspace(int targets, int pulses);
+int sarbp_pga_update(const double* smooth, int targets, int pulses, const double* pos, const double* xyz, double k,
+                     const double* centre, const double* left, const double* right, int window, double* delta,
+                     double* stats, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Brightest cell of every tile of a magnitude image (float32 [nr, nu]) split into
  * nr_tiles x nu_tiles tiles as numpy.array_split does: tile_max float32 and
  * tile_index int64 (row-major flat index; ties to the smallest) per tile,
