@@ -2124,23 +2124,25 @@ struct PulseRec {
     float4 a;  // A_hi.x, A_hi.y, A_hi.z, frac(phase / 2pi)
     float4 b;  // A_lo.x, A_lo.y, A_lo.z, |pos - O|^2
     float4 c;  // (pos - O).x, .y, .z, weight
-    float4 d;  // the leaf's A quantum (a power of two), its inverse
+    float4 d;  // the leaf's A quantum (a power of two), its inverse, its largest |A| component and |A.x|
 };
 
 __device__ __forceinline__ void leaf_pulses(double K, const double* __restrict__ pos, const double* __restrict__ weight,
                                             const double* __restrict__ phase, const PolarDesc& g,
-                                            PulseRec* __restrict__ recs, int& amax) {
-    if (threadIdx.x == 0) amax = 0;
+                                            PulseRec* __restrict__ recs, int amax[2]) {
+    if (threadIdx.x < 2) amax[threadIdx.x] = 0;
     __syncthreads();
-    float m = 0.0f;
+    float m = 0.0f, mx = 0.0f;
     for (int n = g.a + threadIdx.x; n < g.b; n += blockDim.x) {
         const double ax = pos[3 * n] - g.ox, ay = pos[3 * n + 1] - g.oy, az = pos[3 * n + 2] - g.oz;
         m = fmaxf(m, (float)(fabs(K) * fmax(fabs(ax), fmax(fabs(ay), fabs(az)))));
+        mx = fmaxf(mx, (float)(fabs(K) * fabs(ax)));
     }
-    atomicMax(&amax, __float_as_int(m));  // non-negative floats order like their bit patterns
+    atomicMax(amax, __float_as_int(m));  // non-negative floats order like their bit patterns
+    atomicMax(amax + 1, __float_as_int(mx));
     __syncthreads();
     int e = 0;
-    frexp((double)__int_as_float(amax) * 1.0001 + 1e-30, &e);
+    frexp((double)__int_as_float(amax[0]) * 1.0001 + 1e-30, &e);
     const double scale = ldexp(1.0, e - 10), inv_scale = ldexp(1.0, 10 - e);
     for (int n = g.a + threadIdx.x; n < g.b; n += blockDim.x) {
         const double ax = pos[3 * n] - g.ox, ay = pos[3 * n + 1] - g.oy, az = pos[3 * n + 2] - g.oz;
@@ -2152,7 +2154,7 @@ __device__ __forceinline__ void leaf_pulses(double K, const double* __restrict__
         r.a.w = (float)(t - rint(t));
         r.b.w = (float)(ax * ax + ay * ay + az * az);
         r.c = make_float4((float)ax, (float)ay, (float)az, (float)weight[n]);
-        r.d = make_float4((float)scale, (float)inv_scale, 0.0f, 0.0f);
+        r.d = make_float4((float)scale, (float)inv_scale, __int_as_float(amax[0]), __int_as_float(amax[1]));
         recs[n] = r;
     }
 }
@@ -2160,7 +2162,7 @@ __device__ __forceinline__ void leaf_pulses(double K, const double* __restrict__
 __global__ void ffbp_leaf_pulses_kernel(double K, const double* __restrict__ pos, const double* __restrict__ weight,
                                         const double* __restrict__ phase, const PolarDesc* __restrict__ nodes,
                                         const int* __restrict__ leaves, PulseRec* __restrict__ recs) {
-    __shared__ int amax;
+    __shared__ int amax[2];
     leaf_pulses(K, pos, weight, phase, nodes[leaves[blockIdx.x]], recs, amax);
 }
 
@@ -2177,36 +2179,56 @@ __global__ void ffbp_leaf_pulses_kernel(double K, const double* __restrict__ pos
 // with C and D once per (pulse, tile column).  The phase's large part alpha_hi D_hi + beta_hi
 // A_hi.z is exact in FP32: alpha_hi and beta_hi are multiples of 2^-11 (11 bits), D_hi and
 // A_hi.z multiples of the leaf's A quantum below 2^10.5 quanta, so each product has at most 22
-// bits and their sum 23.  A thread's four pixels share the tile column and run as two pairs
-// of f32x2 lanes.
+// bits and their sum 23.
+//
+// A thread's pixels are a run of eight columns of one tile row.  Along a run the range hardly
+// changes (the angle step is chosen so that the phase turns by a fraction of a turn per column:
+// millimetres), so everything but the rotation is worked out once per pulse for the run's middle,
+// half-way between its fourth and fifth column, with the derivatives in the column offset
+// m = -3.5 ... 3.5:
+//   C(m) = C + C_1 m + ... + C_4 m^4 (s(u) expanded at the middle; D_j likewise, in radians),
+//   d(m)^2 = r^2 + |a|^2 - 2 r (alpha C(m) + beta a.z),   so with t = r / d and z = 1 / (2 pi K d)
+//   P_1 = t alpha D_1,  P_2 = t alpha D_2 - z P_1^2 / 2,  P_3 = t alpha D_3 - z P_1 P_2,
+//   P_4 = t alpha D_4 - z (P_1 P_3 + P_2^2 / 2)            are the phase's coefficients (radians).
+// The pulse's sample along the run is the window entry's cubic in d, a cubic in m as long as the
+// whole run stays within one range bin; when that holds for all 32 rows of the warp the run takes
+// one window entry (two 16-byte loads instead of sixteen) and the even and odd parts of both
+// polynomials serve the columns +m and -m.  Otherwise each pixel takes its own entry.
+// What bounds it: instruction issue (74% of the cycles; 295 instructions per warp and pulse, a quarter of
+// them windows and records).  4096 pulses in 256 leaves of 16 (1.46 G pixel-pulses): 1.68 ms, with a pixel
+// pair per thread and step 2.47; with every pixel on its own window entry 2.15.  Six blocks per SM (80
+// registers): with five, seven and eight 1.70, 1.73 and 1.82 ms.
 struct LeafRec {
-    float4 p0;  // (a.z, a.z), (-|a|^2, -|a|^2)
-    float4 p1;  // (A_hi.z, A_hi.z), (A_lo.z, A_lo.z)
-    float4 p2;  // (A.z, A.z), (Phi, Phi)
-    int4 w;     // window bias bits, window offset, window count - 1, unused
+    float4 p0;  // a.z, -|a|^2, A_hi.z, A_lo.z
+    float4 p1;  // Phi, and as bits: window byte bias, byte offset of the window, of its last entry in it
 };
 
+// One pulse at the middle of one run of columns.
 struct LeafCol {
-    float4 p0;  // (C, C), (D_hi, D_hi)
-    float4 p1;  // (D_lo, D_lo), (D, D)
+    float4 p0;  // C, D_hi, D_lo, D
+    float4 p1;  // 2 pi D_1 ... 2 pi D_4
 };
 
-constexpr int kLeafColStride = 32;  // LeafCol entries per pulse: the widest leaf tile
+// The middle of a run of columns: (s, u) as float pairs, s's derivatives s_j = s^(j)(u) du^j / j!.
+struct LeafMid {
+    float4 cv;
+    float s1, s2, s3, s4;
+    float du;
+    float lim;  // half a bin, or below 0: the run's pixels take their own window entries
+    int runs;   // the expansion holds for the leaf's pulses
+    int pad;
+};
 
+constexpr int kLeafRun = 8;                                   // columns per thread
+constexpr int kLeafThreads = kSplitTilePixels / kLeafRun;
+constexpr int kLeafGroups = kMaxCols / kLeafRun;              // runs per tile row, at most
+constexpr int kLeafCtas = 6;                                  // per SM, by registers and by the window budget
+constexpr int kLeafWindowBudget = 35 * 1024;
 __host__ __device__ constexpr size_t leaf_col_offset() { return (size_t)kMaxLeafChunk * sizeof(LeafRec); }
-__host__ __device__ constexpr size_t leaf_window_offset(int chunk) {
-    return leaf_col_offset() + (size_t)chunk * kLeafColStride * sizeof(LeafCol);
+__host__ __device__ constexpr size_t leaf_mid_offset() {
+    return leaf_col_offset() + (size_t)kMaxLeafChunk * kLeafGroups * sizeof(LeafCol);
 }
-
-// Two pixels of one tile column (the lanes), rows (row0, row1).
-struct LPair {
-    float2 na, nb;  // -alpha, -beta
-    float2 ah, al;  // alpha = ah + al, ah a multiple of 2^-11
-    float2 bh, bl;  // beta = bh + bl
-    float2 r2, fm;  // 2 r, frac(Q) - 1/2 with Q = (r - range_start) / data_dr
-    float2 ar, ai;  // accumulated image, real and imaginary parts
-    int o0, o1;     // floor(Q) - I_first
-};
+__host__ __device__ constexpr size_t leaf_window_offset() { return leaf_mid_offset() + kLeafGroups * sizeof(LeafMid); }
 
 constexpr float kUnitQ = 1.0f / 2048.0f;  // quantum of unit-vector components (11 bits)
 
@@ -2216,100 +2238,30 @@ __device__ __forceinline__ void unit_split(float p, float e, float& h, float& l,
     full = p + e;
 }
 
-// The row values of pixel row i (tables: (g/r, -oz/r) as float pairs, (2r, frac(Q) - 1/2, floor(Q))).
-__device__ __forceinline__ void leaf_row(const PolarDesc& g, const float4* __restrict__ tables, int i, int I_first,
-                                         float& na, float& nb, float& ah, float& al, float& bh, float& bl, float& r2,
-                                         float& fm, int& o) {
+// The values of one pixel row i (tables: (g/r, -oz/r) as float pairs, (2r, frac(Q) - 1/2, floor(Q))).
+struct LeafRow {
+    float a, b;    // alpha, beta
+    float ah, al;  // alpha = ah + al, ah a multiple of 2^-11
+    float bh, bl;  // beta = bh + bl
+    float r2, fm;  // 2 r, frac(Q) - 1/2 with Q = (r - range_start) / data_dr
+    int o;         // floor(Q) - I_first
+};
+
+__device__ __forceinline__ LeafRow leaf_row(const PolarDesc& g, const float4* __restrict__ tables, int i, int I_first) {
     const float4 r1 = __ldg(tables + g.rows_off + 3 * (long long)i + 1);
     const float4 rq = __ldg(tables + g.rows_off + 3 * (long long)i + 2);
-    float a, b;
-    unit_split(r1.x, r1.y, ah, al, a);
-    unit_split(r1.z, r1.w, bh, bl, b);
-    na = -a;
-    nb = -b;
-    r2 = rq.x;
-    fm = rq.y;
-    o = __float_as_int(rq.z) - I_first;
+    LeafRow q;
+    unit_split(r1.x, r1.y, q.ah, q.al, q.a);
+    unit_split(r1.z, r1.w, q.bh, q.bl, q.b);
+    q.r2 = rq.x;
+    q.fm = rq.y;
+    q.o = __float_as_int(rq.z) - I_first;
+    return q;
 }
 
-// One pixel's windowed sample (the reference's cubic, weight folded in) at bin index bits tq and
-// centred fraction s; with no fitting window the taps come straight from the pulse row.
-template <bool STAGED>
-__device__ __forceinline__ float2 leaf_sample(const float4* wrow, unsigned last, int bias, float tq,
-                                              float s, int o, const float2* drow, int I_first, int samples, float wt) {
-    float2 v;
-    if (STAGED) {
-        const unsigned j = min((unsigned)(__float_as_int(tq) + o - bias), last);
-        const float4 c01 = wrow[2 * j], c23 = wrow[2 * j + 1];
-        const float2 sp = pair(s);
-        v = __ffma2_rn(make_float2(c23.z, c23.w), sp, make_float2(c23.x, c23.y));
-        v = __ffma2_rn(v, sp, make_float2(c01.z, c01.w));
-        v = __ffma2_rn(v, sp, make_float2(c01.x, c01.y));
-    } else {  // the pulse's window does not fit: gather its taps directly
-        const long long gb = (long long)(__float_as_int(tq) - kMagicBits) + o + I_first;
-        v = make_float2(0.0f, 0.0f);
-        if (gb >= 1 && gb <= (long long)samples - 3) {
-            float w[4];
-            lagrange_centred(s, w);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const float2 x = __ldg(drow + gb + b - 1);
-                v.x = fmaf(w[b], x.x, v.x);
-                v.y = fmaf(w[b], x.y, v.y);
-            }
-            v.x *= wt;
-            v.y *= wt;
-        }
-    }
-    return v;
-}
-
-// One pulse on one pixel pair: range, window sample, phase and the accumulation.
-template <bool STAGED>
-__device__ __forceinline__ void leaf_pair_pulse(LPair& q, const LeafRec& R, const LeafCol& Cc, const float4* wrow, unsigned last, int bias, const float2* drow,
-                                                int I_first, int samples, float wt, float2 nKf, float2 ninv_dr) {
-    const float2 magic = pair(kMagic), nmagic = pair(-kMagic), mone = pair(-1.0f);
-    const float2 az = make_float2(R.p0.x, R.p0.y), naa = make_float2(R.p0.z, R.p0.w);
-    const float2 C = make_float2(Cc.p0.x, Cc.p0.y);
-    const float2 nL = __ffma2_rn(q.na, C, __fmul2_rn(q.nb, az));  // -L
-    const float2 nq2 = __ffma2_rn(nL, nL, naa);                    // -(|a|^2 - L^2)
-    const float2 den = __ffma2_rn(pair(2.0f), nL, q.r2);           // 2 (r - L)
-    const float2 B = make_float2(rcp_approx(den.x), rcp_approx(den.y));
-    const float2 ne0 = __fmul2_rn(nq2, B);
-    const float2 neps = __ffma2_rn(__fmul2_rn(ne0, ne0), B, ne0);  // -eps (second order: leaves are wide)
-    const float2 qp = __ffma2_rn(__ffma2_rn(nL, mone, neps), ninv_dr, q.fm);
-    const float2 tq = __fadd2_rn(qp, magic);
-    const float2 s = __ffma2_rn(__fadd2_rn(tq, nmagic), mone, qp);
-    // Phase (turns): the exact part, then the small terms.
-    const float2 tb = __ffma2_rn(q.ah, make_float2(Cc.p0.z, Cc.p0.w), __fmul2_rn(q.bh, make_float2(R.p1.x, R.p1.y)));
-    float2 sm = __ffma2_rn(nKf, neps, make_float2(R.p2.z, R.p2.w));
-    sm = __ffma2_rn(q.ah, make_float2(Cc.p1.x, Cc.p1.y), sm);
-    sm = __ffma2_rn(q.al, make_float2(Cc.p1.z, Cc.p1.w), sm);
-    sm = __ffma2_rn(q.bh, make_float2(R.p1.z, R.p1.w), sm);
-    sm = __ffma2_rn(q.bl, make_float2(R.p2.x, R.p2.y), sm);
-    // The reduced exact term is in [-1/2, 1/2] turn and |sm| <= 1 + K eps (eps is second order in
-    // the pulse's offset from the leaf centre), so the angle stays within a few turns, which the
-    // hardware sin/cos reduce themselves.
-    const float2 rtb = __fadd2_rn(__fadd2_rn(tb, magic), nmagic);
-    const float2 ang = __fmul2_rn(__fadd2_rn(__ffma2_rn(rtb, mone, tb), sm), pair(kTwoPiF));
-    float sn0, cs0, sn1, cs1;
-    __sincosf(ang.x, &sn0, &cs0);
-    __sincosf(ang.y, &sn1, &cs1);
-    const float2 v0 = leaf_sample<STAGED>(wrow, last, bias, tq.x, s.x, q.o0, drow, I_first, samples, wt);
-    const float2 v1 = leaf_sample<STAGED>(wrow, last, bias, tq.y, s.y, q.o1, drow, I_first, samples, wt);
-    q.ar.x = fmaf(v0.x, cs0, q.ar.x);
-    q.ar.x = fmaf(-v0.y, sn0, q.ar.x);
-    q.ai.x = fmaf(v0.x, sn0, q.ai.x);
-    q.ai.x = fmaf(v0.y, cs0, q.ai.x);
-    q.ar.y = fmaf(v1.x, cs1, q.ar.y);
-    q.ar.y = fmaf(-v1.y, sn1, q.ar.y);
-    q.ai.y = fmaf(v1.x, sn1, q.ai.y);
-    q.ai.y = fmaf(v1.y, cs1, q.ai.y);
-}
-
-// C and D of one (pulse, tile column) from the pulse record and the column table (c, u pairs):
-// D in two-float, split on the leaf's A quantum.
-__device__ __forceinline__ LeafCol leaf_col(const PulseRec& pr, float4 cv, float side) {
+// C and D of one (pulse, column) from the pulse record and the column's (c, u) pairs: D in
+// two-float, split on the leaf's A quantum.
+__device__ __forceinline__ float4 leaf_col(const PulseRec& pr, float4 cv, float side) {
     const float sh = side * cv.x, sl = side * cv.y, uh = cv.z, ul = cv.w;
     const float C = fmaf(sh, pr.c.x, uh * pr.c.y);
     const float p1 = sh * pr.a.x, e1 = fmaf(sh, pr.a.x, -p1);
@@ -2323,10 +2275,188 @@ __device__ __forceinline__ LeafCol leaf_col(const PulseRec& pr, float4 cv, float
     rest = fmaf(ul, pr.a.y, rest);
     const float Dh = rintf(S * pr.d.y) * pr.d.x;  // the A quantum is a power of two: exact
     const float Dl = (S - Dh) + rest;             // S - Dh is exact (|S - Dh| <= quantum / 2)
-    LeafCol L;
-    L.p0 = make_float4(C, C, Dh, Dh);
-    L.p1 = make_float4(Dl, Dl, S + rest, S + rest);
-    return L;
+    return make_float4(C, Dh, Dl, S + rest);
+}
+
+// The run of columns from column j0 (window columns; the middle is j0 + 3.5), for pulses with
+// largest |A| component amax and |A.x| axmax (turns) at ranges from r_min.
+__device__ __forceinline__ LeafMid leaf_mid(const SplitParams& P, const PolarDesc& g, int j0, float r_min, float amax,
+                                            float axmax) {
+    const FF u = ff_add(ff_of(g.tf[5]), ff_mul(FF{(float)j0 + 0.5f * (kLeafRun - 1), 0.0f}, ff_of(g.tf[6])));
+    const FF c = ff_sqrt0(ff_add(FF{1.0f, 0.0f}, ff_neg(ff_sqr(u))));
+    const float h = g.tf[6].x + g.tf[6].y, uf = u.h, ic = 1.0f / c.h, hc = h * ic, u2 = uf * uf;
+    LeafMid M;
+    M.cv = make_float4(c.h, c.l, u.h, u.l);
+    const float side = (float)g.side;
+    // c = sqrt(1 - u^2): c' = -u / c, c'' = -1 / c^3, c''' = -3 u / c^5, c'''' = -3 (1 + 4 u^2) / c^7.
+    M.s1 = side * -uf * hc;
+    M.s2 = side * -0.5f * hc * hc * ic;
+    M.s3 = M.s2 * uf * hc * ic;
+    M.s4 = M.s2 * 0.25f * (1.0f + 4.0f * u2) * (hc * ic) * (hc * ic);
+    M.du = h;
+    // What the expansion leaves out: the fifth and sixth order of s, and the fifth of the root.
+    const float m = 0.5f * (kLeafRun - 1), m2 = m * m;
+    const float q5 = fabsf(M.s4 * uf) * (hc * ic) * (3.0f + 4.0f * u2) / (1.0f + 4.0f * u2);
+    const float q6 = fabsf(M.s4) * (hc * ic) * (hc * ic) * 0.5f * (1.0f + 12.0f * u2 + 8.0f * u2 * u2) / (1.0f + 4.0f * u2);
+    const float ir = 1.0f / r_min, turn = m * hc * 1.5f * amax, y = turn * ir / fabsf(P.Kf);
+    const float rest = axmax * m2 * m2 * m * (q5 + m * q6) + turn * (y * y) * (y * y);
+    M.runs = rest <= 5e-8f ? 1 : 0;
+    // The sample's cubic in m leaves out the square of the quadratic term.
+    const float kb = fabsf(P.inv_drf / P.Kf);
+    const float x1 = turn * kb, x2 = m2 * (axmax * fabsf(M.s2)) * kb + 0.5f * turn * y * kb;
+    M.lim = (3.0f * x1 * x1 + x2) * x2 <= 1e-7f ? 0.5f : -1.0f;
+    M.pad = 0;
+    return M;
+}
+
+// The pulses of a chunk on one run.
+__device__ __forceinline__ void leaf_runs(const SplitParams& P, const LeafRec* __restrict__ rec,
+                                          const LeafCol* __restrict__ cols, const char* __restrict__ win, int n,
+                                          const LeafRow& q, float lim, float ar[kLeafRun], float ai[kLeafRun]) {
+    const float inv_dr = P.inv_drf, Kf = P.Kf;
+    const float kz = 1.0f / (kTwoPiF * Kf), kd = inv_dr * kz;
+#pragma unroll 1
+    for (int nl = 0; nl < n; ++nl) {
+        const float4 ra = rec[nl].p0, rb = rec[nl].p1;
+        const float4 ca = cols[nl * kLeafGroups].p0, cb = cols[nl * kLeafGroups].p1;
+        const float L = fmaf(q.a, ca.x, q.b * ra.x);
+        const float nq2 = fmaf(L, L, ra.y);                 // -(|a|^2 - L^2)
+        const float B = rcp_approx(fmaf(-2.0f, L, q.r2));   // 1 / (2 (r - L))
+        const float ne0 = nq2 * B;
+        const float neps = fmaf(ne0 * ne0, B, ne0);
+        const float dd = -L - neps;                          // d - r
+        const float iR = rcp_approx(fmaf(0.5f, q.r2, dd));
+        const float at = q.a * fmaf(-dd, iR, 1.0f);          // alpha r / d
+        // Phase at the middle (turns): the exact part, then the small terms.
+        const float tb = fmaf(q.ah, ca.y, q.bh * ra.z);
+        float sm = fmaf(-Kf, neps, rb.x);
+        sm = fmaf(q.ah, ca.z, sm);
+        sm = fmaf(q.al, ca.w, sm);
+        sm = fmaf(q.bh, ra.w, sm);
+        sm = fmaf(q.bl, ra.z + ra.w, sm);
+        const float P0 = ((tb - round_magic(tb)) + sm) * kTwoPiF;
+        const float z = iR * kz;
+        const float P1 = at * cb.x;
+        const float y1 = z * P1;
+        const float P2 = fmaf(-0.5f * P1, y1, at * cb.y);
+        const float P3 = fmaf(-y1, P2, at * cb.z);
+        const float P4 = fmaf(-y1, P3, fmaf(-0.5f * z * P2, P2, at * cb.w));
+        // Place in the window at the middle, and its slope and curvature (bins).
+        const float qp = fmaf(dd, inv_dr, q.fm);
+        const float tq = qp + kMagic;
+        const float s = qp - (tq - kMagic);
+        const float b1 = P1 * kd, b2 = P2 * kd;
+        const unsigned bias = 32u * (unsigned)q.o + (unsigned)__float_as_int(rb.y), last = (unsigned)__float_as_int(rb.w);
+        const char* w0 = win + __float_as_int(rb.z);
+        const float spread = fmaf(fabsf(b2), 12.25f, fmaf(fabsf(b1), 3.5f, fabsf(s)));
+        if (__all_sync(0xffffffffu, spread <= lim)) {
+            const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(tq) + bias, last));
+            const float4 c01 = w[0], c23 = w[1];
+            float V0[2], V1[2], V2[2], V3[2];
+            const float bb = b1 * b1;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float A0 = c ? c01.y : c01.x, A1 = c ? c01.w : c01.z, A2 = c ? c23.y : c23.x, A3 = c ? c23.w : c23.z;
+                const float T = A3 * s;
+                const float W1 = A2 + T, W2 = fmaf(3.0f, T, A2);
+                const float V = fmaf(W1, s, A1);               // the sample is A0 + V s
+                const float D = fmaf(A2 + W2, s, A1);         // its derivative
+                V0[c] = fmaf(V, s, A0);
+                V1[c] = D * b1;
+                V2[c] = fmaf(W2, bb, D * b2);
+                V3[c] = fmaf(A3, bb, 2.0f * W2 * b2) * b1;
+            }
+#pragma unroll
+            for (int h = 0; h < kLeafRun / 2; ++h) {
+                const float m = 0.5f + h, mm = m * m;
+                const float ae = fmaf(fmaf(P4, mm, P2), mm, P0), ao = fmaf(P3, mm, P1);
+                const float re = fmaf(V2[0], mm, V0[0]), ro = fmaf(V3[0], mm, V1[0]);
+                const float ie = fmaf(V2[1], mm, V0[1]), io = fmaf(V3[1], mm, V1[1]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int k = c ? kLeafRun / 2 + h : kLeafRun / 2 - 1 - h;
+                    const float x = c ? m : -m;
+                    const float vr = fmaf(ro, x, re), vi = fmaf(io, x, ie);
+                    float sn, cs;
+                    __sincosf(fmaf(ao, x, ae), &sn, &cs);
+                    ar[k] = fmaf(vr, cs, ar[k]);
+                    ar[k] = fmaf(-vi, sn, ar[k]);
+                    ai[k] = fmaf(vr, sn, ai[k]);
+                    ai[k] = fmaf(vi, cs, ai[k]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kLeafRun; ++k) {
+                const float x = (float)k - 0.5f * (kLeafRun - 1);
+                const float p = fmaf(fmaf(b2, x, b1), x, qp);
+                const float t = p + kMagic, f = p - (t - kMagic);
+                const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(t) + bias, last));
+                const float4 c01 = w[0], c23 = w[1];
+                const float vr = fmaf(fmaf(fmaf(c23.z, f, c23.x), f, c01.z), f, c01.x);
+                const float vi = fmaf(fmaf(fmaf(c23.w, f, c23.y), f, c01.w), f, c01.y);
+                float sn, cs;
+                __sincosf(fmaf(fmaf(fmaf(fmaf(P4, x, P3), x, P2), x, P1), x, P0), &sn, &cs);
+                ar[k] = fmaf(vr, cs, ar[k]);
+                ar[k] = fmaf(-vi, sn, ar[k]);
+                ai[k] = fmaf(vr, sn, ai[k]);
+                ai[k] = fmaf(vi, cs, ai[k]);
+            }
+        }
+    }
+}
+
+// n pulses from c0 on the run's pixels one by one, with the taps from the pulse rows: pulses whose
+// window does not fit, and columns too wide for the expansion (both rare, hence out of line).
+__device__ __noinline__ void leaf_direct(const SplitParams& P, const PolarDesc* __restrict__ node,
+                                         const float4* __restrict__ tables, const PulseRec* __restrict__ precs, int i, int j0, int c0, int n,
+                                         float2* __restrict__ more) {
+    const PolarDesc& g = *node;
+    const float side = (float)g.side;
+    const LeafRow q = leaf_row(g, tables, i, 0);
+#pragma unroll 1
+    for (int k = 0; k < kLeafRun; ++k) {
+        const float4 cv = __ldg(tables + g.cols_off + min(j0 + k, g.nu - 1));
+        float sr = 0.0f, si = 0.0f;
+#pragma unroll 1
+        for (int nl = c0; nl < c0 + n; ++nl) {
+            const PulseRec pr = precs[nl];
+            const float4 cd = leaf_col(pr, cv, side);
+            const float L = fmaf(q.a, cd.x, q.b * pr.c.z);
+            const float nq2 = fmaf(L, L, -pr.b.w);
+            const float B = rcp_approx(fmaf(-2.0f, L, q.r2));
+            const float ne0 = nq2 * B;
+            const float neps = fmaf(ne0 * ne0, B, ne0);
+            const float qp = fmaf(-L - neps, P.inv_drf, q.fm);
+            const float t = qp + kMagic, f = qp - (t - kMagic);
+            const long long gb = (long long)(__float_as_int(t) - kMagicBits) + q.o;
+            if (!(gb >= 1 && gb <= (long long)P.in.samples - 3)) continue;
+            const float2* row = P.in.data + (size_t)nl * P.in.samples + gb - 1;
+            float w[4], vr = 0.0f, vi = 0.0f;
+            lagrange_centred(f, w);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float2 x = __ldg(row + b);
+                vr = fmaf(w[b], x.x, vr);
+                vi = fmaf(w[b], x.y, vi);
+            }
+            vr *= pr.c.w;
+            vi *= pr.c.w;
+            const float tb = fmaf(q.ah, cd.y, q.bh * pr.a.z);
+            float sm = fmaf(-P.Kf, neps, pr.a.w);
+            sm = fmaf(q.ah, cd.z, sm);
+            sm = fmaf(q.al, cd.w, sm);
+            sm = fmaf(q.bh, pr.b.z, sm);
+            sm = fmaf(q.bl, pr.a.z + pr.b.z, sm);
+            float sn, cs;
+            __sincosf(((tb - round_magic(tb)) + sm) * kTwoPiF, &sn, &cs);
+            sr = fmaf(vr, cs, sr);
+            sr = fmaf(-vi, sn, sr);
+            si = fmaf(vr, sn, si);
+            si = fmaf(vi, cs, si);
+        }
+        more[k] = make_float2(sr, si);
+    }
 }
 
 // One leaf tile: the per-item body of the leaf kernels.  precs holds the pulse records of
@@ -2336,32 +2466,33 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
                                           float2* __restrict__ arena, float2* root_out, int root, char* smem,
                                           int* s_base, float* s_wt, int& s_nfit) {
     const PolarDesc g = nodes[it.node];
-    const int lc = g.tile_lc, cols_t = 1 << lc, rows_t = kSplitTilePixels >> lc;
+    const int lc = g.tile_lc, rows_t = kSplitTilePixels >> lc;  // 32 rows or more: a warp has one run of columns
+    const int groups = (1 << lc) / kLeafRun;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int col = tid & (cols_t - 1);
+    const int row = tid & (rows_t - 1), group = tid / rows_t;
     const int ifirst = min(g.win_r0 + it.tile_r, g.nr - 1);
     const int ilast = min(g.win_r0 + it.tile_r + rows_t - 1, g.nr - 1);
     const float4 rfirst = __ldg(tables + g.rows_off + 3 * (long long)ifirst + 2);
     const int I_first = __float_as_int(rfirst.z);
     const int I_span = __float_as_int(__ldg(tables + g.rows_off + 3 * (long long)ilast + 2).z) - I_first;
     const float r_min = 0.5f * rfirst.x;
-    // Pixel k of this thread is row (tid >> lc) + k (256 >> lc) of its column; pairs (0, 1), (2, 3).
-    LPair px[2];
+    const int ipix = min(g.win_r0 + it.tile_r + row, g.nr - 1);
+    const int jpix = g.win_u0 + it.tile_u + kLeafRun * group;
+    const LeafRow q = leaf_row(g, tables, ipix, I_first);
+    float ar[kLeafRun], ai[kLeafRun];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        LPair& q = px[h];
-        const int i0 = min(g.win_r0 + it.tile_r + (tid >> lc) + (kThreads >> lc) * (2 * h), g.nr - 1);
-        const int i1 = min(g.win_r0 + it.tile_r + (tid >> lc) + (kThreads >> lc) * (2 * h + 1), g.nr - 1);
-        leaf_row(g, tables, i0, I_first, q.na.x, q.nb.x, q.ah.x, q.al.x, q.bh.x, q.bl.x, q.r2.x, q.fm.x, q.o0);
-        leaf_row(g, tables, i1, I_first, q.na.y, q.nb.y, q.ah.y, q.al.y, q.bh.y, q.bl.y, q.r2.y, q.fm.y, q.o1);
-        q.ar = q.ai = make_float2(0.0f, 0.0f);
-    }
+    for (int k = 0; k < kLeafRun; ++k) ar[k] = ai[k] = 0.0f;
     LeafRec* rec = reinterpret_cast<LeafRec*>(smem);
     LeafCol* cols = reinterpret_cast<LeafCol*>(smem + leaf_col_offset());
-    float4* win = reinterpret_cast<float4*>(smem + leaf_window_offset(P.chunk));
+    LeafMid* mids = reinterpret_cast<LeafMid*>(smem + leaf_mid_offset());
+    float4* win = reinterpret_cast<float4*>(smem + leaf_window_offset());
     const PulseInputs& in = P.in;
-    const float2 nKf = pair(-P.Kf), ninv_dr = pair(-P.inv_drf);
     const float side = (float)g.side;
+    __syncthreads();  // a persistent block's last tile may still read its runs' middles
+    if (lane == 0 && row == 0) {
+        const float4 pd = precs[g.a].d;
+        mids[group] = leaf_mid(P, g, jpix, r_min, pd.z, pd.w);
+    }
     for (int c0 = g.a; c0 < g.b;) {
         const int want = min(P.chunk, g.b - c0);
         __syncthreads();
@@ -2374,15 +2505,13 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
                 const float hw = (amag + eps_max) * fabsf(P.inv_drf) + 1e-3f;
                 const int bo = (int)floorf(-0.5f - hw), top = (int)ceilf(0.5f + hw);
                 const long long cnt = (long long)I_span + top - bo + 1;
-                count = cnt <= P.cap ? (int)cnt : P.cap + 1;
+                count = hw < 1e6f && cnt <= P.cap ? (int)cnt : P.cap + 1;
                 s_base[lane] = I_first + bo;
                 s_wt[lane] = pr.c.w;
                 LeafRec r;
-                r.p0 = make_float4(pr.c.z, pr.c.z, -pr.b.w, -pr.b.w);
-                r.p1 = make_float4(pr.a.z, pr.a.z, pr.b.z, pr.b.z);
-                const float Az = pr.a.z + pr.b.z;
-                r.p2 = make_float4(Az, Az, pr.a.w, pr.a.w);
-                r.w = make_int4(kMagicBits + bo, 0, count - 1, 0);
+                r.p0 = make_float4(pr.c.z, -pr.b.w, pr.a.z, pr.b.z);
+                r.p1 = make_float4(pr.a.w, __int_as_float((int)(0u - 32u * (unsigned)(kMagicBits + bo))), 0.0f,
+                                   __int_as_float(32 * (count - 1)));
                 rec[lane] = r;
             }
             int inc = count;
@@ -2392,63 +2521,61 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
                 if (lane >= o) inc += v;
             }
             const unsigned fits = __ballot_sync(0xffffffffu, lane < want && inc <= P.cap);
-            if (lane < want) rec[lane].w.y = inc - count;
+            if (lane < want) rec[lane].p1.z = __int_as_float(32 * (inc - count));
             if (lane == 0) s_nfit = __popc(fits);
         }
         __syncthreads();
         const int nfit = s_nfit;
         const int chn = nfit > 0 ? nfit : 1;
-        for (int e = tid; e < (chn << lc); e += kThreads) {  // C, D per (pulse, column)
-            const int nl = e >> lc, cc = e & (cols_t - 1);
-            const float4 cv = __ldg(tables + g.cols_off + min(g.win_u0 + it.tile_u + cc, g.nu - 1));
-            cols[nl * kLeafColStride + cc] = leaf_col(precs[c0 + nl], cv, side);
+        const LeafMid& M = mids[group];
+        const bool runs = M.runs != 0 && nfit > 0;
+        for (int e = tid; e < nfit * groups; e += kLeafThreads) {  // one (pulse, run of columns) each
+            const int nl = e / groups, gi = e - nl * groups;
+            const LeafMid& m = mids[gi];
+            const PulseRec pr = precs[c0 + nl];
+            const float Ax = (pr.a.x + pr.b.x) * kTwoPiF, Ay = (pr.a.y + pr.b.y) * kTwoPiF;
+            LeafCol& o = cols[nl * kLeafGroups + gi];
+            o.p0 = leaf_col(pr, m.cv, side);
+            o.p1 = make_float4(fmaf(Ax, m.s1, Ay * m.du), Ax * m.s2, Ax * m.s3, Ax * m.s4);
         }
-        if (nfit > 0) {
-            for (int nl = warp; nl < nfit; nl += kThreads / 32) {
-                const int off = rec[nl].w.y;
-                const int cnt = rec[nl].w.z + 1;
-                const long long b0 = s_base[nl];
-                const float a = s_wt[nl];
-                const float2* row = in.data + (size_t)(c0 + nl) * in.samples;
-                stage_window_shfl(row, in.samples, b0, cnt, a, win + 2 * off, lane);
-            }
+        for (int nl = warp; nl < nfit; nl += kLeafThreads / 32) {
+            const float2* drow = in.data + (size_t)(c0 + nl) * in.samples;
+            stage_window_shfl(drow, in.samples, s_base[nl], __float_as_int(rec[nl].p1.w) / 32 + 1, s_wt[nl],
+                              win + __float_as_int(rec[nl].p1.z) / 16, lane);
         }
         __syncthreads();
-        if (nfit > 0) {
-#pragma unroll 1
-            for (int nl = 0; nl < nfit; ++nl) {
-                const LeafRec R = rec[nl];
-                const LeafCol Cc = cols[nl * kLeafColStride + col];
-                const float4* wrow = win + 2 * R.w.y;
+        if (runs) {
+            leaf_runs(P, rec, cols + group, reinterpret_cast<const char*>(win), nfit, q, M.lim, ar, ai);
+        } else {
+            float2 more[kLeafRun];
+            leaf_direct(P, nodes + it.node, tables, precs, ipix, jpix, c0, chn, more);
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    leaf_pair_pulse<true>(px[h], R, Cc, wrow, (unsigned)R.w.z, R.w.x, nullptr, I_first, in.samples, 0.0f,
-                                          nKf, ninv_dr);
+            for (int k = 0; k < kLeafRun; ++k) {
+                ar[k] += more[k].x;
+                ai[k] += more[k].y;
             }
-        } else {  // one pulse whose window does not fit: its taps come straight from the pulse row
-            const LeafRec R = rec[0];
-            const LeafCol Cc = cols[col];
-            const float2* drow = in.data + (size_t)c0 * in.samples;
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                leaf_pair_pulse<false>(px[h], R, Cc, nullptr, 0u, 0, drow, I_first, in.samples, s_wt[0], nKf, ninv_dr);
         }
         c0 += chn;
     }
+    // Each warp holds 32 rows of eight columns: 64 bytes of a row per thread, as float4 where the
+    // image's rows are 16-byte aligned.
     float2* dst = g.dst ? g.dst : (it.node == root ? root_out : arena + g.out_offset);
-    const int wu = it.tile_u + col;
+    const int wr = it.tile_r + row, wu = it.tile_u + kLeafRun * group;
+    if (wr < g.win_nr && wu < g.win_nu) {
+        float2* p = dst + (long long)wr * g.out_stride + wu;
+        if (wu + kLeafRun <= g.win_nu && (reinterpret_cast<unsigned long long>(p) & 15) == 0) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int wr0 = it.tile_r + (tid >> lc) + (kThreads >> lc) * (2 * h);
-        const int wr1 = wr0 + (kThreads >> lc);
-        if (wu < g.win_nu) {
-            if (wr0 < g.win_nr) dst[(long long)wr0 * g.out_stride + wu] = make_float2(px[h].ar.x, px[h].ai.x);
-            if (wr1 < g.win_nr) dst[(long long)wr1 * g.out_stride + wu] = make_float2(px[h].ar.y, px[h].ai.y);
+            for (int k = 0; k < kLeafRun; k += 2)
+                reinterpret_cast<float4*>(p)[k / 2] = make_float4(ar[k], ai[k], ar[k + 1], ai[k + 1]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kLeafRun; ++k)
+                if (wu + k < g.win_nu) p[k] = make_float2(ar[k], ai[k]);
         }
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
+__global__ void __launch_bounds__(kLeafThreads, kLeafCtas) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
                                                                  const TileItem* __restrict__ items,
                                                                  const float4* __restrict__ tables,
                                                                  const PulseRec* __restrict__ precs,
@@ -3195,7 +3322,7 @@ int lattice_capacity(int chunk, int window_bins) {
 // Leaf window entries: the windows share the CTA's shared memory with the chunk's pulse and
 // (pulse, column) records, within the same per-CTA total as the direct kernels' windows.
 int leaf_capacity(int chunk, int window_bins) {
-    return capacity_for(chunk, window_bins, kWindowBudget - (int)leaf_window_offset(chunk));
+    return capacity_for(chunk, window_bins, kLeafWindowBudget - (int)leaf_window_offset());
 }
 
 }  // namespace
@@ -3374,9 +3501,9 @@ int launch_split_ffbp_leaves(const PulseInputs& in, const PolarDesc* nodes, cons
                              float2* root_out, int root, cudaStream_t s) {
     if (nitems <= 0) return SARBP_OK;
     SplitParams P = make_params(in, chunk, leaf_capacity(chunk, window_bins), 1);
-    const size_t smem = leaf_window_offset(chunk) + (size_t)P.cap * 32;
+    const size_t smem = leaf_window_offset() + (size_t)P.cap * 32;
     if (int st = prepare(split_leaf_kernel, smem)) return st;
-    split_leaf_kernel<<<nitems, kThreads, smem, s>>>(P, nodes, items, tables, reinterpret_cast<const PulseRec*>(precs),
+    split_leaf_kernel<<<nitems, kLeafThreads, smem, s>>>(P, nodes, items, tables, reinterpret_cast<const PulseRec*>(precs),
                                                      arena, root_out, root);
     note_launches(1);
     return check_launch("split_ffbp_leaves");
@@ -3543,7 +3670,7 @@ __global__ void __launch_bounds__(kThreads, 4) batch_direct_kernel(const BatchSc
 }
 
 // Leaf tiles of every FFBP scene.
-__global__ void __launch_bounds__(kThreads, 3) batch_leaf_kernel(const BatchScene* __restrict__ scenes,
+__global__ void __launch_bounds__(kLeafThreads, kLeafCtas) batch_leaf_kernel(const BatchScene* __restrict__ scenes,
                                                                  const PolarDesc* __restrict__ nodes,
                                                                  const TileItem* __restrict__ items, int nitems,
                                                                  const float4* __restrict__ tables,
@@ -3598,7 +3725,7 @@ __global__ void batch_tables_kernel(const BatchScene* __restrict__ scenes, const
 
 __global__ void batch_leaf_pulses_kernel(const BatchScene* __restrict__ scenes, const PolarDesc* __restrict__ nodes,
                                          const int* __restrict__ leaves, PulseRec* __restrict__ recs) {
-    __shared__ int amax;
+    __shared__ int amax[2];
     const PolarDesc& g = nodes[leaves[blockIdx.x]];
     const BatchScene& sc = scenes[g.pad];
     leaf_pulses(sc.P.K, sc.P.in.pos, sc.P.in.weight, sc.P.in.phase, g, recs + sc.prec_offset, amax);
@@ -3630,7 +3757,7 @@ size_t split_batch_pack_scene(const BatchSceneDesc& d, void* dst) {
     b.lc = d.lc;
     b.prec_offset = d.prec_offset;
     memcpy(dst, &b, sizeof(b));
-    return (d.kind == 0 ? window_offset() + raw_bytes_for(b.P.cap, kMaxChunk) : leaf_window_offset(d.chunk)) +
+    return (d.kind == 0 ? window_offset() + raw_bytes_for(b.P.cap, kMaxChunk) : leaf_window_offset()) +
            (size_t)b.P.cap * 32;
 }
 
@@ -3642,7 +3769,7 @@ int split_batch_occupancy(size_t direct_smem, size_t leaf_smem, int* direct_per_
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(direct_per_sm, batch_direct_kernel, kThreads,
                                                                   direct_smem);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(leaf_per_sm, batch_leaf_kernel, kThreads, leaf_smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(leaf_per_sm, batch_leaf_kernel, kLeafThreads, leaf_smem);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(merge_per_sm, batch_merge_kernel, kMergeThreads, merge_smem());
     if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "occupancy query: %s", cudaGetErrorString(e));
@@ -3694,7 +3821,7 @@ int launch_split_batch_leaves(const void* scenes, const PolarDesc* nodes, const 
                               size_t smem, unsigned long long* trace, cudaStream_t s) {
     if (nitems <= 0) return SARBP_OK;
     if (int st = prepare(batch_leaf_kernel, smem)) return st;
-    batch_leaf_kernel<<<blocks, kThreads, smem, s>>>(reinterpret_cast<const BatchScene*>(scenes), nodes, items, nitems,
+    batch_leaf_kernel<<<blocks, kLeafThreads, smem, s>>>(reinterpret_cast<const BatchScene*>(scenes), nodes, items, nitems,
                                                      tables, reinterpret_cast<const PulseRec*>(precs), arena, counter,
                                                      trace);
     note_launches(1);
