@@ -50,6 +50,8 @@ constexpr int kPointPX = kPointTile / kThreads;  // pixels per thread of the poi
 constexpr int kMergeThreads = 128;
 constexpr int kMaxRows = kSplitTilePixels >> 2;  // tile_lc >= 2
 constexpr int kMaxCols = 32;                     // tile_lc <= 5
+constexpr int kColRun = 8;                       // angle columns per run of a polar tile
+constexpr int kMaxMids = kMaxCols / kColRun;
 constexpr int kMaxChunk = 64;      // pulses per chunk of the direct kernels: two warps compute the records
 constexpr int kMaxLeafChunk = 32;  // pulses per chunk of the FFBP leaf kernels: one warp computes the records
 // Window bytes per CTA: with kMaxChunk records this keeps three CTAs per SM within 227 KB.
@@ -85,7 +87,8 @@ struct Rec {
                // points: a = W in 2^-16 turns/m and Phi in 2^-32 turns, e = u / dr in 2^-12 bins/m and c.x the
                // middle's place in the window in 2^-28 bins (integers); b = u, 2R; c.y that place, FP32;
                // d = rest of W, rest of u.x / dr; e.w rest of u.y / dr)
-    float4 d;  // u.z, W_hi.z, W_lo.z                (lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z)
+    float4 d;  // u.z, W_hi.z, W_lo.z                (polar runs: -2 pi K a.x, -2 pi K a.y with a = pos - origin, the
+               // limit of column_run; lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z)
     float4 e;  // lattice adjoint: the pairs (2R, 2R), (frac(Q) - 1/2, frac(Q) - 1/2) of packed-FP32 operands;
                // lattice forward: (-, window bias bits, window offset bits, window count - 1 bits)
 };
@@ -144,8 +147,10 @@ struct TileShared {
 struct PolarTables {
     double rx[kMaxRows], ry[kMaxRows];
     float rxh[kMaxRows], rxl[kMaxRows], ryh[kMaxRows], ryl[kMaxRows], dg[kMaxRows], psi[kMaxRows];
-    double cxd[kMaxCols], cyd[kMaxCols];
-    float cxh[kMaxCols], cxl[kMaxCols], cyh[kMaxCols], cyl[kMaxCols], dcs[kMaxCols], duu[kMaxCols];
+    double cxd[kMaxCols + kMaxMids], cyd[kMaxCols + kMaxMids];  // the columns, then the middles of their runs
+    float cxh[kMaxCols + kMaxMids], cxl[kMaxCols + kMaxMids], cyh[kMaxCols + kMaxMids], cyl[kMaxCols + kMaxMids];
+    float dcs[kMaxCols + kMaxMids], duu[kMaxCols + kMaxMids];
+    float mid_c[kMaxMids], mid_u[kMaxMids];
 };
 
 struct SplitParams {
@@ -256,8 +261,9 @@ __device__ __forceinline__ void pixel_from_offsets(const TileShared& S, double o
 // ---- per-tile set-up: tile centre, quantum, per-pixel offsets -------------------
 // Polar tile: rows/cols of a polar grid window; separable FP64 row and column
 // tables give each pixel offset as an exact hi part plus an FP32 remainder.
-__device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T, Pix px[kPX],
-                            bool demodulate) {
+// The tables and the tile's centre and bounds; RUNS: also the middles of the runs of columns.
+template <bool RUNS>
+__device__ void polar_tables(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T, bool demodulate) {
     const PolarDesc& g = J.g;
     const int tid = threadIdx.x;
     const int cols_t = 1 << J.lc, rows_t = kSplitTilePixels >> J.lc;
@@ -295,6 +301,17 @@ __device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, P
         m[5] = (float)fabs(dc);
         m[6] = (float)fabs(du);
     }
+    const int groups = cols_t / kColRun, mid = tid - kMaxCols;
+    if (RUNS && mid >= 0 && mid < groups) {
+        const double u = g.u0 + ((double)(g.win_u0 + J.tile_u + kColRun * mid) + 0.5 * (kColRun - 1)) * g.du;
+        const double c = sqrt(fmax(0.0, 1.0 - u * u)), dc = c - cc;
+        T.cxd[tid] = side * gc * dc;
+        T.cyd[tid] = gc * (u - uc);
+        T.dcs[tid] = (float)(side * dc);
+        T.duu[tid] = (float)(u - uc);
+        T.mid_c[mid] = (float)c;
+        T.mid_u[mid] = (float)u;
+    }
     block_max<7>(S, m);
     // Bounds on |delta_x|, |delta_y| (slightly enlarged for the FP32 maxima).
     const float bx = (m[0] + m[3] + m[2] * m[5]) * 1.0001f + 1e-6f;
@@ -308,17 +325,34 @@ __device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, P
         S.bnd[1] = by;
         S.bnd[2] = 0.0f;
         set_quantum(S, fmaxf(bx, by), 12);
+        if (RUNS) {  // for the records: centre - origin, and bounds of the runs' expansion (see make_record)
+            split2(side * gc * cc, S.sth[0], S.stl[0]);
+            split2(gc * uc, S.sth[1], S.stl[1]);
+            const float um = fabsf((float)uc) + m[6], h = fabsf((float)g.du);
+            const float ic = rsqrtf(fmaxf(1.0f - um * um, 0.0f)), hc = h * ic, hcc = hc * ic, u2 = um * um;
+            const float e2 = 0.5f * hc * hc * ic, q4 = e2 * 0.25f * hcc * hcc;  // times (1 + 4 u^2): the fourth order
+            S.sth[2] = q4 * (um * hcc * (3.0f + 4.0f * u2) * 525.3f +
+                             hcc * hcc * 0.5f * (1.0f + 12.0f * u2 + 8.0f * u2 * u2) * 1838.4f);
+            S.sth[3] = 3.5f * hc;
+            S.sth[4] = 12.25f * e2;
+        }
     }
     __syncthreads();
     if (tid < rows_t) {
         quantize(T.rx[tid], S.scale_d, S.inv_scale_d, T.rxh[tid], T.rxl[tid]);
         quantize(T.ry[tid], S.scale_d, S.inv_scale_d, T.ryh[tid], T.ryl[tid]);
     }
-    if (tid < cols_t) {
+    if (tid < cols_t || (RUNS && mid >= 0 && mid < groups)) {
         quantize(T.cxd[tid], S.scale_d, S.inv_scale_d, T.cxh[tid], T.cxl[tid]);
         quantize(T.cyd[tid], S.scale_d, S.inv_scale_d, T.cyh[tid], T.cyl[tid]);
     }
     __syncthreads();
+}
+
+__device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T, Pix px[kPX],
+                            bool demodulate) {
+    polar_tables<false>(P, J, S, T, demodulate);
+    const int tid = threadIdx.x, cols_t = 1 << J.lc;
 #pragma unroll
     for (int k = 0; k < kPX; ++k) {
         const int p = tid + kThreads * k;
@@ -945,8 +979,22 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
     const float eps = S.rhof * S.rhof / (2.0f * fmaxf(Rf - S.rhof, 1.0f));
     const float hw = (lin + eps) * fabsf(P.inv_drf) + 1e-3f;
     const float lo = floorf(Fm - hw), hi = ceilf(Fm + hw);
+    // Runs of columns of a polar grid: the pulse's offset a from the grid's origin, and what the expansion in
+    // the column leaves out at the run's ends, in turns (fifth and sixth order of a.x cos, fifth of the root).
+    float ax = 0.0f, ay = 0.0f, lim = 0.5f;
+    bool runs_ok = true;
+    if (MODE == 4) {
+        const FF fx = ff_add(FF{S.sth[0], S.stl[0]}, ff_neg(vx)), fy = ff_add(FF{S.sth[1], S.stl[1]}, ff_neg(vy));
+        ax = fx.h + fx.l;
+        ay = fy.h + fy.l;
+        const float turn = S.sth[3] * (fabsf(ax) + fabsf(ay)), y = turn / Rf;
+        runs_ok = fabsf(P.Kf) * (fabsf(ax) * S.sth[2] + turn * (y * y) * (y * y)) <= 1e-7f;
+        // The sample's cubic leaves out the square of the quadratic term.
+        const float x1 = turn * fabsf(P.inv_drf), x2 = fmaf(S.sth[4], fabsf(ax), 0.5f * turn * y) * fabsf(P.inv_drf);
+        lim = (3.0f * x1 * x1 + x2) * x2 <= 1e-7f ? 0.5f : -1.0f;
+    }
     const bool ok = Rf > 0.0f && fabsf(Q.h) < 1.0e7f && hi - lo + 1.0f <= (float)P.cap &&
-                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf;
+                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf && runs_ok;
     const int bo = ok ? (int)lo : 0;
     S.base[lane] = ok ? (int)I + bo : 0;
     S.wt[lane] = (float)in.weight[n];
@@ -970,7 +1018,7 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         const int mid = __float2int_rn(Fm * 268435456.0f);  // |Fm| <= 1/2
         r.c.x = __int_as_float((int)((unsigned)mid - ((unsigned)bo << 28)));
         r.c.y = Fm - (float)bo;
-    } else if (MODE != 0) {
+    } else if (MODE == 1 || MODE == 2) {
         // Lattice tile: the linear phase W . delta of pixel (i, j) is i B_row + j B_col with
         // B = W . step.  Both are split on one power-of-two quantum with <= 10 significant
         // bits, so i B_row_hi + j B_col_hi is exact in FP32 for |i|, |j| < 2^12.
@@ -1039,8 +1087,9 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         r.d.x = uzf;
         r.d.w = 0.0f;
         r.e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (MODE == 4) r.d = make_float4(-kTwoPiF * P.Kf * ax, -kTwoPiF * P.Kf * ay, lim, 0.0f);
     }
-    if (MODE == 0 || MODE == 2) r.c.x = t1;
+    if (MODE == 0 || MODE == 2 || MODE == 4) r.c.x = t1;
     float4& rw = rec_window<MODE>(r);
     if (MODE != 3) rw.y = __int_as_float(kMagicBits + bo);
     const int count = ok ? (int)(hi - lo) + 1 : P.cap + 1;
@@ -1355,6 +1404,87 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
     if (threadIdx.x == 0)
         asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"((unsigned)__cvta_generic_to_shared(&mbar)) : "memory");
 #endif
+}
+
+// One pulse on a run of eight angle columns whose range changes by less than a bin's width as a rule
+// (polar grids): phase P0 + P1 m + ... + P4 m^4 (radians) and place in the window (bins) qp + b1 m + b2 m^2
+// at the columns m = -3.5 ... 3.5.  bias, last: byte offset in the window w0 of the entry that index bits 0
+// would address, and of the last entry.  The sample along the run is the window entry's cubic, a cubic in m
+// as long as the whole run stays within one range bin; when that holds for all the warp's runs (lim = 1/2;
+// below 0: never) the run takes one window entry (two 16-byte loads instead of sixteen), and the even and
+// odd parts of both polynomials serve the columns +m and -m.  Otherwise each pixel takes its own entry.
+__device__ __forceinline__ void column_run(float P0, float P1, float P2, float P3, float P4, float qp, float b1, float b2,
+                                           float lim, const char* __restrict__ w0, unsigned bias, unsigned last,
+                                           float ar[kColRun], float ai[kColRun]) {
+    const float tq = qp + kMagic;
+    const float s = qp - (tq - kMagic);
+    const float spread = fmaf(fabsf(b2), 12.25f, fmaf(fabsf(b1), 3.5f, fabsf(s)));
+    if (__all_sync(0xffffffffu, spread <= lim)) {
+        const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(tq) + bias, last));
+        const float4 c01 = w[0], c23 = w[1];
+        float V0[2], V1[2], V2[2], V3[2];
+        const float bb = b1 * b1;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const float A0 = c ? c01.y : c01.x, A1 = c ? c01.w : c01.z, A2 = c ? c23.y : c23.x, A3 = c ? c23.w : c23.z;
+            const float T = A3 * s;
+            const float W1 = A2 + T, W2 = fmaf(3.0f, T, A2);
+            const float V = fmaf(W1, s, A1);               // the sample is A0 + V s
+            const float D = fmaf(A2 + W2, s, A1);         // its derivative
+            V0[c] = fmaf(V, s, A0);
+            V1[c] = D * b1;
+            V2[c] = fmaf(W2, bb, D * b2);
+            V3[c] = fmaf(A3, bb, 2.0f * W2 * b2) * b1;
+        }
+#pragma unroll
+        for (int h = 0; h < kColRun / 2; ++h) {
+            const float m = 0.5f + h, mm = m * m;
+            const float ae = fmaf(fmaf(P4, mm, P2), mm, P0), ao = fmaf(P3, mm, P1);
+            const float re = fmaf(V2[0], mm, V0[0]), ro = fmaf(V3[0], mm, V1[0]);
+            const float ie = fmaf(V2[1], mm, V0[1]), io = fmaf(V3[1], mm, V1[1]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int k = c ? kColRun / 2 + h : kColRun / 2 - 1 - h;
+                const float x = c ? m : -m;
+                const float vr = fmaf(ro, x, re), vi = fmaf(io, x, ie);
+                float sn, cs;
+                __sincosf(fmaf(ao, x, ae), &sn, &cs);
+                ar[k] = fmaf(vr, cs, ar[k]);
+                ar[k] = fmaf(-vi, sn, ar[k]);
+                ai[k] = fmaf(vr, sn, ai[k]);
+                ai[k] = fmaf(vi, cs, ai[k]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kColRun; ++k) {
+            const float x = (float)k - 0.5f * (kColRun - 1);
+            const float p = fmaf(fmaf(b2, x, b1), x, qp);
+            const float t = p + kMagic, f = p - (t - kMagic);
+            const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(t) + bias, last));
+            const float4 c01 = w[0], c23 = w[1];
+            const float vr = fmaf(fmaf(fmaf(c23.z, f, c23.x), f, c01.z), f, c01.x);
+            const float vi = fmaf(fmaf(fmaf(c23.w, f, c23.y), f, c01.w), f, c01.y);
+            float sn, cs;
+            __sincosf(fmaf(fmaf(fmaf(fmaf(P4, x, P3), x, P2), x, P1), x, P0), &sn, &cs);
+            ar[k] = fmaf(vr, cs, ar[k]);
+            ar[k] = fmaf(-vi, sn, ar[k]);
+            ai[k] = fmaf(vr, sn, ai[k]);
+            ai[k] = fmaf(vi, cs, ai[k]);
+        }
+    }
+}
+
+// Coefficients along a run of columns: at = (ground range) / d, z = 1 / (2 pi K d) at the run's middle and
+// T_j the phase's coefficients at unit ground range and distance (radians).  From
+//   d(m)^2 = d^2 - 2 g sum_j (a . s_j) m^j   (a the pulse's offset from the grid's origin).
+__device__ __forceinline__ void run_phase(float at, float z, float T1, float T2, float T3, float T4, float& P1, float& P2,
+                                          float& P3, float& P4) {
+    P1 = at * T1;
+    const float y1 = z * P1;
+    P2 = fmaf(-0.5f * P1, y1, at * T2);
+    P3 = fmaf(-y1, P2, at * T3);
+    P4 = fmaf(-y1, P3, fmaf(-0.5f * z * P2, P2, at * T4));
 }
 
 struct PolarBody {
@@ -1889,6 +2019,157 @@ __global__ void __launch_bounds__(kThreads, 3) split_polar_kernel(SplitParams P,
     store_window(J, g.win_nr, g.win_nu, px, P.out + blockIdx.y * P.split_stride, P.out_stride);
 }
 
+// Add the two halves' images of a tile in runs of eight pixels: each half passes on four pixels of every run
+// through shared memory and finishes the other four (store(k, value)).
+template <class Store>
+__device__ __forceinline__ void add_halves(float2* ex, int half, int slot, const float ar[kRun], const float ai[kRun],
+                                           Store store) {
+    __syncthreads();  // the last chunk's windows are consumed
+#pragma unroll
+    for (int k = 0; k < kRun / 2; ++k)
+        ex[(kRun / 2 * half + k) * kRunThreads + slot] =
+            half ? make_float2(ar[k], ai[k]) : make_float2(ar[k + kRun / 2], ai[k + kRun / 2]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRun / 2; ++k) {
+        const float2 o = ex[(kRun / 2 * (1 - half) + k) * kRunThreads + slot];
+        store(kRun / 2 * half + k, half ? make_float2(o.x + ar[k + kRun / 2], o.y + ai[k + kRun / 2])
+                                        : make_float2(ar[k] + o.x, ai[k] + o.y));
+    }
+}
+
+// Polar tile in runs of eight columns: a run's middle and what the expansion along it needs.
+struct PolarRun {
+    float dx, dy, dxh, dyh, dxl, dyl, d2, psi;  // the middle's offset from the tile centre, -K r modulo a turn
+    float g;                                    // ground range of the row
+    float s1, s2, s3, s4, h;                    // s = side sqrt(1 - u^2): s^(j)(u) du^j / j!; du
+};
+
+__device__ __forceinline__ void setup_polar_runs(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T,
+                                                 int row, int group, PolarRun& q) {
+    polar_tables<true>(P, J, S, T, true);
+    const int m = kMaxCols + group;
+    q.dxh = T.rxh[row] + T.cxh[m];  // exact: both multiples of the quantum
+    q.dyh = T.ryh[row] + T.cyh[m];
+    q.dxl = fmaf(T.dg[row], T.dcs[m], T.rxl[row] + T.cxl[m]);
+    q.dyl = fmaf(T.dg[row], T.duu[m], T.ryl[row] + T.cyl[m]);
+    q.dx = q.dxh + q.dxl;
+    q.dy = q.dyh + q.dyl;
+    q.d2 = q.dx * q.dx + q.dy * q.dy;
+    q.psi = T.psi[row];
+    q.g = T.dg[row] + sqrtf(S.sth[0] * S.sth[0] + S.sth[1] * S.sth[1]);
+    const float u = T.mid_u[group], ic = 1.0f / T.mid_c[group];
+    q.h = (float)J.g.du;
+    const float hc = q.h * ic, hcc = hc * ic;
+    q.s1 = (float)J.g.side * -u * hc;
+    q.s2 = (float)J.g.side * -0.5f * hc * hc * ic;
+    q.s3 = q.s2 * u * hcc;
+    q.s4 = q.s2 * 0.25f * (1.0f + 4.0f * u * u) * hcc * hcc;
+    __syncthreads();  // the tables alias the window region
+}
+
+// Pulses the fast path cannot stage on a run's pixels, every second one from `first`: offsets in two-float
+// from FP64 (rare, and out of line so that it costs the fast path no registers).
+__device__ __noinline__ void polar_run_slow(const SplitParams& P, const TileShared& S, const PolarDesc& g, int i, int j0,
+                                            int first, int nslow, int c0, const SlowRec* srec, float2* sum) {
+    const double r = g.r0 + (double)i * g.dr, gr = sqrt(fmax(0.0, r * r - g.oz * g.oz)), t = -P.K * r;
+#pragma unroll 1
+    for (int k = 0; k < kColRun; ++k) {
+        const double u = g.u0 + (double)(j0 + k) * g.du;
+        Pix q;
+        pixel_from_offsets(S, g.ox + (double)g.side * gr * sqrt(fmax(0.0, 1.0 - u * u)) - S.cx, g.oy + gr * u - S.cy, 0.0,
+                           q);
+        // Pulse by pulse onto the run's sums, so that the image does not depend on the chunks.
+        for (int j = first; j < nslow; j += 2) {
+            const float2 v = slow_pixel(P, srec, j, j + 1, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
+                                        (float)(t - rint(t)));
+            sum[k].x += v.x;
+            sum[k].y += v.y;
+        }
+    }
+}
+
+// Direct BP on a polar tile in runs of eight columns; the block's halves take alternate pulses as the
+// lattice tiles' do.  Range, phase and window place are worked out once per run (split arithmetic at its
+// middle, as polar_chunk does per pixel) and expanded along it from the polar geometry (run_phase).
+// What bounds it: instruction issue (77% of the cycles, 248 instructions per warp and pulse) and the last of
+// few waves.  1024 pulses onto 720 x 1600: 1.28 ms, pixel by pixel (polar_chunk) 1.76; with every pixel on its
+// own window entry 1.66, with 64 registers and four blocks per SM 1.35, with shuffled staging 1.31.
+struct PolarRunBody {
+    static constexpr int kRecMode = 4;
+    static constexpr bool kShflWindows = false;
+    const SplitParams& P;
+    const TileShared& S;
+    const Job& J;
+    const PolarRun& q;
+    int i, j0;
+    float* ar;
+    float* ai;
+    __device__ int group() const { return threadIdx.x / kRunThreads; }
+    __device__ void fast(const Rec* rec, const float4* win, int nfit, int c0) {
+        const float inv_dr = P.inv_drf, Kf = P.Kf, kz = 1.0f / (kTwoPiF * Kf), kd = inv_dr * kz;
+#pragma unroll 1
+        for (int nl = (c0 - J.p0 + group()) & 1; nl < nfit; nl += 2) {
+            const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c, rd = rec[nl].d;
+            const float L = fmaf(rb.x, q.dx, rb.y * q.dy);
+            const float q2 = fmaf(-L, L, q.d2);
+            const float B = rcp_approx(fmaf(2.0f, L, rb.z));
+            const float e0 = q2 * B;
+            const float eps = fmaf(-e0 * e0, B, e0);
+            const float Le = L + eps;
+            const float iR = rcp_approx(fmaf(0.5f, rb.z, Le));
+            const float tb = fmaf(ra.x, q.dxh, ra.y * q.dyh);
+            float sm = fmaf(Kf, eps, rc.x);
+            sm = fmaf(ra.x, q.dxl, sm);
+            sm = fmaf(ra.y, q.dyl, sm);
+            sm = fmaf(ra.z, q.dx, sm);
+            sm = fmaf(ra.w, q.dy, sm);
+            const float P0 = ((tb - round_magic(tb)) + (sm + q.psi)) * kTwoPiF;
+            float P1, P2, P3, P4;
+            run_phase(q.g * iR, iR * kz, fmaf(rd.x, q.s1, rd.y * q.h), rd.x * q.s2, rd.x * q.s3, rd.x * q.s4, P1, P2, P3,
+                      P4);
+            column_run(P0, P1, P2, P3, P4, fmaf(Le, inv_dr, rb.w), P1 * kd, P2 * kd, rd.z,
+                       reinterpret_cast<const char*>(win + 2 * __float_as_int(rc.z)), 0u - 32u * (unsigned)__float_as_int(rc.y),
+                       32u * (unsigned)__float_as_int(rc.w), ar, ai);
+        }
+    }
+    __device__ void slow(int c0, int nslow, const SlowRec* srec) {
+        float2 sum[kColRun];
+#pragma unroll
+        for (int k = 0; k < kColRun; ++k) sum[k] = make_float2(ar[k], ai[k]);
+        polar_run_slow(P, S, J.g, i, j0, (c0 - J.p0 + group()) & 1, nslow, c0, srec, sum);
+#pragma unroll
+        for (int k = 0; k < kColRun; ++k) {
+            ar[k] = sum[k].x;
+            ai[k] = sum[k].y;
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kThreads, 3) split_polar_runs_kernel(SplitParams P, PolarDesc g) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ TileShared S;
+    Job J;
+    J.g = g;
+    J.lc = g.tile_lc;  // 3 to 5: whole runs, and a warp's 32 rows in one run of columns
+    tile_of(blockIdx.x, g.win_nu, J.lc, J.tile_r, J.tile_u);
+    split_range(g.a, g.b, P.pulse_split, blockIdx.y, J.p0, J.p1);
+    const int rows_t = kSplitTilePixels >> J.lc, slot = threadIdx.x & (kRunThreads - 1);
+    const int row = slot & (rows_t - 1), col = kColRun * (slot / rows_t);
+    PolarRun q;
+    setup_polar_runs(P, J, S, *reinterpret_cast<PolarTables*>(smem + window_offset()), row, col / kColRun, q);
+    float ar[kColRun], ai[kColRun];
+#pragma unroll
+    for (int k = 0; k < kColRun; ++k) ar[k] = ai[k] = 0.0f;
+    PolarRunBody body{P, S, J, q, g.win_r0 + J.tile_r + row, g.win_u0 + J.tile_u + col, ar, ai};
+    chunk_loop(P, J, S, smem, true, body);
+    float2* out = P.out + blockIdx.y * P.split_stride;
+    add_halves(reinterpret_cast<float2*>(smem + window_offset()), body.group(), slot, ar, ai, [&](int k, float2 v) {
+        const int wr = J.tile_r + row, wu = J.tile_u + col + k;
+        if (wr < g.win_nr && wu < g.win_nu) out[(long long)wr * P.out_stride + wu] = v;
+    });
+}
+
 // One lattice tile over pulses [p0, p1): the per-item body shared by the one-tile-per-CTA
 // kernel and the persistent batch kernel.
 __device__ __forceinline__ void lattice_tile(const SplitParams& P, const sarbp_lattice& lat, int lc, int tile_r,
@@ -1917,23 +2198,10 @@ __device__ __forceinline__ void lattice_tile(const SplitParams& P, const sarbp_l
     for (int k = 0; k < kRun; ++k) ar[k] = ai[k] = 0.0f;
     LatticeBody body{P, S, J, di, dj, d2, ds, s2, ar, ai};
     chunk_loop(P, J, S, smem, true, body);
-    // Add the two halves' images: each half passes on four rows of every run and finishes the other four.
-    __syncthreads();  // the last chunk's windows are consumed
-    const int half = body.group();
-    float2* ex = reinterpret_cast<float2*>(smem + window_offset());
-#pragma unroll
-    for (int k = 0; k < kRun / 2; ++k)
-        ex[(kRun / 2 * half + k) * kRunThreads + slot] =
-            half ? make_float2(ar[k], ai[k]) : make_float2(ar[k + kRun / 2], ai[k + kRun / 2]);
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kRun / 2; ++k) {
-        const float2 o = ex[(kRun / 2 * (1 - half) + k) * kRunThreads + slot];
-        const float2 v = half ? make_float2(o.x + ar[k + kRun / 2], o.y + ai[k + kRun / 2])
-                              : make_float2(ar[k] + o.x, ai[k] + o.y);
-        const int wr = tile_r + row0 + kRun / 2 * half + k, wu = tile_u + col;
+    add_halves(reinterpret_cast<float2*>(smem + window_offset()), body.group(), slot, ar, ai, [&](int k, float2 v) {
+        const int wr = tile_r + row0 + k, wu = tile_u + col;
         if (wr < lat.rows && wu < lat.cols) out[(long long)wr * lat.cols + wu] = v;
-    }
+    });
 }
 
 __global__ void __launch_bounds__(kThreads, 4) split_lattice_kernel(SplitParams P, sarbp_lattice lat, int lc) {
@@ -2219,7 +2487,7 @@ struct LeafMid {
     int pad;
 };
 
-constexpr int kLeafRun = 8;                                   // columns per thread
+constexpr int kLeafRun = kColRun;                             // columns per thread
 constexpr int kLeafThreads = kSplitTilePixels / kLeafRun;
 constexpr int kLeafGroups = kMaxCols / kLeafRun;              // runs per tile row, at most
 constexpr int kLeafCtas = 6;                                  // per SM, by registers and by the window budget
@@ -2336,73 +2604,10 @@ __device__ __forceinline__ void leaf_runs(const SplitParams& P, const LeafRec* _
         sm = fmaf(q.bl, ra.z + ra.w, sm);
         const float P0 = ((tb - round_magic(tb)) + sm) * kTwoPiF;
         const float z = iR * kz;
-        const float P1 = at * cb.x;
-        const float y1 = z * P1;
-        const float P2 = fmaf(-0.5f * P1, y1, at * cb.y);
-        const float P3 = fmaf(-y1, P2, at * cb.z);
-        const float P4 = fmaf(-y1, P3, fmaf(-0.5f * z * P2, P2, at * cb.w));
-        // Place in the window at the middle, and its slope and curvature (bins).
-        const float qp = fmaf(dd, inv_dr, q.fm);
-        const float tq = qp + kMagic;
-        const float s = qp - (tq - kMagic);
-        const float b1 = P1 * kd, b2 = P2 * kd;
-        const unsigned bias = 32u * (unsigned)q.o + (unsigned)__float_as_int(rb.y), last = (unsigned)__float_as_int(rb.w);
-        const char* w0 = win + __float_as_int(rb.z);
-        const float spread = fmaf(fabsf(b2), 12.25f, fmaf(fabsf(b1), 3.5f, fabsf(s)));
-        if (__all_sync(0xffffffffu, spread <= lim)) {
-            const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(tq) + bias, last));
-            const float4 c01 = w[0], c23 = w[1];
-            float V0[2], V1[2], V2[2], V3[2];
-            const float bb = b1 * b1;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const float A0 = c ? c01.y : c01.x, A1 = c ? c01.w : c01.z, A2 = c ? c23.y : c23.x, A3 = c ? c23.w : c23.z;
-                const float T = A3 * s;
-                const float W1 = A2 + T, W2 = fmaf(3.0f, T, A2);
-                const float V = fmaf(W1, s, A1);               // the sample is A0 + V s
-                const float D = fmaf(A2 + W2, s, A1);         // its derivative
-                V0[c] = fmaf(V, s, A0);
-                V1[c] = D * b1;
-                V2[c] = fmaf(W2, bb, D * b2);
-                V3[c] = fmaf(A3, bb, 2.0f * W2 * b2) * b1;
-            }
-#pragma unroll
-            for (int h = 0; h < kLeafRun / 2; ++h) {
-                const float m = 0.5f + h, mm = m * m;
-                const float ae = fmaf(fmaf(P4, mm, P2), mm, P0), ao = fmaf(P3, mm, P1);
-                const float re = fmaf(V2[0], mm, V0[0]), ro = fmaf(V3[0], mm, V1[0]);
-                const float ie = fmaf(V2[1], mm, V0[1]), io = fmaf(V3[1], mm, V1[1]);
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int k = c ? kLeafRun / 2 + h : kLeafRun / 2 - 1 - h;
-                    const float x = c ? m : -m;
-                    const float vr = fmaf(ro, x, re), vi = fmaf(io, x, ie);
-                    float sn, cs;
-                    __sincosf(fmaf(ao, x, ae), &sn, &cs);
-                    ar[k] = fmaf(vr, cs, ar[k]);
-                    ar[k] = fmaf(-vi, sn, ar[k]);
-                    ai[k] = fmaf(vr, sn, ai[k]);
-                    ai[k] = fmaf(vi, cs, ai[k]);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < kLeafRun; ++k) {
-                const float x = (float)k - 0.5f * (kLeafRun - 1);
-                const float p = fmaf(fmaf(b2, x, b1), x, qp);
-                const float t = p + kMagic, f = p - (t - kMagic);
-                const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(t) + bias, last));
-                const float4 c01 = w[0], c23 = w[1];
-                const float vr = fmaf(fmaf(fmaf(c23.z, f, c23.x), f, c01.z), f, c01.x);
-                const float vi = fmaf(fmaf(fmaf(c23.w, f, c23.y), f, c01.w), f, c01.y);
-                float sn, cs;
-                __sincosf(fmaf(fmaf(fmaf(fmaf(P4, x, P3), x, P2), x, P1), x, P0), &sn, &cs);
-                ar[k] = fmaf(vr, cs, ar[k]);
-                ar[k] = fmaf(-vi, sn, ar[k]);
-                ai[k] = fmaf(vr, sn, ai[k]);
-                ai[k] = fmaf(vi, cs, ai[k]);
-            }
-        }
+        float P1, P2, P3, P4;
+        run_phase(at, z, cb.x, cb.y, cb.z, cb.w, P1, P2, P3, P4);
+        column_run(P0, P1, P2, P3, P4, fmaf(dd, inv_dr, q.fm), P1 * kd, P2 * kd, lim, win + __float_as_int(rb.z),
+                   32u * (unsigned)q.o + (unsigned)__float_as_int(rb.y), (unsigned)__float_as_int(rb.w), ar, ai);
     }
 }
 
@@ -3265,7 +3470,7 @@ size_t dynamic_smem(int cap, bool polar) {
 
 template <class K>
 int prepare(K kernel, size_t smem) {
-    if (smem > 48 * 1024) {
+    if (smem > 40 * 1024) {  // 48 KB without the attribute, static shared memory included
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     }
@@ -3378,14 +3583,25 @@ int split_polar_tile_lc_slack(const PolarDesc& g, double slack, double* radius) 
 
 int launch_split_polar(const PulseInputs& in, const PolarDesc& g, int pulse_split, int chunk, int window_bins,
                        float2* out, long long out_stride, long long split_stride, cudaStream_t s) {
-    SplitParams P = make_params(in, chunk, capacity_for(chunk, window_bins), pulse_split);
+    // Runs of columns need tiles at least a run wide and an angle step at which the expansion holds for any
+    // pulse the grid resolves (K |a| du below half a turn: 0.5 du^4 turns at fifth order).
+    const double ua = fabs(g.u0 + g.win_u0 * g.du), ub = fabs(g.u0 + (g.win_u0 + g.win_nu - 1) * g.du);
+    const bool runs = g.tile_lc >= 3 && fabs(g.du) <= 0.002 * (1.0 - fmax(ua, ub) * fmax(ua, ub));
+    int cap = capacity_for(chunk, window_bins);
+    if (runs) cap = std::max(cap, kSplitTilePixels * (int)sizeof(float2) / 32);  // the halves' exchange
+    SplitParams P = make_params(in, chunk, cap, pulse_split);
     P.out = out;
     P.out_stride = out_stride;
     P.split_stride = split_stride;
     const size_t smem = dynamic_smem(P.cap, true);
-    if (int st = prepare(split_polar_kernel, smem)) return st;
     dim3 grid(tiles_of(g.win_nr, g.win_nu, g.tile_lc), pulse_split);
-    split_polar_kernel<<<grid, kThreads, smem, s>>>(P, g);
+    if (runs) {
+        if (int st = prepare(split_polar_runs_kernel, smem)) return st;
+        split_polar_runs_kernel<<<grid, kThreads, smem, s>>>(P, g);
+    } else {
+        if (int st = prepare(split_polar_kernel, smem)) return st;
+        split_polar_kernel<<<grid, kThreads, smem, s>>>(P, g);
+    }
     note_launches(1);
     return check_launch("split_polar");
 }
