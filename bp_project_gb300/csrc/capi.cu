@@ -721,6 +721,11 @@ int sarbp_ffbp_plan_create(const sarbp_ffbp_node* nodes, int n_nodes, int crop_r
         double radius = 0.0;
         d.tile_lc = split_polar_tile_lc(d, &radius);
         if (d.left >= 0 && mode == SARBP_SPLIT) d.tile_lc = split_polar_tile_lc_slack(d, kMergeTileSlack, nullptr);
+        d.run_k = 0.0f;
+        if (d.left >= 0 && mode == SARBP_SPLIT) {
+            const PolarDesc* children[2] = {&p->nodes[d.left], &p->nodes[d.right]};
+            d.run_k = split_merge_run_limit(d, children);
+        }
         const bool external = d.left < 0 && d.a < 0;
         if (d.left < 0 && mode == SARBP_SPLIT && !external) {
             // Leaves use the origin formulation: precision does not depend on the tile shape.  Of the
@@ -992,10 +997,13 @@ int sarbp_ffbp_execute(const sarbp_ffbp_plan* plan, const float* data, int pulse
         }
         for (int h = 1; h <= plan->max_height && st == SARBP_OK && !plan->merge_queue; ++h) {
             const size_t first = (size_t)(plan->stage_begin[h] - plan->stage_begin[1]);
+            int kinds = 0;
+            for (int i = 0; i < plan->n_nodes; ++i)
+                if (plan->height[i] == h) kinds |= merges_in_runs(plan->nodes[i], (float)(k * kInvTwoPi)) ? kMergeRuns : kMergePairs;
             st = launch_split_ffbp_merges(k, nodes, items + plan->stage_begin[h], plan->stage_count[h], tables,
                                           reinterpret_cast<char*>(crecs) + 2 * first * crec_size, arena, root_out, 0,
                                           plan->staged ? plan->merge_box_bytes[h] : 0, plan->queue_limit_ns,
-                                          plan->withheld, s);
+                                          plan->withheld, kinds == (kMergeRuns | kMergePairs) ? kMergeEither : kinds, s);
         }
     } else {
         const int2* blocks = reinterpret_cast<const int2*>(base + plan->node_bytes);

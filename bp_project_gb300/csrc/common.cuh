@@ -105,6 +105,8 @@ struct PolarDesc {
     // tile's centre pixel and is box_h x box_w elements; box_w == 0: not staged.
     int box_r, box_u, box_h, box_w;
     double inv_dr, inv_du;  // 1 / dr, 1 / du
+    float run_k;            // merge nodes: the largest K (turns/m) at which the node's tiles merge in runs of rows
+    int pad2;
 };
 
 // Fills PolarDesc::tf and the reciprocals from the FP64 fields (host).
@@ -117,6 +119,12 @@ inline void split_geometry(PolarDesc& d) {
         d.tf[i] = make_float2(h, (float)(v[i] - (double)h));
     }
 }
+
+// Whether merge node g's tiles merge in runs of rows at K turns/m, and what is known of the nodes of a launch.
+__host__ __device__ inline bool merges_in_runs(const PolarDesc& g, float K) {
+    return fabsf(K) >= 1e-3f && fabsf(K) <= g.run_k;
+}
+enum MergeKind { kMergeEither = 0, kMergeRuns = 1, kMergePairs = 2 };
 
 struct TileItem {
     int node;
@@ -197,6 +205,8 @@ int split_wait_timeouts(int* count);
 int split_polar_tile_lc(const PolarDesc& g, double* radius);
 // The widest tile shape whose radius is within `slack` (>= 1) of the smallest (FFBP merge tiles).
 int split_polar_tile_lc_slack(const PolarDesc& g, double slack, double* radius);
+// Largest K (turns/m; 0: none) at which merge node g, with its tile shape and children, merges in runs of rows.
+float split_merge_run_limit(const PolarDesc& g, const PolarDesc* children[2]);
 int launch_split_polar(const PulseInputs& in, const PolarDesc& g, int pulse_split, int chunk, int window_bins,
                        float2* out, long long out_stride, long long split_stride, cudaStream_t s);
 int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pulse_split, int chunk,
@@ -320,7 +330,7 @@ int launch_split_ffbp_merge_queue(double k, const PolarDesc* nodes, const TileIt
 // than their copies deliver, so that their waits run out.
 int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* items, int nitems,
                              const float4* tables, const void* crecs, float2* arena, float2* root_out, int root,
-                             size_t box_bytes, unsigned long long wait_ns, int withheld, cudaStream_t s);
+                             size_t box_bytes, unsigned long long wait_ns, int withheld, int kind, cudaStream_t s);
 // Shared-memory bytes of one staged child footprint (rows x cols complex64, 128-byte granules).
 __host__ __device__ inline size_t split_box_bytes(int rows, int cols) { return ((size_t)rows * cols * 8 + 127) / 128 * 128; }
 // Largest staged footprint per child, 13 KB: the 32 x 32 and 16 x 64 tiles of near-range plans need

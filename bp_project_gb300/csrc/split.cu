@@ -52,6 +52,8 @@ constexpr int kMaxRows = kSplitTilePixels >> 2;  // tile_lc >= 2
 constexpr int kMaxCols = 32;                     // tile_lc <= 5
 constexpr int kColRun = 8;                       // angle columns per run of a polar tile
 constexpr int kMaxMids = kMaxCols / kColRun;
+constexpr int kMergeRun = 8;                     // parent rows per run of a merge tile
+constexpr int kMergeRows = kMaxRows / kMergeRun; // runs per tile column, at most
 constexpr int kMaxChunk = 64;      // pulses per chunk of the direct kernels: two warps compute the records
 constexpr int kMaxLeafChunk = 32;  // pulses per chunk of the FFBP leaf kernels: one warp computes the records
 // Window bytes per CTA: with kMaxChunk records this keeps three CTAs per SM within 227 KB.
@@ -431,7 +433,7 @@ __device__ __forceinline__ TabCol tab_col(const PolarDesc& g, const float4* __re
     const float ch = cv.x - c0v.x, cl = cv.y - c0v.y;  // c in (0, 1] within a factor 2: exact
     // u_j - u_0 = (j - j0) du, formed from the integer offset (no cancellation).
     const float kj = (float)(j - j0);
-    const float duh = (float)g.du, dul = (float)(g.du - (double)duh);
+    const float duh = g.tf[6].x, dul = g.tf[6].y;
     const float uh = kj * duh;
     const float ul = fmaf(kj, duh, -uh) + kj * dul;
     TabCol C;
@@ -475,8 +477,12 @@ __device__ __forceinline__ void tab_quantum(const PolarDesc& g, int lc, int tile
     const float mdg = fmaxf(fabsf(ra.dg), fabsf(rb.dg));
     const float mcx = fmaxf(fabsf(ca.cxh), fabsf(cb.cxh)), mcy = fmaxf(fabsf(ca.cyh), fabsf(cb.cyh));
     const float mdc = fmaxf(fabsf(ca.dcs), fabsf(cb.dcs)), mdu = fmaxf(fabsf(ca.duu), fabsf(cb.duu));
-    const float bx = fmaf(fmaf(mdg, mdc, mrx + mcx), 1.0001f, 1e-6f);
-    const float by = fmaf(fmaf(mdg, mdu, mry + mcy), 1.0001f, 1e-6f);
+    // The last run of rows may reach past the grid: its middle lies less than half a run beyond the last row.
+    const float over = g.run_k > 0.0f && g.win_r0 + tile_r + rows_t > g.nr
+                           ? 0.5f * kMergeRun * fabsf(g.tf[4].x) / __ldg(tables + g.rows_off + 3 * (long long)min(g.win_r0 + tile_r, g.nr - 1) + 1).x
+                           : 0.0f;
+    const float bx = fmaf(fmaf(mdg, mdc, mrx + mcx) + over, 1.0001f, 1e-6f);
+    const float by = fmaf(fmaf(mdg, mdu, mry + mcy) + over, 1.0001f, 1e-6f);
     const int e = ((__float_as_int(fmaxf(bx, by)) >> 23) & 0xff) - 126;
     q = __int_as_float((e - 12 + 127) << 23);
     iq = __int_as_float((12 - e + 127) << 23);
@@ -2568,7 +2574,7 @@ __device__ __forceinline__ LeafMid leaf_mid(const SplitParams& P, const PolarDes
     const float q6 = fabsf(M.s4) * (hc * ic) * (hc * ic) * 0.5f * (1.0f + 12.0f * u2 + 8.0f * u2 * u2) / (1.0f + 4.0f * u2);
     const float ir = 1.0f / r_min, turn = m * hc * 1.5f * amax, y = turn * ir / fabsf(P.Kf);
     const float rest = axmax * m2 * m2 * m * (q5 + m * q6) + turn * (y * y) * (y * y);
-    M.runs = rest <= 5e-8f ? 1 : 0;
+    M.runs = rest <= 5e-8f && fabsf(P.Kf) > 1e-3f ? 1 : 0;
     // The sample's cubic in m leaves out the square of the quadratic term.
     const float kb = fabsf(P.inv_drf / P.Kf);
     const float x1 = turn * kb, x2 = m2 * (axmax * fabsf(M.s2)) * kb + 0.5f * turn * y * kb;
@@ -2799,6 +2805,7 @@ struct ChildRec {
     float4 b;  // u.x, u.y, 2 RR, frac(Qr) - 1/2
     float4 c;  // Phi, h.x, h.y, 2 G
     float4 d;  // G, frac(Qu) - 1/2
+    float4 e;  // merge tiles: parent's origin - child's (x, y), r_c - RR
     float inv_sdr, inv_sdu;
     int ir0, iu0, snr, snu;
     const float2* img;
@@ -2839,6 +2846,7 @@ __device__ __forceinline__ ChildRec child_rec_at(FF K, float scale_w, float inv_
     R.b = make_float4(ux.h + ux.l, uy.h + uy.l, 2.0f * (RR.h + RR.l), fr);
     R.c = make_float4(phi, ff_mul(vx, iG).h, hy.h + hy.l, 2.0f * Gf);
     R.d = make_float4(Gf, fu, 0.0f, 0.0f);
+    R.e = make_float4(RR.h, RR.l, 0.0f, 0.0f);
     R.inv_sdr = c.tf[7].x;
     R.inv_sdu = c.tf[8].x;
     const bool ok = fabsf(Qr.h) < 1.0e7f && fabsf(Qu.h) < 1.0e7f && G.h > 0.0f;  // false for NaN
@@ -2876,6 +2884,10 @@ __device__ __forceinline__ void child_record(FF K, float scale_w, float inv_scal
     const FF py = ff_add(ff_of(g.tf[1]), ff_mul(g0, FF{cv.z, cv.w}));
     ChildRec R = child_rec_at(K, scale_w, inv_scale_w, c, px, py, arena + c.out_offset);
     if (!(t & 1)) tab_quantum(g, g.tile_lc, it.tile_r, it.tile_u, tables, R.d.z, R.d.w);
+    const FF r = ff_add(ff_of(g.tf[3]), ff_mul(FF{(float)i0, 0.0f}, ff_of(g.tf[4])));
+    const FF off = ff_add(r, FF{-R.e.x, -R.e.y});
+    const FF dx = ff_add(ff_of(g.tf[0]), ff_neg(ff_of(c.tf[0]))), dy = ff_add(ff_of(g.tf[1]), ff_neg(ff_of(c.tf[1])));
+    R.e = make_float4(dx.h + dx.l, dy.h + dy.l, off.h + off.l, 0.0f);
     if (tmaps != nullptr && c.box_w > 0 && R.ir0 > -(1 << 30)) {
         R.br0 = R.ir0 - c.box_r;
         R.bu0 = (R.iu0 - c.box_u) & ~1;
@@ -3227,8 +3239,306 @@ __device__ __forceinline__ void child_vpair(float Kf, const ChildDup& C, const V
     oB = __ffma2_rn(pair(vB.x), make_float2(csB, snB), __fmul2_rn(pair(vB.y), make_float2(-snB, csB)));
 }
 
+// ---- merge tiles in runs of rows --------------------------------------------------------------
+//
+// A thread forms a run of eight parent rows in one column.  Along a run the child's range and angle and
+// the demodulated phase K (d - r) are smooth, so they are worked out once per (run, child) at the
+// run's middle (half-way between its fourth and fifth row, m = 0), in the split arithmetic that child_value uses per
+// pixel, and expanded in the row offset m = -3.5 ... 3.5.  With the parent's ground direction e = (side c, u),
+// its ground range g(m) (g^2 = r^2 - z^2, r = r_0 + m h), q = e . (O - C) the offset of its origin from the
+// child's along e, and d the child's range (d^2 = r^2 + 2 q g + const):
+//   D_1 = d_1 - h = (h (r - d) + q g_1) / d          (no cancellation of the row step)
+//   d_2 = (2 q g_2 - D_1 (2 h + D_1)) / 2 d,  d_3 = (q g_3 - d_1 d_2) / d
+// and with G the child's ground range, cos = (g + q) / G, a = e_y - u' cos, n_j = g_j / G the child's angle is
+//   u'_1 = a n_1,  u'_2 = a n_2 - (a cos + u' sin^2 / 2) n_1^2,  u'_3 = a n_3 + ...
+// (the Legendre expansion of 1 / G(m)).  g_j per row: h r / g, -h^2 z^2 / 2 g^3, h^3 z^2 r / 2 g^5.
+// The third orders go into the slopes with 9.25, the linear fit of m^3 over the run.
+// split_merge_run_limit says for which nodes all this holds; the others go pair by pair (child_vpair).
+struct MergeRow {
+    float4 o;  // R_hi.x, R_hi.y, R_lo.x, R_lo.y: (g - g_c) (side c, u) at the tile centre's column
+    float4 p;  // g - g_c, psi = -K r modulo a turn, r - r_c, g
+    float4 w;  // g_1, g_2, g_3, -
+};
+struct MergeCol {
+    float4 o;  // C_hi.x, C_hi.y, C_lo.x, C_lo.y: g_c (side (c - c_c), u - u_c)
+    float4 p;  // side (c - c_c), u - u_c, side c, u
+};
+
+struct MergeTab {
+    MergeRow row[kMergeRows];
+    MergeCol col[kMaxCols];
+};
+
+// A tile's child: its record, and the bins (relative to the record's) at which a pixel's stencil lies
+// inside the child image and, when staged, inside the staged footprint.
+struct __align__(16) MergeChild {
+    ChildRec r;
+    float2 bins;  // child range bins per turn of phase, as a float pair
+    int box;      // staged: the footprint's offset in shared memory (elements)
+    float lo_r, hi_r, lo_u, hi_u;
+};
+
+__device__ __forceinline__ void merge_child(FF K, const PolarDesc& c, const ChildRec& r, int box, MergeChild& C) {
+    int r0 = 1, r1 = r.snr - 3, u0 = 1, u1 = r.snu - 3;
+    if (r.bw > 0) {
+        r0 = max(r0, r.br0 + 1);
+        r1 = min(r1, r.br0 + r.bh - 3);
+        u0 = max(u0, r.bu0 + 1);
+        u1 = min(u1, r.bu0 + r.bw - 3);
+    }
+    C.r = r;
+    const FF b = ff_mul(ff_of(c.tf[7]), ff_rcp(K));
+    C.bins = make_float2(b.h, b.l);
+    C.box = box;
+    const bool ok = r.ir0 > -(1 << 30);
+    C.lo_r = ok ? (float)(r0 - r.ir0) : 1.0f;
+    C.hi_r = ok ? (float)(r1 - r.ir0) : -1.0f;
+    C.lo_u = ok ? (float)(u0 - r.iu0) : 1.0f;
+    C.hi_u = ok ? (float)(u1 - r.iu0) : -1.0f;
+}
+
+// Row `row` (a whole number, or half-way between two) of node g, `off` rows from the tile's centre row.
+__device__ __forceinline__ MergeRow merge_row(FF K, const PolarDesc& g, float4 r0v, float4 c0v, float row, float off,
+                                              float q, float iq) {
+    const float side = (float)g.side;
+    const FF r = ff_add(ff_of(g.tf[3]), ff_mul(FF{row, 0.0f}, ff_of(g.tf[4])));
+    const FF z = ff_of(g.tf[2]);
+    const FF gg = ff_sqrt0(ff_add(ff_sqr(r), ff_neg(ff_sqr(z))));
+    const FF ph = ff_mul(ff_neg(K), r);
+    float psi = (ph.h - rintf(ph.h)) + ph.l;
+    psi -= rintf(psi);
+    const float dh = gg.h - r0v.x, dl = gg.l - r0v.y;  // nearby values: dh is exact
+    MergeRow R;
+    float p, e;
+    two_prod(dh, dl, c0v.x, c0v.y, p, e);
+    R.o.x = side * p;
+    R.o.z = side * e;
+    two_prod(dh, dl, c0v.z, c0v.w, p, e);
+    R.o.y = p;
+    R.o.w = e;
+    quantize_pair(R.o.x, R.o.z, q, iq);
+    quantize_pair(R.o.y, R.o.w, q, iq);
+    const float h = g.tf[4].x, gf = gg.h, ig = 1.0f / gf, zh = z.h * h * ig;
+    R.p = make_float4(dh + dl, psi, off * h, gf);
+    R.w.x = h * r.h * ig;
+    R.w.y = -0.5f * zh * zh * ig;
+    R.w.z = -R.w.y * R.w.x * ig;
+    R.w.w = 0.0f;
+    return R;
+}
+
+// The tables of a merge tile: its runs' middles and its columns, in FP32 two-float arithmetic from the node's
+// geometry and column table, with the offsets quantized on the tile's quantum (q, iq).
+template <int THREADS>
+__device__ __forceinline__ void setup_merge(FF K, const Job& J, MergeTab& T, const float4* __restrict__ tables, float q,
+                                            float iq) {
+    const PolarDesc& g = J.g;
+    const int tid = threadIdx.x;
+    const int cols_t = 1 << J.lc, rows_t = kSplitTilePixels >> J.lc;
+    float4 r0v, c0v;
+    int j0;
+    tab_centre(g, J.lc, J.tile_r, J.tile_u, tables, r0v, c0v, j0);
+    const float side = (float)g.side;
+    static_assert(kMergeRows + kMaxCols <= THREADS, "one run's middle or column per thread");
+    if (tid < rows_t / kMergeRun) {
+        const int i0 = min(g.win_r0 + J.tile_r + (rows_t >> 1), g.nr - 1), i = g.win_r0 + J.tile_r + kMergeRun * tid;
+        T.row[tid] = merge_row(K, g, r0v, c0v, (float)i + 0.5f * (kMergeRun - 1),
+                               (float)(i - i0) + 0.5f * (kMergeRun - 1), q, iq);
+    }
+    const int c = tid - kMergeRows;
+    if (c >= 0 && c < cols_t) {
+        const int j = min(g.win_u0 + J.tile_u + c, g.nu - 1);
+        TabCol C = tab_col(g, tables, r0v, c0v, j, j0);
+        quantize_pair(C.cxh, C.cxl, q, iq);
+        quantize_pair(C.cyh, C.cyl, q, iq);
+        const float4 cv = __ldg(tables + g.cols_off + j);
+        T.col[c].o = make_float4(C.cxh, C.cyh, C.cxl, C.cyl);
+        T.col[c].p = make_float4(C.dcs, C.duu, side * (cv.x + cv.y), cv.z + cv.w);
+    }
+    __syncthreads();
+}
+
+// The middle of a run: its offset from the tile centre and its row's and column's values.
+struct MergeRun {
+    Pix x;  // dx, dy, their parts, d2, psi
+    float rho, g, g1, g2, g3, ex, ey;
+};
+
+__device__ __forceinline__ MergeRun merge_run(const MergeRow& R, const MergeCol& C) {
+    const float4 ro = R.o, rp = R.p, rw = R.w, co = C.o, cp = C.p;
+    MergeRun m;
+    m.x.dxh = ro.x + co.x;  // exact: both multiples of the quantum
+    m.x.dyh = ro.y + co.y;
+    m.x.dxl = fmaf(rp.x, cp.x, ro.z + co.z);
+    m.x.dyl = fmaf(rp.x, cp.y, ro.w + co.w);
+    m.x.dx = m.x.dxh + m.x.dxl;
+    m.x.dy = m.x.dyh + m.x.dyl;
+    m.x.d2 = fmaf(m.x.dx, m.x.dx, m.x.dy * m.x.dy);
+    m.x.psi = rp.y;
+    m.rho = rp.z;
+    m.g = rp.w;
+    m.g1 = rw.x;
+    m.g2 = rw.y;
+    m.g3 = rw.z;
+    m.ex = cp.z;
+    m.ey = cp.w;
+    return m;
+}
+
+// A child along a run: range place ir + m + 1/2 + (r0 + r1 m + r2 m^2) and angle place iu + (u0 + u1 m + ...), in
+// bins from the record's, and the phase (radians), as polynomials in m.
+struct ChildRun {
+    int ir, iu;
+    float r0, r1, r2;
+    float u0, u1, u2;
+    float p0, p1, p2;
+    int at, row;  // staged: index in the footprint that the bits of the rounded places add to, and the row length
+    bool inside;  // every stencil of the run lies where the child's bounds say
+    bool ahead;   // the run lies in front of the child's origin
+};
+
+__device__ __forceinline__ ChildRun child_run(FF K, float h, const MergeChild& C, const MergeRun& m) {
+    const ChildRec& R = C.r;
+    ChildRun o;
+    const float4 ra = R.a, rb = R.b, rc = R.c, re = R.e;
+    const float2 rd = make_float2(R.d.x, R.d.y);
+    // K L = tb + tl turns with tb exact, and so the range place below: an FP32 L would be off by 1e-6 bins.
+    const float L = fmaf(rb.x, m.x.dx, rb.y * m.x.dy);
+    const float q2 = fmaf(-L, L, m.x.d2);
+    const float B = rcp_approx(fmaf(2.0f, L, rb.z));
+    const float e0 = q2 * B;
+    const float eps = fmaf(-e0 * e0, B, e0);
+    const float Le = L + eps;
+    const float tb = fmaf(ra.x, m.x.dxh, ra.y * m.x.dyh);
+    float tl = fmaf(ra.x, m.x.dxl, ra.y * m.x.dyl);
+    tl = fmaf(ra.z, m.x.dx, tl);
+    tl = fmaf(ra.w, m.x.dy, tl);
+    const float tot = (tb - round_magic(tb)) + ((fmaf(K.h, eps, rc.x) + tl) + m.x.psi);
+    o.p0 = (tot - round_magic(tot)) * kTwoPiF;
+    const float iR = rcp_approx(fmaf(0.5f, rb.z, Le));
+    const float q = fmaf(m.ex, re.x, m.ey * re.y);
+    const float d1 = fmaf(h, (re.z + m.rho) - Le, q * m.g1) * iR;
+    const float r1 = h + d1;
+    const float r2 = fmaf(-d1, h + r1, 2.0f * q * m.g2) * (0.5f * iR);
+    const float r3 = fmaf(-r1, r2, q * m.g3) * iR;
+    const float k2 = K.h * kTwoPiF;
+    o.p1 = k2 * fmaf(9.25f, r3, d1);
+    o.p2 = k2 * r2;
+    const float pb = tb * C.bins.x, pr = round_magic(pb);
+    float fr = (pb - pr) + fmaf(tb, C.bins.x, -pb);
+    fr = fmaf(tb, C.bins.y, fr);
+    fr = fmaf(tl, C.bins.x, fr);
+    fr = fmaf(eps, R.inv_sdr, fr) + rb.w;
+    o.ir = (int)pr;
+    o.r0 = fr - 0.5f;
+    o.r1 = fmaf(d1, R.inv_sdr, fmaf(h, R.inv_sdr, -1.0f));
+    o.r2 = r2 * R.inv_sdr;
+    const float Lg = fmaf(rc.y, m.x.dx, rc.z * m.x.dy);
+    const float q2h = fmaf(-Lg, Lg, m.x.d2);
+    const float Bh = rcp_approx(fmaf(2.0f, Lg, rc.w));
+    const float eh = q2h * Bh;
+    const float dG = Lg + fmaf(-eh * eh, Bh, eh);
+    const float gp = rd.x + dG;
+    const float iG = rcp_approx(gp);
+    const float duu = fmaf(-rc.z, dG, m.x.dy) * iG;
+    const float pu = fmaf(duu, R.inv_sdu, rd.y), ur = round_magic(pu);
+    o.iu = (int)ur;
+    o.u0 = pu - ur;
+    const float cs = (m.g + q) * iG, up = rc.z + duu;
+    const float a = fmaf(-up, cs, m.ey), us = up * fmaf(-cs, cs, 1.0f);
+    const float n1 = m.g1 * iG, n2 = m.g2 * iG, n3 = m.g3 * iG;
+    const float a2 = -fmaf(cs, a, 0.5f * us), a3 = fmaf(fmaf(1.5f * cs, cs, -0.5f), a, us * cs);
+    const float as = a * R.inv_sdu;
+    const float u3 = fmaf(fmaf(a3, n1 * n1, 2.0f * a2 * n2) * R.inv_sdu, n1, as * n3);
+    o.u1 = fmaf(9.25f, u3, as * n1);
+    o.u2 = fmaf(a2 * R.inv_sdu, n1 * n1, as * n2);
+    const float wr = fmaf(12.25f, fabsf(o.r2), 3.5f * fabsf(o.r1 + 1.0f));
+    const float wu = fmaf(12.25f, fabsf(o.u2), 3.5f * fabsf(o.u1));
+    // The first tap of the run's upper pixel, less the places' rounding constant (wrapping arithmetic).
+    o.row = R.bw;
+    o.at = (int)((unsigned)R.bw * (unsigned)(o.ir + R.ir0 - kMergeRun / 2 - R.br0 - kMagicBits) +
+                 (unsigned)(o.iu + R.iu0 - 1 - R.bu0 - kMagicBits)) + C.box;
+    o.ahead = gp > 0.0f;
+    o.inside = o.ahead && pr + fr - wr >= C.lo_r && pr + fr + wr <= C.hi_r && pu - wu >= C.lo_u && pu + wu <= C.hi_u;
+    return o;
+}
+
+// The child image at bins (ir, iu) and fractions (sr, su); 0 where the stencil leaves it.
+template <int SRC>
+__device__ __forceinline__ float2 child_gather(const ChildRec& R, int ir, int iu, float sr, float su, bool ahead) {
+    if (!(ir >= 1 && ir <= R.snr - 3 && iu >= 1 && iu <= R.snu - 3 && ahead)) return make_float2(0.0f, 0.0f);
+    float wr[4], wu[4];
+    lagrange_centred(sr, wr);
+    lagrange_centred(su, wu);
+    return child_stencil<SRC>(R.img + (size_t)(ir - 1) * R.sstr + (iu - 1), R.sstr, wr, wu);
+}
+
+// Child C at the parent rows m and m + 1 of a run (the two lanes of f32x2 operations), rotated, with the weights,
+// the sum order and the shared 5x4 blocks of child_vpair.  boxes (STAGED): the staged footprints; a warp
+// whose runs lie inside the child's (`inside`, for all its lanes) reads shared memory, any other warp the child
+// image.  The taps are the same values either way.
+template <bool COHERENT, bool STAGED>
+__device__ __forceinline__ void child_pair(const MergeChild& C, const ChildRun& t, bool inside, int k, float m, float2& oA,
+                                           float2& oB, const float2* boxes) {
+    constexpr int SRC = COHERENT ? kCoherent : kLdg;
+    const float2 magic = pair(kMagic), nmagic = pair(-kMagic), mone = pair(-1.0f);
+    const float n = m + 1.0f;
+    const float2 qr = make_float2(fmaf(fmaf(t.r2, m, t.r1), m, t.r0), fmaf(fmaf(t.r2, n, t.r1), n, t.r0));
+    const float2 qu = make_float2(fmaf(fmaf(t.u2, m, t.u1), m, t.u0), fmaf(fmaf(t.u2, n, t.u1), n, t.u0));
+    const float2 tr = __fadd2_rn(qr, magic), tu = __fadd2_rn(qu, magic);
+    const float2 sr = __ffma2_rn(__fadd2_rn(tr, nmagic), mone, qr);
+    const float2 su = __ffma2_rn(__fadd2_rn(tu, nmagic), mone, qu);
+    float snA, csA, snB, csB;
+    __sincosf(fmaf(fmaf(t.p2, m, t.p1), m, t.p0), &snA, &csA);
+    __sincosf(fmaf(fmaf(t.p2, n, t.p1), n, t.p0), &snB, &csB);
+    float2 vA = make_float2(0.0f, 0.0f), vB = vA;
+    const bool share = __float_as_int(tr.y) == __float_as_int(tr.x) && __float_as_int(tu.y) == __float_as_int(tu.x);
+    const bool block = inside && __all_sync(0xffffffffu, share);
+    if (block) {
+        float wrA[4], wuA[4], wrB[4], wuB[4];
+        float2 wr2[4], wu2[4];
+        lagrange_centred2(sr, wr2);  // both pixels' weights as lane pairs
+        lagrange_centred2(su, wu2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            wrA[k] = wr2[k].x;
+            wrB[k] = wr2[k].y;
+            wuA[k] = wu2[k].x;
+            wuB[k] = wu2[k].y;
+        }
+        if (STAGED) {
+            const int at = (int)((unsigned)(__float_as_int(tr.x) + 2 * k) * (unsigned)t.row + (unsigned)__float_as_int(tu.x)) + t.at;
+            child_pair_block<kShared>(boxes + at, t.row, wrA, wuA, wrB, wuB, vA, vB);
+        } else {
+            const int ir = __float_as_int(tr.x) + t.ir + C.r.ir0 + 2 * k - kMergeRun / 2 - kMagicBits;
+            const int iu = __float_as_int(tu.x) + t.iu + C.r.iu0 - 1 - kMagicBits;
+            child_pair_block<SRC>(C.r.img + (size_t)ir * C.r.sstr + iu, C.r.sstr, wrA, wuA, wrB, wuB, vA, vB);
+        }
+    } else if (STAGED && inside) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            float wr[4], wu[4];
+            lagrange_centred(c ? sr.y : sr.x, wr);
+            lagrange_centred(c ? su.y : su.x, wu);
+            const int at = (int)((unsigned)(__float_as_int(c ? tr.y : tr.x) + 2 * k + c) * (unsigned)t.row +
+                                 (unsigned)__float_as_int(c ? tu.y : tu.x)) + t.at;
+            (c ? vB : vA) = child_stencil<kShared>(boxes + at, t.row, wr, wu);
+        }
+    } else {
+    const int ir0 = t.ir + C.r.ir0 + 2 * k - (kMergeRun / 2 - 1) - kMagicBits, iu0 = t.iu + C.r.iu0 - kMagicBits;  // of the upper pixel
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            (c ? vB : vA) = child_gather<SRC>(C.r, __float_as_int(c ? tr.y : tr.x) + ir0 + c, __float_as_int(c ? tu.y : tu.x) + iu0,
+                                              c ? sr.y : sr.x, c ? su.y : su.x, t.ahead);
+    }
+    // (vr cs - vi sn, vr sn + vi cs)
+    oA = __ffma2_rn(pair(vA.x), make_float2(csA, snA), __fmul2_rn(pair(vA.y), make_float2(-snA, csA)));
+    oB = __ffma2_rn(pair(vB.x), make_float2(csB, snB), __fmul2_rn(pair(vB.y), make_float2(-snB, csB)));
+}
+
 // Bytes of a merge tile's tables in dynamic shared memory (the staged footprints follow them).
 constexpr int kTabBytes = (int)((sizeof(TabF) + 127) / 128 * 128);
+static_assert(sizeof(MergeTab) <= sizeof(TabF), "either kind of tables");
 
 // Staged merge tiles: one thread starts the TMA copies of both children's footprints (2-D tiles
 // of the child images, the box's first column even so that it starts on a 16-byte boundary;
@@ -3260,28 +3570,28 @@ __device__ __forceinline__ void stage_children(const ChildRec* __restrict__ crec
 
 // One merge tile: both children regridded onto the parent tile, each rounded to complex64,
 // then added (the reference's rounding points).  crec points at the tile's two child records.
-// Thread t of THREADS forms the column pairs (rows 2 m and 2 m + 1 of column t mod cols) for
-// m = t / cols + i THREADS / cols; its offsets come back from the shared tables per pair, which
+// Thread t of kMergeThreads forms the column pairs (rows 2 m and 2 m + 1 of column t mod cols) for
+// m = t / cols + i kMergeThreads / cols; its offsets come back from the shared tables per pair, which
 // keeps the live state small.
 // STAGED: smem is 128-byte aligned and holds [tables | child 0's footprint | child 1's], which
 // stage_children's copies fill (completion on the mbarrier at shared address bar).  Each warp
 // waits for them, at most wait_ns; a warp whose wait runs out counts a timeout and gathers from
 // the child images instead (the same values), and waits once more, as long, before the CTA ends,
 // so that no copy into its shared memory is still in flight when it exits.
-template <bool COHERENT = false, int THREADS = kThreads, bool STAGED = false>
-__device__ __forceinline__ void merge_tile(float Kf, const PolarDesc* __restrict__ nodes, const TileItem it,
+template <bool COHERENT, bool STAGED>
+__device__ __forceinline__ void merge_tile_pairs(float Kf, const PolarDesc& g, const TileItem it,
                                            const float4* __restrict__ tables, const ChildRec* __restrict__ crec,
                                            ChildDup* C, float2* __restrict__ arena, float2* root_out, int root,
-                                           char* smem, unsigned bar = 0, unsigned long long wait_ns = 0) {
+                                           char* smem, unsigned bar, unsigned long long wait_ns) {
     Job J;
-    J.g = nodes[it.node];
+    J.g = g;
     J.lc = J.g.tile_lc;
     J.tile_r = it.tile_r;
     J.tile_u = it.tile_u;
     if (threadIdx.x < 2) child_dup_store(crec[threadIdx.x], C[threadIdx.x]);
     const float4 d0 = __ldg(&crec[0].d);  // (G, frac(Qu) - 1/2, tile quantum, its inverse)
     TabF& T = *reinterpret_cast<TabF*>(smem);
-    setup_polar_tab<THREADS>(J, T, tables, d0.z, d0.w);
+    setup_polar_tab<kMergeThreads>(J, T, tables, d0.z, d0.w);
     const float2* sbox[2] = {nullptr, nullptr};
     bool waited = true;
     if (STAGED && (C[0].xw > 0 || C[1].xw > 0)) {
@@ -3297,14 +3607,14 @@ __device__ __forceinline__ void merge_tile(float Kf, const PolarDesc* __restrict
     }
     float2* dst = J.g.dst ? J.g.dst : (it.node == root ? root_out : arena + J.g.out_offset);
     const int col = threadIdx.x & ((1 << J.lc) - 1), wu = J.tile_u + col;
-    constexpr int kPairs = kSplitTilePixels / (2 * THREADS);  // column pairs per thread
+    constexpr int kPairs = kSplitTilePixels / (2 * kMergeThreads);  // column pairs per thread
     float2 m[2 * kPairs];
     // Gathering tiles keep all their pairs' gathers in flight (unrolled); staged tiles read shared
     // memory with short latency, and the smaller loop body keeps their instruction cache warm.
     constexpr int kUnroll = STAGED ? 1 : kPairs;
 #pragma unroll kUnroll
     for (int k = 0; k < kPairs; ++k) {
-        const int row = 2 * ((threadIdx.x >> J.lc) + (THREADS >> J.lc) * k);
+        const int row = 2 * ((threadIdx.x >> J.lc) + (kMergeThreads >> J.lc) * k);
         const VPix v = tab_vpair(T, row, col);
         float2 a0, b0, a1, b1;
         child_vpair<COHERENT, STAGED>(Kf, C[0], v, a0, b0, sbox[0]);
@@ -3326,7 +3636,7 @@ __device__ __forceinline__ void merge_tile(float Kf, const PolarDesc* __restrict
     if (COHERENT) {
 #pragma unroll
         for (int k = 0; k < kPairs; ++k) {
-            const int wr = J.tile_r + 2 * ((threadIdx.x >> J.lc) + (THREADS >> J.lc) * k);
+            const int wr = J.tile_r + 2 * ((threadIdx.x >> J.lc) + (kMergeThreads >> J.lc) * k);
             if (wu < J.g.win_nu) {
                 if (wr < J.g.win_nr) dst[(long long)wr * J.g.out_stride + wu] = m[2 * k];
                 if (wr + 1 < J.g.win_nr) dst[(long long)(wr + 1) * J.g.out_stride + wu] = m[2 * k + 1];
@@ -3336,6 +3646,92 @@ __device__ __forceinline__ void merge_tile(float Kf, const PolarDesc* __restrict
     if (STAGED && !waited) timed_wait(bar, 0, wait_ns);  // the copies may still land: not past the CTA's end
 }
 
+// The same in runs of rows: thread t forms rows 8 m ... 8 m + 7 of column t mod cols for m = t / cols, in pairs.
+template <bool COHERENT, bool STAGED>
+__device__ __forceinline__ void merge_tile_runs(FF K, const PolarDesc* __restrict__ nodes, const PolarDesc& g,
+                                                const TileItem it, const float4* __restrict__ tables,
+                                                const ChildRec* __restrict__ crec, MergeChild* C,
+                                                float2* __restrict__ arena, float2* root_out, int root, char* smem,
+                                                unsigned bar, unsigned long long wait_ns) {
+    Job J;
+    J.g = g;
+    J.lc = J.g.tile_lc;
+    J.tile_r = it.tile_r;
+    J.tile_u = it.tile_u;
+    if (threadIdx.x < 2)
+        merge_child(K, nodes[threadIdx.x ? g.right : g.left], crec[threadIdx.x],
+                    STAGED && threadIdx.x && crec[0].bw > 0 ? (int)split_box_bytes(crec[0].bh, crec[0].bw) / 8 : 0,
+                    C[threadIdx.x]);
+    const float4 d0 = __ldg(&crec[0].d);  // (G, frac(Qu) - 1/2, tile quantum, its inverse)
+    MergeTab& T = *reinterpret_cast<MergeTab*>(smem);
+    setup_merge<kMergeThreads>(K, J, T, tables, d0.z, d0.w);
+    // Staged: the footprints, and the second one's offset (elements) when both are there.
+    const float2* boxes = reinterpret_cast<const float2*>(smem + kTabBytes);
+    bool waited = true;
+    if (STAGED && (C[0].r.bw > 0 || C[1].r.bw > 0)) {
+        waited = __all_sync(0xffffffffu, timed_wait(bar, 0, wait_ns));
+        if (!waited && (threadIdx.x & 31) == 0) atomicAdd(&g_wait_timeouts, 1);
+    }
+    float2* dst = J.g.dst ? J.g.dst : (it.node == root ? root_out : arena + J.g.out_offset);
+    const int col = threadIdx.x & ((1 << J.lc) - 1), run = threadIdx.x >> J.lc;
+    const int wu = J.tile_u + col, wr = J.tile_r + kMergeRun * run;
+    const int rows = wu < J.g.win_nu ? J.g.win_nr - wr : 0;  // of the run, in the window
+    float2* px = dst + (long long)wr * J.g.out_stride + wu;
+    float2 v[kMergeRun];
+    const float h = J.g.tf[4].x;
+    const ChildRun t0 = child_run(K, h, C[0], merge_run(T.row[run], T.col[col]));
+    asm volatile("" ::: "memory");
+    const ChildRun t1 = child_run(K, h, C[1], merge_run(T.row[run], T.col[col]));
+    const bool in0 = __all_sync(0xffffffffu, t0.inside && (!STAGED || (waited && C[0].r.bw > 0)));
+    const bool in1 = __all_sync(0xffffffffu, t1.inside && (!STAGED || (waited && C[1].r.bw > 0)));
+    // A small loop body keeps the instruction cache warm; coherent tiles keep their results in registers.
+    constexpr int kPairs = kMergeRun / 2, kUnroll = COHERENT ? kPairs : 1;
+    float x = -0.5f * (kMergeRun - 1);
+#pragma unroll kUnroll
+    for (int k = 0; k < kPairs; ++k, x += 2.0f) {
+        float2 a0, b0, a1, b1;
+        child_pair<COHERENT, STAGED>(C[0], t0, in0, k, x, a0, b0, boxes);
+        child_pair<COHERENT, STAGED>(C[1], t1, in1, k, x, a1, b1, boxes);
+        const float2 mA = __fadd2_rn(a0, a1), mB = __fadd2_rn(b0, b1);
+        if (!COHERENT) {
+            if (2 * k < rows) px[0] = mA;
+            if (2 * k + 1 < rows) px[J.g.out_stride] = mB;
+            px += 2 * J.g.out_stride;
+        } else {
+            // Coherent child loads may not pass this thread's earlier image stores, so the
+            // results are stored after the last gather.
+            v[2 * k] = mA;
+            v[2 * k + 1] = mB;
+        }
+    }
+    if (COHERENT) {
+#pragma unroll
+        for (int k = 0; k < kMergeRun; ++k)
+            if (k < rows) px[k * J.g.out_stride] = v[k];
+    }
+    if (STAGED && !waited) timed_wait(bar, 0, wait_ns);  // the copies may still land: not past the CTA's end
+}
+
+// The children of a merge tile in shared memory, for either kind.
+union MergeChildren {
+    __device__ MergeChildren() {}
+    ChildDup dup[2];
+    MergeChild run[2];
+};
+
+// One merge tile; KIND: kMergeRuns or kMergePairs where the caller knows that the node merges so.
+template <bool COHERENT = false, bool STAGED = false, int KIND = kMergeEither>
+__device__ __forceinline__ void merge_tile(FF K, const PolarDesc* __restrict__ nodes, const TileItem it,
+                                           const float4* __restrict__ tables, const ChildRec* __restrict__ crec,
+                                           MergeChildren& C, float2* __restrict__ arena, float2* root_out, int root,
+                                           char* smem, unsigned bar = 0, unsigned long long wait_ns = 0) {
+    const PolarDesc& g = nodes[it.node];
+    if (KIND == kMergeRuns || (KIND == kMergeEither && merges_in_runs(g, K.h)))
+        merge_tile_runs<COHERENT, STAGED>(K, nodes, g, it, tables, crec, C.run, arena, root_out, root, smem, bar, wait_ns);
+    else
+        merge_tile_pairs<COHERENT, STAGED>(K.h, g, it, tables, crec, C.dup, arena, root_out, root, smem, bar, wait_ns);
+}
+
 __global__ void __launch_bounds__(kMergeThreads, 8) split_merge_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
                                                                   const TileItem* __restrict__ items,
                                                                   const float4* __restrict__ tables,
@@ -3343,15 +3739,16 @@ __global__ void __launch_bounds__(kMergeThreads, 8) split_merge_kernel(SplitPara
                                                                   float2* __restrict__ arena, float2* root_out,
                                                                   int root) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ ChildDup C[2];
-    merge_tile<false, kMergeThreads>(P.Kf, nodes, items[blockIdx.x], tables, crecs + 2 * (long long)blockIdx.x, C, arena,
+    __shared__ MergeChildren C;
+    merge_tile<false>(FF{P.Kh, P.Kl}, nodes, items[blockIdx.x], tables, crecs + 2 * (long long)blockIdx.x, C, arena,
                                      root_out, root, smem);
 }
 
 // The merge with both children's footprints staged in shared memory by TMA (tiles whose child
 // records carry tensor maps; any other child gathers from its image as in split_merge_kernel).
 // The dynamic shared memory is 128 bytes of alignment slack, the tables and the footprints.
-__global__ void __launch_bounds__(kMergeThreads, 8) split_merge_staged_kernel(SplitParams P,
+template <int KIND>
+__global__ void __launch_bounds__(kMergeThreads, KIND == kMergeRuns ? 6 : 8) split_merge_staged_kernel(SplitParams P,
                                                                          const PolarDesc* __restrict__ nodes,
                                                                          const TileItem* __restrict__ items,
                                                                          const float4* __restrict__ tables,
@@ -3360,7 +3757,7 @@ __global__ void __launch_bounds__(kMergeThreads, 8) split_merge_staged_kernel(Sp
                                                                          float2* root_out, int root,
                                                                          unsigned long long wait_ns, int withheld) {
     extern __shared__ __align__(128) char smem_raw[];
-    __shared__ ChildDup C[2];
+    __shared__ MergeChildren C;
     __shared__ __align__(8) unsigned long long mbar;
     const unsigned raw = (unsigned)__cvta_generic_to_shared(smem_raw);
     char* smem = smem_raw + (((raw + 127u) & ~127u) - raw);
@@ -3369,7 +3766,7 @@ __global__ void __launch_bounds__(kMergeThreads, 8) split_merge_staged_kernel(Sp
     const TileItem it = items[blockIdx.x];
     if (threadIdx.x == 0)
         stage_children(crec, (unsigned)__cvta_generic_to_shared(smem + kTabBytes), bar, it.node == withheld ? 16u : 0u);
-    merge_tile<false, kMergeThreads, true>(P.Kf, nodes, it, tables, crec, C, arena, root_out, root, smem, bar, wait_ns);
+    merge_tile<false, true, KIND>(FF{P.Kh, P.Kl}, nodes, it, tables, crec, C, arena, root_out, root, smem, bar, wait_ns);
 }
 
 // All merge levels in one persistent launch.  Items are in height order; a CTA claims the next
@@ -3384,14 +3781,14 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
 }
 
 
-__global__ void __launch_bounds__(kThreads, 4) split_merge_queue_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
+__global__ void __launch_bounds__(kMergeThreads, 6) split_merge_queue_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
                                                                         const TileItem* __restrict__ items, int nitems,
                                                                         const float4* __restrict__ tables,
                                                                         const ChildRec* __restrict__ crecs,
                                                                         float2* arena, float2* root_out, int root,
                                                                         MergeQueue Q) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ ChildDup C[2];
+    __shared__ MergeChildren C;
     __shared__ int s_item, s_ok;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -3420,7 +3817,7 @@ __global__ void __launch_bounds__(kThreads, 4) split_merge_queue_kernel(SplitPar
         const int idx = s_item;
         if (idx >= nitems || !s_ok) return;
         const TileItem it = items[idx];
-        merge_tile<true>(P.Kf, nodes, it, tables, crecs + 2 * (long long)idx, C, arena, root_out, root, smem);
+        merge_tile<true>(FF{P.Kh, P.Kl}, nodes, it, tables, crecs + 2 * (long long)idx, C, arena, root_out, root, smem);
         __syncthreads();  // every thread's writes of this tile are issued
         if (threadIdx.x == 0) {
             __threadfence();
@@ -3581,12 +3978,46 @@ int split_polar_tile_lc_slack(const PolarDesc& g, double slack, double* radius) 
     return best;
 }
 
+float split_merge_run_limit(const PolarDesc& g, const PolarDesc* children[2]) {
+    // Nearest and farthest rows, widest column of the window (its last tiles' overhang included).
+    const int rows_t = kSplitTilePixels >> g.tile_lc, cols_t = 1 << g.tile_lc;
+    const double ra = g.r0 + g.win_r0 * g.dr, rb = ra + (g.win_nr - 1 + rows_t) * g.dr, z = fabs(g.oz);
+    const double r0 = fmin(ra, rb), r1 = fmax(ra, rb), h = fabs(g.dr);
+    const double ua = fabs(g.u0 + g.win_u0 * g.du), ub = fabs(g.u0 + (g.win_u0 + g.win_nu - 1) * g.du);
+    const double um = fmax(ua, ub), cm = sqrt(fmax(1e-12, 1.0 - um * um)), m = 0.5 * (kMergeRun - 1), m4 = m * m * m * m;
+    if (!(r0 - 8.0 * h > z) || !(um < 1.0)) return 0.0f;
+    const double gn = sqrt((r0 - 8.0 * h) * (r0 - 8.0 * h) - z * z), gf = sqrt(r1 * r1 - z * z), ig = 1.0 / gn;
+    // K at which the FP32 rounding of eps (1e-8 of K rho^2 / R) stays below 6e-8 turns.
+    const double er = 0.5 * rows_t * h * r0 * ig, eu = 0.5 * cols_t * fabs(g.du) * gf / cm, rho2 = er * er + eu * eu;
+    double limit = 6.0 * r0 / rho2;
+    for (int k = 0; k < 2; ++k) {
+        const PolarDesc& c = *children[k];
+        const double dx = g.ox - c.ox, dy = g.oy - c.oy, dz = fabs(g.oz - c.oz), off = sqrt(dx * dx + dy * dy);
+        const double q = fabs(dx) + um * fabs(dy);
+        if (!(gn > 4.0 * off) || !(r0 > 4.0 * (off + dz))) return 0.0f;
+        // What child_run leaves out at a run's ends: of the phase and of the angle place the fourth order and the
+        // third beyond its linear fit (10.5 of m^3), of the range place the third.
+        const double id = 1.0 / (r0 - off - dz), iG = 1.0 / (gn - off);
+        const double x = h * r0 * ig, y2 = h * h * z * z * ig * ig;  // the step of g; g_2 = y2 / 2 g
+        const double f2 = q * y2 * ig, f3 = f2 * x * ig, f4 = 1.25 * f3 * x * ig;
+        const double d1 = h * (off + dz + q * r0 * ig) * id, r2 = (f2 + 3.0 * h * d1) * id, r3 = (f3 + 2.0 * h * r2) * id;
+        const double turns = 10.5 * r3 + m4 * (f4 + 2.0 * h * r3 + r2 * r2) * id;  // per K
+        const double n1 = x * iG, n2 = 0.5 * y2 * ig * iG, n3 = n2 * x * ig;
+        const double angle = 2.0 * off * iG / fabs(c.du) *
+                             (10.5 * (n3 + 2.0 * n1 * n2 + n1 * n1 * n1) +
+                              m4 * (1.25 * n3 * x * ig + 2.0 * n1 * n3 + n2 * n2 + 3.0 * n1 * n1 * n2 + n1 * n1 * n1 * n1));
+        if (!(m * m * m * r3 / fabs(c.dr) <= 2e-6) || !(angle <= 2e-6)) return 0.0f;
+        limit = fmin(limit, 3e-7 / fmax(turns, 1e-30));
+    }
+    return (float)limit;
+}
+
 int launch_split_polar(const PulseInputs& in, const PolarDesc& g, int pulse_split, int chunk, int window_bins,
                        float2* out, long long out_stride, long long split_stride, cudaStream_t s) {
     // Runs of columns need tiles at least a run wide and an angle step at which the expansion holds for any
     // pulse the grid resolves (K |a| du below half a turn: 0.5 du^4 turns at fifth order).
     const double ua = fabs(g.u0 + g.win_u0 * g.du), ub = fabs(g.u0 + (g.win_u0 + g.win_nu - 1) * g.du);
-    const bool runs = g.tile_lc >= 3 && fabs(g.du) <= 0.002 * (1.0 - fmax(ua, ub) * fmax(ua, ub));
+    const bool runs = g.tile_lc >= 3 && fabs(in.k) > 1e-2 && fabs(g.du) <= 0.002 * (1.0 - fmax(ua, ub) * fmax(ua, ub));
     int cap = capacity_for(chunk, window_bins);
     if (runs) cap = std::max(cap, kSplitTilePixels * (int)sizeof(float2) / 32);  // the halves' exchange
     SplitParams P = make_params(in, chunk, cap, pulse_split);
@@ -3727,7 +4158,7 @@ int launch_split_ffbp_leaves(const PulseInputs& in, const PolarDesc* nodes, cons
 
 int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* items, int nitems,
                              const float4* tables, const void* crecs, float2* arena, float2* root_out, int root,
-                             size_t box_bytes, unsigned long long wait_ns, int withheld, cudaStream_t s) {
+                             size_t box_bytes, unsigned long long wait_ns, int withheld, int kind, cudaStream_t s) {
     if (nitems <= 0) return SARBP_OK;
     PulseInputs none{};
     none.k = k;
@@ -3735,8 +4166,11 @@ int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* i
     SplitParams P = make_params(none, 1, 4, 1);
     if (box_bytes > 0) {
         const size_t smem = 128 + kTabBytes + box_bytes;
-        if (int st = prepare(split_merge_staged_kernel, smem)) return st;
-        split_merge_staged_kernel<<<nitems, kMergeThreads, smem, s>>>(
+        const auto kernel = kind == kMergeRuns    ? split_merge_staged_kernel<kMergeRuns>
+                            : kind == kMergePairs ? split_merge_staged_kernel<kMergePairs>
+                                                  : split_merge_staged_kernel<kMergeEither>;
+        if (int st = prepare(kernel, smem)) return st;
+        kernel<<<nitems, kMergeThreads, smem, s>>>(
             P, nodes, items, tables, reinterpret_cast<const ChildRec*>(crecs), arena, root_out, root, wait_ns, withheld);
         note_launches(1);
         return check_launch("split_ffbp_merges (staged)");
@@ -3763,10 +4197,10 @@ int launch_split_ffbp_merge_queue(double k, const PolarDesc* nodes, const TileIt
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, split_merge_queue_kernel, kThreads, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, split_merge_queue_kernel, kMergeThreads, smem);
     if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "merge queue: %s", cudaGetErrorString(e));
     const int blocks = std::max(1, std::min(nitems, sms * std::max(1, per_sm)));
-    split_merge_queue_kernel<<<blocks, kThreads, smem, s>>>(P, nodes, items, nitems, tables,
+    split_merge_queue_kernel<<<blocks, kMergeThreads, smem, s>>>(P, nodes, items, nitems, tables,
                                                             reinterpret_cast<const ChildRec*>(crecs), arena,
                                                             root_out, root, Q);
     note_launches(1);
@@ -3920,13 +4354,14 @@ __global__ void __launch_bounds__(kMergeThreads, 8) batch_merge_kernel(const Bat
                                                                   float2* __restrict__ arena, int* counter,
                                                                   unsigned long long* trace) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ ChildDup C[2];
+    __shared__ MergeChildren C;
     __shared__ int s_item;
     for (;;) {
         const int idx = next_item(counter, s_item);
         if (idx >= nitems) return;
         const TileItem it = items[idx];
-        merge_tile<false, kMergeThreads>(scenes[it.pad].P.Kf, nodes, it, tables, crecs + 2 * (long long)idx, C, arena,
+        const SplitParams& P = scenes[it.pad].P;
+        merge_tile<false>(FF{P.Kh, P.Kl}, nodes, it, tables, crecs + 2 * (long long)idx, C, arena,
                                          nullptr, -1, smem);
         trace_item(trace, it.pad);
     }
