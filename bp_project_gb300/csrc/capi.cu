@@ -774,6 +774,14 @@ int sarbp_ffbp_plan_create(const sarbp_ffbp_node* nodes, int n_nodes, int crop_r
         delete p;
         return fail(SARBP_ERR_PLAN, "plan too large");
     }
+    // All merges of a height run alike (one kernel per launch).
+    for (int h = 1; h <= p->max_height; ++h) {
+        float run_k = INFINITY;
+        for (int i = 0; i < n_nodes; ++i)
+            if (p->height[i] == h) run_k = std::min(run_k, p->nodes[i].run_k);
+        for (int i = 0; i < n_nodes; ++i)
+            if (p->height[i] == h) p->nodes[i].run_k = run_k;
+    }
     p->leaf_chunk = leaf_pulses;
     p->node_bytes = align_up(sizeof(PolarDesc) * n_nodes);
     p->work_bytes = align_up(mode == SARBP_SPLIT ? sizeof(TileItem) * p->items.size() : sizeof(int2) * p->blocks.size());
@@ -997,13 +1005,12 @@ int sarbp_ffbp_execute(const sarbp_ffbp_plan* plan, const float* data, int pulse
         }
         for (int h = 1; h <= plan->max_height && st == SARBP_OK && !plan->merge_queue; ++h) {
             const size_t first = (size_t)(plan->stage_begin[h] - plan->stage_begin[1]);
-            int kinds = 0;
-            for (int i = 0; i < plan->n_nodes; ++i)
-                if (plan->height[i] == h) kinds |= merges_in_runs(plan->nodes[i], (float)(k * kInvTwoPi)) ? kMergeRuns : kMergePairs;
+            int node = 0;
+            while (plan->height[node] != h) ++node;
             st = launch_split_ffbp_merges(k, nodes, items + plan->stage_begin[h], plan->stage_count[h], tables,
                                           reinterpret_cast<char*>(crecs) + 2 * first * crec_size, arena, root_out, 0,
                                           plan->staged ? plan->merge_box_bytes[h] : 0, plan->queue_limit_ns,
-                                          plan->withheld, kinds == (kMergeRuns | kMergePairs) ? kMergeEither : kinds, s);
+                                          plan->withheld, merges_in_runs(plan->nodes[node], (float)(k * kInvTwoPi)), s);
         }
     } else {
         const int2* blocks = reinterpret_cast<const int2*>(base + plan->node_bytes);

@@ -120,11 +120,10 @@ inline void split_geometry(PolarDesc& d) {
     }
 }
 
-// Whether merge node g's tiles merge in runs of rows at K turns/m, and what is known of the nodes of a launch.
+// Whether merge node g's tiles merge in runs of rows at K turns/m.
 __host__ __device__ inline bool merges_in_runs(const PolarDesc& g, float K) {
     return fabsf(K) >= 1e-3f && fabsf(K) <= g.run_k;
 }
-enum MergeKind { kMergeEither = 0, kMergeRuns = 1, kMergePairs = 2 };
 
 struct TileItem {
     int node;
@@ -330,7 +329,7 @@ int launch_split_ffbp_merge_queue(double k, const PolarDesc* nodes, const TileIt
 // than their copies deliver, so that their waits run out.
 int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* items, int nitems,
                              const float4* tables, const void* crecs, float2* arena, float2* root_out, int root,
-                             size_t box_bytes, unsigned long long wait_ns, int withheld, int kind, cudaStream_t s);
+                             size_t box_bytes, unsigned long long wait_ns, int withheld, bool runs, cudaStream_t s);
 // Shared-memory bytes of one staged child footprint (rows x cols complex64, 128-byte granules).
 __host__ __device__ inline size_t split_box_bytes(int rows, int cols) { return ((size_t)rows * cols * 8 + 127) / 128 * 128; }
 // Largest staged footprint per child, 13 KB: the 32 x 32 and 16 x 64 tiles of near-range plans need

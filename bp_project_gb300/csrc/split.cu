@@ -1419,9 +1419,19 @@ __device__ void chunk_loop(const SplitParams& P, const Job& J, TileShared& S, ch
 // as long as the whole run stays within one range bin; when that holds for all the warp's runs (lim = 1/2;
 // below 0: never) the run takes one window entry (two 16-byte loads instead of sixteen), and the even and
 // odd parts of both polynomials serve the columns +m and -m.  Otherwise each pixel takes its own entry.
-__device__ __forceinline__ void column_run(float P0, float P1, float P2, float P3, float P4, float qp, float b1, float b2,
+// PARTS = 2: the thread forms half of the run's columns, the inner (part 0) or the outer four, by the same
+// arithmetic; ar[2 i + c] then belongs to column run_column<2>(part, i, c).
+template <int PARTS>
+__device__ __forceinline__ int run_column(int part, int i, int c) {
+    const int h = (PARTS == 1 ? 0 : part * (kColRun / 2 / PARTS)) + i;
+    return c ? kColRun / 2 + h : kColRun / 2 - 1 - h;
+}
+
+template <int PARTS>
+__device__ __forceinline__ void column_run(int part, float P0, float P1, float P2, float P3, float P4, float qp, float b1, float b2,
                                            float lim, const char* __restrict__ w0, unsigned bias, unsigned last,
-                                           float ar[kColRun], float ai[kColRun]) {
+                                           float ar[kColRun / PARTS],
+                                           float ai[kColRun / PARTS]) {
     const float tq = qp + kMagic;
     const float s = qp - (tq - kMagic);
     const float spread = fmaf(fabsf(b2), 12.25f, fmaf(fabsf(b1), 3.5f, fabsf(s)));
@@ -1443,14 +1453,14 @@ __device__ __forceinline__ void column_run(float P0, float P1, float P2, float P
             V3[c] = fmaf(A3, bb, 2.0f * W2 * b2) * b1;
         }
 #pragma unroll
-        for (int h = 0; h < kColRun / 2; ++h) {
-            const float m = 0.5f + h, mm = m * m;
+        for (int h = 0; h < kColRun / 2 / PARTS; ++h) {
+            const float m = (PARTS == 1 ? 0.5f : 0.5f + (float)(part * (kColRun / 2 / PARTS))) + h, mm = m * m;
             const float ae = fmaf(fmaf(P4, mm, P2), mm, P0), ao = fmaf(P3, mm, P1);
             const float re = fmaf(V2[0], mm, V0[0]), ro = fmaf(V3[0], mm, V1[0]);
             const float ie = fmaf(V2[1], mm, V0[1]), io = fmaf(V3[1], mm, V1[1]);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const int k = c ? kColRun / 2 + h : kColRun / 2 - 1 - h;
+                const int k = PARTS == 1 ? run_column<1>(0, h, c) : 2 * h + c;
                 const float x = c ? m : -m;
                 const float vr = fmaf(ro, x, re), vi = fmaf(io, x, ie);
                 float sn, cs;
@@ -1463,8 +1473,8 @@ __device__ __forceinline__ void column_run(float P0, float P1, float P2, float P
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < kColRun; ++k) {
-            const float x = (float)k - 0.5f * (kColRun - 1);
+        for (int k = 0; k < kColRun / PARTS; ++k) {
+            const float x = (float)(PARTS == 1 ? k : run_column<PARTS>(part, k / 2, k % 2)) - 0.5f * (kColRun - 1);
             const float p = fmaf(fmaf(b2, x, b1), x, qp);
             const float t = p + kMagic, f = p - (t - kMagic);
             const float4* w = reinterpret_cast<const float4*>(w0 + min(32u * (unsigned)__float_as_int(t) + bias, last));
@@ -2134,7 +2144,7 @@ struct PolarRunBody {
             float P1, P2, P3, P4;
             run_phase(q.g * iR, iR * kz, fmaf(rd.x, q.s1, rd.y * q.h), rd.x * q.s2, rd.x * q.s3, rd.x * q.s4, P1, P2, P3,
                       P4);
-            column_run(P0, P1, P2, P3, P4, fmaf(Le, inv_dr, rb.w), P1 * kd, P2 * kd, rd.z,
+            column_run<1>(0, P0, P1, P2, P3, P4, fmaf(Le, inv_dr, rb.w), P1 * kd, P2 * kd, rd.z,
                        reinterpret_cast<const char*>(win + 2 * __float_as_int(rc.z)), 0u - 32u * (unsigned)__float_as_int(rc.y),
                        32u * (unsigned)__float_as_int(rc.w), ar, ai);
         }
@@ -2583,10 +2593,11 @@ __device__ __forceinline__ LeafMid leaf_mid(const SplitParams& P, const PolarDes
     return M;
 }
 
-// The pulses of a chunk on one run.
-__device__ __forceinline__ void leaf_runs(const SplitParams& P, const LeafRec* __restrict__ rec,
+// The pulses of a chunk on one run (or its part).
+template <int PARTS>
+__device__ __forceinline__ void leaf_runs(int part, const SplitParams& P, const LeafRec* __restrict__ rec,
                                           const LeafCol* __restrict__ cols, const char* __restrict__ win, int n,
-                                          const LeafRow& q, float lim, float ar[kLeafRun], float ai[kLeafRun]) {
+                                          const LeafRow& q, float lim, float ar[kLeafRun / PARTS], float ai[kLeafRun / PARTS]) {
     const float inv_dr = P.inv_drf, Kf = P.Kf;
     const float kz = 1.0f / (kTwoPiF * Kf), kd = inv_dr * kz;
 #pragma unroll 1
@@ -2612,7 +2623,7 @@ __device__ __forceinline__ void leaf_runs(const SplitParams& P, const LeafRec* _
         const float z = iR * kz;
         float P1, P2, P3, P4;
         run_phase(at, z, cb.x, cb.y, cb.z, cb.w, P1, P2, P3, P4);
-        column_run(P0, P1, P2, P3, P4, fmaf(dd, inv_dr, q.fm), P1 * kd, P2 * kd, lim, win + __float_as_int(rb.z),
+        column_run<PARTS>(part, P0, P1, P2, P3, P4, fmaf(dd, inv_dr, q.fm), P1 * kd, P2 * kd, lim, win + __float_as_int(rb.z),
                    32u * (unsigned)q.o + (unsigned)__float_as_int(rb.y), (unsigned)__float_as_int(rb.w), ar, ai);
     }
 }
@@ -2671,7 +2682,9 @@ __device__ __noinline__ void leaf_direct(const SplitParams& P, const PolarDesc* 
 }
 
 // One leaf tile: the per-item body of the leaf kernels.  precs holds the pulse records of
-// the leaf's scene (indexed by pulse); a node with a destination pointer writes there.
+// the leaf's scene (indexed by pulse); a node with a destination pointer writes there.  PARTS = 2: two threads
+// per run, for launches of few tiles.
+template <int PARTS>
 __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc* __restrict__ nodes, const TileItem it,
                                           const float4* __restrict__ tables, const PulseRec* __restrict__ precs,
                                           float2* __restrict__ arena, float2* root_out, int root, char* smem,
@@ -2680,7 +2693,9 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     const int lc = g.tile_lc, rows_t = kSplitTilePixels >> lc;  // 32 rows or more: a warp has one run of columns
     const int groups = (1 << lc) / kLeafRun;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row = tid & (rows_t - 1), group = tid / rows_t;
+    constexpr int kThr = kLeafThreads * PARTS;
+    const int slot = tid & (kLeafThreads - 1), part = tid / kLeafThreads;
+    const int row = slot & (rows_t - 1), group = slot / rows_t;
     const int ifirst = min(g.win_r0 + it.tile_r, g.nr - 1);
     const int ilast = min(g.win_r0 + it.tile_r + rows_t - 1, g.nr - 1);
     const float4 rfirst = __ldg(tables + g.rows_off + 3 * (long long)ifirst + 2);
@@ -2690,9 +2705,9 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     const int ipix = min(g.win_r0 + it.tile_r + row, g.nr - 1);
     const int jpix = g.win_u0 + it.tile_u + kLeafRun * group;
     const LeafRow q = leaf_row(g, tables, ipix, I_first);
-    float ar[kLeafRun], ai[kLeafRun];
+    float ar[kLeafRun / PARTS], ai[kLeafRun / PARTS];
 #pragma unroll
-    for (int k = 0; k < kLeafRun; ++k) ar[k] = ai[k] = 0.0f;
+    for (int k = 0; k < kLeafRun / PARTS; ++k) ar[k] = ai[k] = 0.0f;
     LeafRec* rec = reinterpret_cast<LeafRec*>(smem);
     LeafCol* cols = reinterpret_cast<LeafCol*>(smem + leaf_col_offset());
     LeafMid* mids = reinterpret_cast<LeafMid*>(smem + leaf_mid_offset());
@@ -2700,7 +2715,7 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     const PulseInputs& in = P.in;
     const float side = (float)g.side;
     __syncthreads();  // a persistent block's last tile may still read its runs' middles
-    if (lane == 0 && row == 0) {
+    if (part == 0 && lane == 0 && row == 0) {
         const float4 pd = precs[g.a].d;
         mids[group] = leaf_mid(P, g, jpix, r_min, pd.z, pd.w);
     }
@@ -2740,7 +2755,7 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
         const int chn = nfit > 0 ? nfit : 1;
         const LeafMid& M = mids[group];
         const bool runs = M.runs != 0 && nfit > 0;
-        for (int e = tid; e < nfit * groups; e += kLeafThreads) {  // one (pulse, run of columns) each
+        for (int e = tid; e < nfit * groups; e += kThr) {  // one (pulse, run of columns) each
             const int nl = e / groups, gi = e - nl * groups;
             const LeafMid& m = mids[gi];
             const PulseRec pr = precs[c0 + nl];
@@ -2749,21 +2764,22 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
             o.p0 = leaf_col(pr, m.cv, side);
             o.p1 = make_float4(fmaf(Ax, m.s1, Ay * m.du), Ax * m.s2, Ax * m.s3, Ax * m.s4);
         }
-        for (int nl = warp; nl < nfit; nl += kLeafThreads / 32) {
+        for (int nl = warp; nl < nfit; nl += kThr / 32) {
             const float2* drow = in.data + (size_t)(c0 + nl) * in.samples;
             stage_window_shfl(drow, in.samples, s_base[nl], __float_as_int(rec[nl].p1.w) / 32 + 1, s_wt[nl],
                               win + __float_as_int(rec[nl].p1.z) / 16, lane);
         }
         __syncthreads();
         if (runs) {
-            leaf_runs(P, rec, cols + group, reinterpret_cast<const char*>(win), nfit, q, M.lim, ar, ai);
+            leaf_runs<PARTS>(part, P, rec, cols + group, reinterpret_cast<const char*>(win), nfit, q, M.lim, ar, ai);
         } else {
             float2 more[kLeafRun];
             leaf_direct(P, nodes + it.node, tables, precs, ipix, jpix, c0, chn, more);
 #pragma unroll
-            for (int k = 0; k < kLeafRun; ++k) {
-                ar[k] += more[k].x;
-                ai[k] += more[k].y;
+            for (int k = 0; k < kLeafRun / PARTS; ++k) {
+                const float2 v = more[PARTS == 1 ? k : run_column<PARTS>(part, k / 2, k % 2)];
+                ar[k] += v.x;
+                ai[k] += v.y;
             }
         }
         c0 += chn;
@@ -2774,19 +2790,22 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     const int wr = it.tile_r + row, wu = it.tile_u + kLeafRun * group;
     if (wr < g.win_nr && wu < g.win_nu) {
         float2* p = dst + (long long)wr * g.out_stride + wu;
-        if (wu + kLeafRun <= g.win_nu && (reinterpret_cast<unsigned long long>(p) & 15) == 0) {
+        if (PARTS == 1 && wu + kLeafRun <= g.win_nu && (reinterpret_cast<unsigned long long>(p) & 15) == 0) {
 #pragma unroll
-            for (int k = 0; k < kLeafRun; k += 2)
+            for (int k = 0; k < kLeafRun / PARTS; k += 2)
                 reinterpret_cast<float4*>(p)[k / 2] = make_float4(ar[k], ai[k], ar[k + 1], ai[k + 1]);
         } else {
 #pragma unroll
-            for (int k = 0; k < kLeafRun; ++k)
-                if (wu + k < g.win_nu) p[k] = make_float2(ar[k], ai[k]);
+            for (int k = 0; k < kLeafRun / PARTS; ++k) {
+                const int j = PARTS == 1 ? k : run_column<PARTS>(part, k / 2, k % 2);
+                if (wu + j < g.win_nu) p[j] = make_float2(ar[k], ai[k]);
+            }
         }
     }
 }
 
-__global__ void __launch_bounds__(kLeafThreads, kLeafCtas) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
+template <int PARTS>
+__global__ void __launch_bounds__(kLeafThreads * PARTS, kLeafCtas / PARTS) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
                                                                  const TileItem* __restrict__ items,
                                                                  const float4* __restrict__ tables,
                                                                  const PulseRec* __restrict__ precs,
@@ -2796,7 +2815,7 @@ __global__ void __launch_bounds__(kLeafThreads, kLeafCtas) split_leaf_kernel(Spl
     __shared__ int s_base[kMaxLeafChunk];
     __shared__ float s_wt[kMaxLeafChunk];
     __shared__ int s_nfit;
-    leaf_tile(P, nodes, items[blockIdx.x], tables, precs, arena, root_out, root, smem, s_base, s_wt, s_nfit);
+    leaf_tile<PARTS>(P, nodes, items[blockIdx.x], tables, precs, arena, root_out, root, smem, s_base, s_wt, s_nfit);
 }
 
 // ---- FFBP: merges (both child regrids of one parent tile) --------------------------------
@@ -3719,6 +3738,8 @@ union MergeChildren {
     MergeChild run[2];
 };
 
+enum MergeKind { kMergeEither, kMergeRuns, kMergePairs };
+
 // One merge tile; KIND: kMergeRuns or kMergePairs where the caller knows that the node merges so.
 template <bool COHERENT = false, bool STAGED = false, int KIND = kMergeEither>
 __device__ __forceinline__ void merge_tile(FF K, const PolarDesc* __restrict__ nodes, const TileItem it,
@@ -4149,16 +4170,21 @@ int launch_split_ffbp_leaves(const PulseInputs& in, const PolarDesc* nodes, cons
     if (nitems <= 0) return SARBP_OK;
     SplitParams P = make_params(in, chunk, leaf_capacity(chunk, window_bins), 1);
     const size_t smem = leaf_window_offset() + (size_t)P.cap * 32;
-    if (int st = prepare(split_leaf_kernel, smem)) return st;
-    split_leaf_kernel<<<nitems, kLeafThreads, smem, s>>>(P, nodes, items, tables, reinterpret_cast<const PulseRec*>(precs),
-                                                     arena, root_out, root);
+    // With up to two tiles per SM a sub-partition has only one or two of their warps, and a tile's latency
+    // counts: two threads per run (the same image).  32 pulses, 150 tiles: 17.1 us, one thread per run 20.8;
+    // 240 tiles 22.6 and 24.4; 160 tiles of 64 pulses 37.5 and 37.3; four threads per run 17.7, 32.6 and 55.0.
+    const bool few = nitems <= 2 * 152;
+    const auto kernel = few ? split_leaf_kernel<2> : split_leaf_kernel<1>;
+    if (int st = prepare(kernel, smem)) return st;
+    kernel<<<nitems, kLeafThreads * (few ? 2 : 1), smem, s>>>(P, nodes, items, tables,
+                                                              reinterpret_cast<const PulseRec*>(precs), arena, root_out, root);
     note_launches(1);
     return check_launch("split_ffbp_leaves");
 }
 
 int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* items, int nitems,
                              const float4* tables, const void* crecs, float2* arena, float2* root_out, int root,
-                             size_t box_bytes, unsigned long long wait_ns, int withheld, int kind, cudaStream_t s) {
+                             size_t box_bytes, unsigned long long wait_ns, int withheld, bool runs, cudaStream_t s) {
     if (nitems <= 0) return SARBP_OK;
     PulseInputs none{};
     none.k = k;
@@ -4166,9 +4192,7 @@ int launch_split_ffbp_merges(double k, const PolarDesc* nodes, const TileItem* i
     SplitParams P = make_params(none, 1, 4, 1);
     if (box_bytes > 0) {
         const size_t smem = 128 + kTabBytes + box_bytes;
-        const auto kernel = kind == kMergeRuns    ? split_merge_staged_kernel<kMergeRuns>
-                            : kind == kMergePairs ? split_merge_staged_kernel<kMergePairs>
-                                                  : split_merge_staged_kernel<kMergeEither>;
+        const auto kernel = runs ? split_merge_staged_kernel<kMergeRuns> : split_merge_staged_kernel<kMergePairs>;
         if (int st = prepare(kernel, smem)) return st;
         kernel<<<nitems, kMergeThreads, smem, s>>>(
             P, nodes, items, tables, reinterpret_cast<const ChildRec*>(crecs), arena, root_out, root, wait_ns, withheld);
@@ -4341,7 +4365,7 @@ __global__ void __launch_bounds__(kLeafThreads, kLeafCtas) batch_leaf_kernel(con
             load_scene(scenes, it.pad, sc);
             if (threadIdx.x == 0) s_scene = it.pad;
         }
-        leaf_tile(sc.P, nodes, it, tables, precs + sc.prec_offset, arena, nullptr, -1, smem, s_base, s_wt, s_nfit);
+        leaf_tile<1>(sc.P, nodes, it, tables, precs + sc.prec_offset, arena, nullptr, -1, smem, s_base, s_wt, s_nfit);
         trace_item(trace, it.pad);
     }
 }
