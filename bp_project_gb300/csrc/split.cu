@@ -2805,7 +2805,7 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
 }
 
 template <int PARTS>
-__global__ void __launch_bounds__(kLeafThreads * PARTS, kLeafCtas / PARTS) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
+__global__ void __launch_bounds__(kLeafThreads * PARTS, PARTS == 1 ? kLeafCtas : 2) split_leaf_kernel(SplitParams P, const PolarDesc* __restrict__ nodes,
                                                                  const TileItem* __restrict__ items,
                                                                  const float4* __restrict__ tables,
                                                                  const PulseRec* __restrict__ precs,
@@ -4171,8 +4171,8 @@ int launch_split_ffbp_leaves(const PulseInputs& in, const PolarDesc* nodes, cons
     SplitParams P = make_params(in, chunk, leaf_capacity(chunk, window_bins), 1);
     const size_t smem = leaf_window_offset() + (size_t)P.cap * 32;
     // With up to two tiles per SM a sub-partition has only one or two of their warps, and a tile's latency
-    // counts: two threads per run (the same image).  32 pulses, 150 tiles: 17.1 us, one thread per run 20.8;
-    // 240 tiles 22.6 and 24.4; 160 tiles of 64 pulses 37.5 and 37.3; four threads per run 17.7, 32.6 and 55.0.
+    // counts: two threads per run (the same image).  32 pulses, 150 tiles: 16.3 us, one thread per run 20.8;
+    // 240 tiles 22.3 and 24.4; 160 tiles of 64 pulses 36.6 and 37.3; four threads per run 17.7, 32.6 and 55.0.
     const bool few = nitems <= 2 * 152;
     const auto kernel = few ? split_leaf_kernel<2> : split_leaf_kernel<1>;
     if (int st = prepare(kernel, smem)) return st;
