@@ -1,20 +1,23 @@
 // Spatial order of a point list for split-precision direct BP.
 //
-// The points kernel forms tiles of 1024 consecutive points; its fast path needs tiles of at most
+// The points kernel forms tiles of 512 consecutive points; its fast path needs tiles of at most
 // about 20 m radius, while a raster of terrain points puts a tile on a strip of hundreds of metres
 // and every pulse on the two-float fallback.  These kernels order a list by the Hilbert curve of a 256 x 256
 // raster over its bounding square: two stable 8-bit counting passes, so the order (and with it the
 // image) is the same on every run.  Nothing is ordered when no tile is wide: the kernels
 // then return at once, and the points kernel takes the list as it is.
 // 192,384 terrain points in raster order (501 to a row, half a metre apart), 1024 pulses: 2.50 ms as they
-// come, 0.64 ms ordered, of which the ordering is about 0.05; error against FP64 2.8e-7 either way.
+// come, 0.62 ms ordered, of which the ordering is about 0.05; error against FP64 2.8e-7 either way.
 #include "common.cuh"
 
 namespace sarbp {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kKeys = 4096;            // keys per block of a counting pass
+// Blocks of a counting pass, at most, each on a whole number of rounds of kThreads keys.  192,384 points in 0.618 ms
+// all in all; with 188 blocks 0.621, 376 0.633, and 4096 keys per block 0.637 (8,000 points: 30 us of
+// ordering instead of 67).
+constexpr int kMaxBlocks = 94;
 constexpr int kTilePoints = kPointTile;  // points per tile of the points kernel
 constexpr float kWideRadius = 16.0f;   // tiles above this radius (m) are worth ordering
 constexpr int kDigits = 256;
@@ -97,7 +100,7 @@ __device__ __forceinline__ unsigned hilbert(unsigned x, unsigned y) {
 // Counts of each digit in each block's keys, digit-major: counts[digit * blocks + block].  FIRST: the keys
 // are made from the points.
 template <bool FIRST>
-__global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __restrict__ xyz, int npts,
+__global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __restrict__ xyz, int npts, int per,
                                                                 const PointOrder* __restrict__ h,
                                                                 unsigned short* __restrict__ keys,
                                                                 int* __restrict__ counts) {
@@ -108,8 +111,8 @@ __global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __
     const float x0 = unordered(h->low[0]), y0 = unordered(h->low[1]);
     const float span = fmaxf(unordered(~h->high[0]) - x0, unordered(~h->high[1]) - y0);
     const float scale = 255.99f / fmaxf(span, 1e-6f);
-    const int end = min(npts, (int)(blockIdx.x + 1) * kKeys);
-    for (int i = blockIdx.x * kKeys + threadIdx.x; i < end; i += kThreads) {
+    const int end = min(npts, (int)(blockIdx.x + 1) * per);
+    for (int i = blockIdx.x * per + threadIdx.x; i < end; i += kThreads) {
         unsigned key;
         if (FIRST) {
             // Cells outside 0 .. 255 (no numbers, overflow) go to the edge cells.
@@ -126,45 +129,48 @@ __global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __
     counts[threadIdx.x * gridDim.x + blockIdx.x] = hist[threadIdx.x];
 }
 
-// Exclusive prefix sum of n counts in place (one block).
+// Exclusive prefix sum of n counts in place (one block, n a multiple of 4, counts 16-byte aligned): rounds of
+// four counts per thread, the next round's load in flight.  48,128 counts: 10 us, with a stretch of them per
+// thread 41.
 __global__ void __launch_bounds__(1024) points_scan_kernel(const PointOrder* __restrict__ h, int* __restrict__ counts,
                                                            int n) {
     if (h->narrow) return;
-    __shared__ int warps[32];
-    const int per = (n + 1023) / 1024, b = min(n, (int)threadIdx.x * per), e = min(n, b + per);
-    int sum = 0;
-    for (int i = b; i < e; ++i) sum += counts[i];
+    __shared__ int warps[2][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += v;
-    }
-    if (lane == 31) warps[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        int w = warps[lane];
+    int4* c = reinterpret_cast<int4*>(counts);
+    const int quads = n / 4;
+    int4 next = (int)threadIdx.x < quads ? c[threadIdx.x] : make_int4(0, 0, 0, 0);
+    int carry = 0;
+    for (int q0 = 0, round = 0; q0 < quads; q0 += 1024, round ^= 1) {
+        const int q = q0 + threadIdx.x;
+        const int4 v = next;
+        next = q + 1024 < quads ? c[q + 1024] : make_int4(0, 0, 0, 0);
+        const int sum = v.x + v.y + v.z + v.w;
+        int inc = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += v;
+            const int u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
         }
-        warps[lane] = w;
-    }
-    __syncthreads();
-    int at = inc - sum + (warp ? warps[warp - 1] : 0);
-    for (int i = b; i < e; ++i) {
-        const int v = counts[i];
-        counts[i] = at;
-        at += v;
+        if (lane == 31) warps[round][warp] = inc;
+        __syncthreads();  // rounds use the two rows in turn, so one barrier each is enough
+        int w = warps[round][lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += u;
+        }
+        const int before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+        int at = carry + inc - sum + (warp ? before : 0);
+        carry += __shfl_sync(0xffffffffu, w, 31);
+        if (q < quads) c[q] = make_int4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
     }
 }
 
 // Stable scatter of one pass: a round of 256 keys at a time, ranked by warp (lanes with the same digit) and
 // over the warps.  FIRST: the payload is the point's index.
 template <bool FIRST>
-__global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, const PointOrder* __restrict__ h,
+__global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, int per, const PointOrder* __restrict__ h,
                                                                   const unsigned short* __restrict__ keys,
                                                                   const int* __restrict__ index,
                                                                   const int* __restrict__ counts,
@@ -175,7 +181,7 @@ __global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, cons
     __shared__ int seen[kThreads / 32][kDigits];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     base[threadIdx.x] = counts[threadIdx.x * gridDim.x + blockIdx.x];
-    const int begin = blockIdx.x * kKeys, end = min(npts, begin + kKeys);
+    const int begin = blockIdx.x * per, end = min(npts, begin + per);
     for (int r = begin; r < end; r += kThreads) {
         for (int w = 0; w < kThreads / 32; ++w) seen[w][threadIdx.x] = 0;
         __syncthreads();
@@ -204,7 +210,8 @@ __global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, cons
 }
 
 size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
-int order_blocks(int npts) { return (npts + kKeys - 1) / kKeys; }
+int keys_per_block(int npts) { return kThreads * ((npts + kThreads * kMaxBlocks - 1) / (kThreads * kMaxBlocks)); }
+int order_blocks(int npts) { return (npts + keys_per_block(npts) - 1) / keys_per_block(npts); }
 
 }  // namespace
 
@@ -227,17 +234,17 @@ int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder*
     auto* keys1 = reinterpret_cast<unsigned short*>(take(sizeof(unsigned short) * (size_t)npts));
     auto* index1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)npts));
     auto* index2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)npts));
-    const int blocks = order_blocks(npts);
+    const int blocks = order_blocks(npts), per = keys_per_block(npts);
     auto* counts = reinterpret_cast<int*>(take(sizeof(int) * (size_t)kDigits * blocks));
     const cudaError_t e = cudaMemsetAsync(h, 0xff, sizeof(PointOrder), s);
     if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "points order: %s", cudaGetErrorString(e));
     points_extent_kernel<<<(npts + kTilePoints - 1) / kTilePoints, kThreads, 0, s>>>(xyz, npts, h);
-    points_count_kernel<true><<<blocks, kThreads, 0, s>>>(xyz, npts, h, keys, counts);
+    points_count_kernel<true><<<blocks, kThreads, 0, s>>>(xyz, npts, per, h, keys, counts);
     points_scan_kernel<<<1, 1024, 0, s>>>(h, counts, kDigits * blocks);
-    points_scatter_kernel<true><<<blocks, kThreads, 0, s>>>(npts, h, keys, nullptr, counts, keys1, index1);
-    points_count_kernel<false><<<blocks, kThreads, 0, s>>>(xyz, npts, h, keys1, counts);
+    points_scatter_kernel<true><<<blocks, kThreads, 0, s>>>(npts, per, h, keys, nullptr, counts, keys1, index1);
+    points_count_kernel<false><<<blocks, kThreads, 0, s>>>(xyz, npts, per, h, keys1, counts);
     points_scan_kernel<<<1, 1024, 0, s>>>(h, counts, kDigits * blocks);
-    points_scatter_kernel<false><<<blocks, kThreads, 0, s>>>(npts, h, keys1, index1, counts, nullptr, index2);
+    points_scatter_kernel<false><<<blocks, kThreads, 0, s>>>(npts, per, h, keys1, index1, counts, nullptr, index2);
     note_launches(7);
     *order = h;
     *index = index2;

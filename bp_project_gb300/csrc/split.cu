@@ -673,7 +673,7 @@ __device__ void setup_points(const Job& J, TileShared& S, PointPix px[kPointPX])
 // a fraction of a bin.  What the roundings leave (rests of W, u / dr and delta, below 1e-3 turns or bins) is FP32.
 // An FP32 range of ten bins alone would put 3e-7 on the fraction, and through it on the image.  Tiles hold
 // 512 points (the range correction, FP32, grows with the square of the tile).  192,384 points, 1024
-// pulses: 0.64 ms; with FP32 products of 10- and 11-bit parts 0.58 ms and an error of 3.6e-7 instead of 2.8e-7.
+// pulses: 0.57 ms; with FP32 products of 10- and 11-bit parts 0.51 ms and an error of 3.6e-7 instead of 2.8e-7.
 __device__ __forceinline__ void points_chunk(const SplitParams& P, const Rec* __restrict__ rec,
                                              const float4* __restrict__ win, const float* __restrict__ rest, int chn,
                                              PointPix px[kPointPX]) {
