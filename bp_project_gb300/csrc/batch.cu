@@ -373,7 +373,8 @@ int sarbp_batch_execute(const sarbp_batch* batch, void* stream) {
                                        batch->direct_smem, trace, s);
     if (st == SARBP_OK)
         st = launch_split_batch_leaves(scenes, nodes, bp_items + batch->n_direct, n_leaf, tables, precs, arena,
-                                       counters + 1, batch->leaf_blocks, batch->leaf_smem, trace, fs);
+                                       counters + 1, batch->leaf_blocks, batch->leaf_smem, trace,
+                                       !fork && batch->n_direct > 0, fs);
     const size_t crec_size = split_ffbp_child_record_bytes();
     for (int h = 1; h <= batch->max_height && st == SARBP_OK; ++h) {
         const int first = batch->level_begin[h - 1], count = batch->level_count[h - 1];

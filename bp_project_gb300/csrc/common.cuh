@@ -258,7 +258,7 @@ int launch_split_batch_direct(const void* scenes, const TileItem* items, int nit
                               size_t smem, unsigned long long* trace, cudaStream_t s);
 int launch_split_batch_leaves(const void* scenes, const PolarDesc* nodes, const TileItem* items, int nitems,
                               const float4* tables, const void* precs, float2* arena, int* counter, int blocks,
-                              size_t smem, unsigned long long* trace, cudaStream_t s);
+                              size_t smem, unsigned long long* trace, bool after_direct, cudaStream_t s);
 int launch_split_batch_merges(const void* scenes, const PolarDesc* nodes, const TileItem* items, int nitems,
                               const float4* tables, const void* crecs, float2* arena, int* counter, int blocks,
                               unsigned long long* trace, cudaStream_t s);
