@@ -1658,18 +1658,19 @@ struct LatticeBody {
     static constexpr bool kShflWindows = false;
     const SplitParams& P;
     const TileShared& S;
-    const Job& J;
+    const sarbp_lattice& lat;
+    int p0;
     float di, dj, d2, ds, s2;  // the run's middle: offsets (rows, columns), |delta|^2, delta . s_row; |s_row|^2
     float* ar;
     float* ai;
     __device__ int group() const { return threadIdx.x / kRunThreads; }
     __device__ void fast(const Rec* rec, const float4* win, int nfit, int c0) {
-        lattice_runs(P, rec, reinterpret_cast<const char*>(win), (c0 - J.p0 + group()) & 1, nfit, di, dj,
+        lattice_runs(P, rec, reinterpret_cast<const char*>(win), (c0 - p0 + group()) & 1, nfit, di, dj,
                      (int)(2.0f * di), (int)dj, d2, ds, s2, ar, ai);
     }
     __device__ void slow(int c0, int nslow, const SlowRec* srec) {
         float2 more[kRun];
-        lattice_run_slow(P, S, J.lat, di, dj, (c0 - J.p0 + group()) & 1, nslow, c0, srec, more);
+        lattice_run_slow(P, S, lat, di, dj, (c0 - p0 + group()) & 1, nslow, c0, srec, more);
 #pragma unroll
         for (int k = 0; k < kRun; ++k) {
             ar[k] += more[k].x;
@@ -2116,7 +2117,8 @@ struct PolarRunBody {
     static constexpr bool kShflWindows = false;
     const SplitParams& P;
     const TileShared& S;
-    const Job& J;
+    const PolarDesc& g;
+    int p0;
     const PolarRun& q;
     int i, j0;
     float* ar;
@@ -2125,7 +2127,7 @@ struct PolarRunBody {
     __device__ void fast(const Rec* rec, const float4* win, int nfit, int c0) {
         const float inv_dr = P.inv_drf, Kf = P.Kf, kz = 1.0f / (kTwoPiF * Kf), kd = inv_dr * kz;
 #pragma unroll 1
-        for (int nl = (c0 - J.p0 + group()) & 1; nl < nfit; nl += 2) {
+        for (int nl = (c0 - p0 + group()) & 1; nl < nfit; nl += 2) {
             const float4 ra = rec[nl].a, rb = rec[nl].b, rc = rec[nl].c, rd = rec[nl].d;
             const float L = fmaf(rb.x, q.dx, rb.y * q.dy);
             const float q2 = fmaf(-L, L, q.d2);
@@ -2153,7 +2155,7 @@ struct PolarRunBody {
         float2 sum[kColRun];
 #pragma unroll
         for (int k = 0; k < kColRun; ++k) sum[k] = make_float2(ar[k], ai[k]);
-        polar_run_slow(P, S, J.g, i, j0, (c0 - J.p0 + group()) & 1, nslow, c0, srec, sum);
+        polar_run_slow(P, S, g, i, j0, (c0 - p0 + group()) & 1, nslow, c0, srec, sum);
 #pragma unroll
         for (int k = 0; k < kColRun; ++k) {
             ar[k] = sum[k].x;
@@ -2177,7 +2179,7 @@ __global__ void __launch_bounds__(kThreads, 3) split_polar_runs_kernel(SplitPara
     float ar[kColRun], ai[kColRun];
 #pragma unroll
     for (int k = 0; k < kColRun; ++k) ar[k] = ai[k] = 0.0f;
-    PolarRunBody body{P, S, J, q, g.win_r0 + J.tile_r + row, g.win_u0 + J.tile_u + col, ar, ai};
+    PolarRunBody body{P, S, g, J.p0, q, g.win_r0 + J.tile_r + row, g.win_u0 + J.tile_u + col, ar, ai};
     chunk_loop(P, J, S, smem, true, body);
     float2* out = P.out + blockIdx.y * P.split_stride;
     add_halves(reinterpret_cast<float2*>(smem + window_offset()), body.group(), slot, ar, ai, [&](int k, float2 v) {
@@ -2212,7 +2214,7 @@ __device__ __forceinline__ void lattice_tile(const SplitParams& P, const sarbp_l
     float ar[kRun], ai[kRun];
 #pragma unroll
     for (int k = 0; k < kRun; ++k) ar[k] = ai[k] = 0.0f;
-    LatticeBody body{P, S, J, di, dj, d2, ds, s2, ar, ai};
+    LatticeBody body{P, S, lat, p0, di, dj, d2, ds, s2, ar, ai};
     chunk_loop(P, J, S, smem, true, body);
     add_halves(reinterpret_cast<float2*>(smem + window_offset()), body.group(), slot, ar, ai, [&](int k, float2 v) {
         const int wr = tile_r + row0 + k, wu = tile_u + col;
