@@ -1565,7 +1565,7 @@ struct PointsBody {
 // What bounds the loop: the register file feeds two operands a cycle to the FMA pipe (a fused
 // multiply-add of three registers takes 1.5 cycles, a packed one 3), so issue sits at 71% with the
 // FMA pipe, the shared-memory pipe and issue all at 60-70%, and every instruction removed shows in
-// the time.  4096 pulses onto 2048 x 2048: 17.2 ms (1001 Gpixel-pulses/s; 28.9 instructions per
+// the time.  4096 pulses onto 2048 x 2048: 17.05 ms (1008 Gpixel-pulses/s; 28.9 instructions per
 // pixel-pulse), 19.6 ms (876; 31.3) with four pixels per thread and the root-free range chain of the
 // adjoint per pixel.  Measured and not kept: runs of 16 (24 warps per SM instead of 32: 16.7 ms, but a larger
 // error on small scenes), the range to the middle in integers too (18.3; error 0.68e-6 instead of 0.80), even
@@ -4322,7 +4322,7 @@ __device__ __forceinline__ int next_item(int* counter, int& s_item) {
 __device__ __forceinline__ void load_scene(const BatchScene* __restrict__ scenes, int scene, BatchScene& sc) {
     const int* src = reinterpret_cast<const int*>(scenes + scene);
     int* dst = reinterpret_cast<int*>(&sc);
-    for (int w = threadIdx.x; w < (int)(sizeof(BatchScene) / sizeof(int)); w += kThreads) dst[w] = src[w];
+    for (int w = threadIdx.x; w < (int)(sizeof(BatchScene) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
 }
 
