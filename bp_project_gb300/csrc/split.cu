@@ -4319,10 +4319,11 @@ __device__ __forceinline__ int next_item(int* counter, int& s_item) {
     return s_item;
 }
 
+template <int THREADS>
 __device__ __forceinline__ void load_scene(const BatchScene* __restrict__ scenes, int scene, BatchScene& sc) {
     const int* src = reinterpret_cast<const int*>(scenes + scene);
     int* dst = reinterpret_cast<int*>(&sc);
-    for (int w = threadIdx.x; w < (int)(sizeof(BatchScene) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
+    for (int w = threadIdx.x; w < (int)(sizeof(BatchScene) / sizeof(int)); w += THREADS) dst[w] = src[w];
     __syncthreads();
 }
 
@@ -4342,7 +4343,7 @@ __global__ void __launch_bounds__(kThreads, 4) batch_direct_kernel(const BatchSc
         if (idx >= nitems) return;
         const TileItem it = items[idx];
         if (it.pad != s_scene) {  // uniform across the block
-            load_scene(scenes, it.pad, sc);
+            load_scene<kThreads>(scenes, it.pad, sc);
             if (threadIdx.x == 0) s_scene = it.pad;
         }
         lattice_tile(sc.P, sc.lat, sc.lc, it.tile_r, it.tile_u, 0, sc.P.in.pulses, sc.P.out, S, smem);
@@ -4373,7 +4374,7 @@ __global__ void __launch_bounds__(kLeafThreads, kLeafCtas) batch_leaf_kernel(con
         }
         const TileItem it = items[idx];
         if (it.pad != s_scene) {
-            load_scene(scenes, it.pad, sc);
+            load_scene<kLeafThreads>(scenes, it.pad, sc);
             if (threadIdx.x == 0) s_scene = it.pad;
         }
         leaf_tile<1>(sc.P, nodes, it, tables, precs + sc.prec_offset, arena, nullptr, -1, smem, s_base, s_wt, s_nfit);
