@@ -969,8 +969,11 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
         const float x1 = turn * fabsf(P.inv_drf), x2 = fmaf(S.sth[4], fabsf(ax), 0.5f * turn * y) * fabsf(P.inv_drf);
         lim = (3.0f * x1 * x1 + x2) * x2 <= 1e-7f ? 0.5f : -1.0f;
     }
+    // Points: the whole numbers of the linear terms stay within 32 bits (offsets in 2^-16 m, W in 2^-16 turns/m,
+    // u / dr in 2^-12 bins/m).
+    const bool whole_ok = MODE != 3 || (S.rhof < 32000.0f && fabsf(P.Kf) < 32000.0f && fabsf(P.inv_drf) < 5.0e5f);
     const bool ok = Rf > 0.0f && fabsf(Q.h) < 1.0e7f && hi - lo + 1.0f <= (float)P.cap &&
-                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf && runs_ok;
+                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf && runs_ok && whole_ok;
     const int bo = ok ? (int)lo : 0;
     S.base[lane] = ok ? (int)I + bo : 0;
     S.wt[lane] = (float)in.weight[n];
