@@ -118,15 +118,22 @@ __device__ __forceinline__ double fast_sqrt(double x, double& yh) {
     return fma(fma(-g1, g1, x), yh, g1);
 }
 
-// Bins 1 <= floor(q) <= n - 3 (the support of a four-point stencil in n samples): the bin and the
-// fraction less 1/2.  One FP64 addition: at 1.5 2^20 the last mantissa bit is worth 2^-32, so rounding
-// down leaves floor(q) in the high word and the fraction's 32 bits in the low one.
-__device__ __forceinline__ bool fast_bin(double q, int n, int& i, float& s) {
-    const double m = __dadd_rd(q, 1572864.0);
+// Bins 1 <= floor(q) <= n - 3 (the support of a four-point stencil in n samples) of q = x / step: the bin and
+// the fraction less 1/2.  One FP64 product and one addition: at 1.5 2^20 the last mantissa bit is worth 2^-32, so
+// rounding down leaves floor(q) in the high word and the fraction's 32 bits in the low one.  Between bins a
+// last-bit difference of the product from the quotient only moves the fraction; at the support's two ends it would
+// let a sample in or keep one out, so there (and in rows of half a million samples and more) the quotient decides.
+__device__ __forceinline__ bool fast_bin(double x, double step, double inv, int n, int& i, float& s) {
+    const double m = __dadd_rd(x * inv, 1572864.0);
+    const int lo = __double2loint(m);
     i = (__double2hiint(m) & 0x000fffff) - 0x80000;
-    s = (float)(__double2loint(m) ^ INT_MIN) * 2.3283064365386963e-10f;
-    if ((__double2hiint(m) >> 20) == 0x413 && i < 0x7fff0) return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
-    if (!(q >= 1.0 && q < (double)(n - 2))) return false;  // rows of half a million samples and more, or no number
+    s = (float)(lo ^ INT_MIN) * 2.3283064365386963e-10f;
+    const int whole = i + (lo < 0);  // the nearest bin
+    const bool end = (unsigned)lo + 2u <= 4u && (whole == 1 || whole == n - 2);
+    if ((__double2hiint(m) >> 20) == 0x413 && i < 0x7fff0 && !end)
+        return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
+    const double q = x / step;
+    if (!(q >= 1.0 && q < (double)(n - 2))) return false;  // or no number
     i = (int)floor(q);
     s = (float)(q - ((double)i + 0.5));
     return true;
@@ -196,7 +203,7 @@ __device__ __forceinline__ void accumulate_mixed(PulseStage<SARBP_MIXED>& st, co
             const double d = fast_sqrt(fma(dx, dx, fma(dy, dy, zz)), yh);
             float vr = 0.0f, vi = 0.0f, f, sn, cs;
             int i;
-            if (fast_bin((d - in.range_start) * inv, in.samples, i, f)) {
+            if (fast_bin(d - in.range_start, in.data_dr, inv, in.samples, i, f)) {
                 float w[4];
                 lagrange_centred(f, w);
                 const float2* row = in.data + (size_t)(c0 + t) * in.samples + i - 1;
@@ -361,7 +368,8 @@ __device__ __forceinline__ bool image_at_mixed(const float2* __restrict__ img, c
     const double u0 = dy * y1, uu = fma(fma(-u0, g, dy), y1, u0);
     int ir, iu;
     float tr, tu;
-    if (fast_bin((rr - src.r0) * src.inv_dr, src.nr, ir, tr) && fast_bin((uu - src.u0) * src.inv_du, src.nu, iu, tu)) {
+    if (fast_bin(rr - src.r0, src.dr, src.inv_dr, src.nr, ir, tr) &&
+        fast_bin(uu - src.u0, src.du, src.inv_du, src.nu, iu, tu)) {
         float wr[4], wu[4];
         lagrange_centred(tr, wr);
         lagrange_centred(tu, wu);
