@@ -972,8 +972,16 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
     // Points: the whole numbers of the linear terms stay within 32 bits (offsets in 2^-16 m, W in 2^-16 turns/m,
     // u / dr in 2^-12 bins/m).
     const bool whole_ok = MODE != 3 || (S.rhof < 32000.0f && fabsf(P.Kf) < 32000.0f && fabsf(P.inv_drf) < 5.0e5f);
+    // Points: the range series e0 - e0^2 B leaves out up to rho^6 / 16 R^5, which may cost 1e-6 turns and 1e-6 bins (at
+    // a tile's corner; the image's error is a few times less).  Near ranges and wide tiles go over that.
+    bool third_ok = true;
+    if (MODE == 3) {
+        const float x = S.rhof / Rf, x2 = x * x;
+        third_ok = fmaxf(fabsf(P.Kf), fabsf(P.inv_drf)) * (x2 * x2 * x) * S.rhof <= 1.6e-5f;
+    }
     const bool ok = Rf > 0.0f && fabsf(Q.h) < 1.0e7f && hi - lo + 1.0f <= (float)P.cap &&
-                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf && runs_ok && whole_ok;
+                    fabsf(P.Kf) * S.rhof * S.rhof <= (float)P.envelope * Rf && S.rhof < 0.25f * Rf && runs_ok && whole_ok &&
+                    third_ok;
     const int bo = ok ? (int)lo : 0;
     S.base[lane] = ok ? (int)I + bo : 0;
     S.wt[lane] = (float)in.weight[n];

@@ -44,3 +44,14 @@ def test_offsets_beyond_the_integer_range(lib, step):
     """A tile of 500 points in a line, up to 30, 33 and 40 km from its centre, seen from 10,000 km at a wavelength of
     63 m: the fast path's offsets are 32-bit integers of 2^-16 m, which end at 32.8 km."""
     assert error(raster(1, 500, step, 3.0e6), 1.0e7, 1000.0, 200.0, 0.2) <= 1e-5
+
+
+@pytest.mark.parametrize("rows,cols,step", [(60, 60, 0.5), (40, 300, 0.1), (22, 23, 1.0)])
+def test_short_range(lib, rows, cols, step):
+    """400 MHz from 40 m height and 40 to 80 m ground range: the range series' third order is up to 1e-3 rad there."""
+    assert error(raster(rows, cols, step, 40.0), 40.0, 0.1, 0.5, 4 * np.pi * 4e8 / 299792458.0) <= 1e-5
+
+
+def test_wide_tiles_at_a_long_wavelength(lib):
+    """Tiles of 33 km half-width from 360 km, k = 1e-5: the same order is 3e-3 bins of 400 m."""
+    assert error(raster(60, 60, 2000.0, 3.0e5), 2.0e5, 100.0, 400.0, 1e-5) <= 1e-5
