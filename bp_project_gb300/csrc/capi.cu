@@ -36,6 +36,22 @@ int check_launch(const char* what) {
     return SARBP_OK;
 }
 
+int allow_shared(const void* kernel, size_t smem) {
+    if (smem <= 40 * 1024) return SARBP_OK;  // 48 KB without the attribute, static shared memory included
+    cudaFuncAttributes a;
+    cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e == cudaSuccess && (size_t)a.maxDynamicSharedSizeBytes >= smem) return SARBP_OK;
+    int dev = 0, most = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    if ((size_t)most < smem + a.sharedSizeBytes)
+        return fail(SARBP_ERR_CUDA, "%zu bytes of shared memory are more than a block can have", smem);
+    return SARBP_OK;
+}
+
 void note_launches(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
 namespace {

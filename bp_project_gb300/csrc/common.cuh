@@ -157,6 +157,10 @@ PulseInputs inputs_of(const float* data, int pulses, int samples, const double* 
 int split_direct_polar(const PulseInputs& in, const sarbp_polar_grid& grid, int chunk_pulses, int pulse_split,
                        float2* parts, float2* out, cudaStream_t s);
 
+// Lets `kernel` be launched with `smem` bytes of dynamic shared memory on the current device.  The limit is the
+// kernel's, not the launch's, and threads share it: it goes to the most that a block can have, and only up.
+int allow_shared(const void* kernel, size_t smem);
+
 // Plain (reference-arithmetic) kernels.
 int launch_plain_polar(int mode, const PulseInputs& in, const PolarDesc& g, int pulse_begin, int pulse_end,
                        int chunk, float2* out, long long out_stride, cudaStream_t s);

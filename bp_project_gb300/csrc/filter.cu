@@ -329,13 +329,6 @@ int launch_tile_argmax(const float* a, int nr, int nu, int nr_tiles, int nu_tile
     return check_launch("tile_argmax");
 }
 
-template <class K>
-int set_smem(K kernel, size_t smem) {
-    if (smem <= 48 * 1024) return SARBP_OK;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return e == cudaSuccess ? SARBP_OK : fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-}
-
 size_t sosfiltfilt_workspace(int rows, int n, int padlen) {
     return (size_t)(n + 2 * padlen) * (size_t)rows * 2 * sizeof(double);
 }
@@ -345,13 +338,13 @@ int launch_sosfiltfilt(const float* x, int rows, int n, const double* sos, const
     const size_t smem = row_smem(n, padlen);
     if (smem <= kRowSmemLimit && sections <= kSpreadSections) {
         const size_t line = (size_t)(n + 2 * padlen) * sizeof(double2);
-        if (int st = set_smem(sosfiltfilt_spread_kernel, line)) return st;
+        if (int st = allow_shared(reinterpret_cast<const void*>(sosfiltfilt_spread_kernel), line)) return st;
         sosfiltfilt_spread_kernel<<<rows, 32, line, s>>>(x, n, sos, zi, sections, padlen, y);
         note_launches(1);
         return check_launch("sosfiltfilt");
     }
     if (smem <= kRowSmemLimit) {
-        if (int st = set_smem(sosfiltfilt_pipe_kernel, smem)) return st;
+        if (int st = allow_shared(reinterpret_cast<const void*>(sosfiltfilt_pipe_kernel), smem)) return st;
         sosfiltfilt_pipe_kernel<<<rows, 32, smem, s>>>(x, n, sos, zi, sections, padlen, y);
         note_launches(1);
         return check_launch("sosfiltfilt");

@@ -492,9 +492,9 @@ bool rc_blocks_fit(int samples, int taps) {
 int launch_rc_blocks(const float2* raw, int pulses, int samples, int taps, const float2* response, float2* out,
                      cudaStream_t s) {
     const size_t smem = blocks_smem(samples);
+    if (int st = allow_shared(reinterpret_cast<const void*>(rc_blocks_kernel), smem)) return st;
     int dev = 0, sms = 0, per_sm = 0;
-    cudaError_t e = cudaFuncSetAttribute(rc_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rc_blocks_kernel, kBlockThreads, smem);
     if (e != cudaSuccess || per_sm < 1) return fail(SARBP_ERR_CUDA, "rc_blocks: %s", cudaGetErrorString(e));

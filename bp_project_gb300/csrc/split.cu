@@ -3874,11 +3874,7 @@ size_t dynamic_smem(int cap, bool polar) {
 
 template <class K>
 int prepare(K kernel, size_t smem) {
-    if (smem > 40 * 1024) {  // 48 KB without the attribute, static shared memory included
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
-    return SARBP_OK;
+    return allow_shared(reinterpret_cast<const void*>(kernel), smem);
 }
 
 // Pulse split that fills the GPU's CTA slots best: the fewest waves ceil(tiles s / slots) / s over

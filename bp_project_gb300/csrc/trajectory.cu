@@ -324,10 +324,7 @@ int launch_pga_update(const double2* smooth, int targets, int pulses, const doub
     double *power = reinterpret_cast<double*>(smoothed + pulses), *coherence = power + targets, *scale = coherence + targets;
     const int block = (targets + 31) / 32 * 32;
     const size_t smem = 6 * sizeof(double) * (size_t)block;
-    if (smem > 40 * 1024) {  // beside the static part, within 48 KB without the attribute
-        const cudaError_t e = cudaFuncSetAttribute(pga_pulses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    }
+    if (int st = allow_shared(reinterpret_cast<const void*>(pga_pulses_kernel), smem)) return st;
     pga_targets_kernel<<<targets, kThreads, 0, s>>>(smooth, pulses, power, coherence);
     pga_weights_kernel<<<1, block, 0, s>>>(power, coherence, targets, scale, stats);
     pga_pulses_kernel<<<pulses - 1, block, smem, s>>>(smooth, targets, pulses, pos, xyz, 1.0 / k, scale, rate);
