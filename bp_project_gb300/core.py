@@ -98,9 +98,12 @@ def direct_polar(data, pos, weight, phase, grid: Grid, range_start, data_dr, k, 
     return out
 
 
-def backproject_points(data, pos, weight, phase, xyz, range_start, data_dr, k, mode=DEFAULT_MODE, pulse_split=1,
+def backproject_points(data, pos, weight, phase, xyz, range_start, data_dr, k, mode=DEFAULT_MODE, pulse_split=0,
                        out=None):
-    """Direct BP at points xyz float64 [M, 3] -> complex64 [M] (ffbp.backproject_points semantics)."""
+    """Direct BP at points xyz float64 [M, 3] -> complex64 [M] (ffbp.backproject_points semantics).
+
+    pulse_split > 1 splits each tile's pulses over that many CTAs (partial images summed in fixed order); 0 (the
+    default) lets the library pick the split that fills the GPU, 1 is one pass over the pulses."""
     p, s = check_pulses(data, pos, weight, phase)
     _require(xyz, "xyz", torch.float64)
     if xyz.dim() != 2 or xyz.shape[1] != 3:

@@ -363,11 +363,8 @@ int sarbp_direct_polar(const float* data, int pulses, int samples, const double*
 
 namespace {
 
-// Split-mode point lists longer than one tile: the spatial order's buffers, then the partial images of
-// the pulse split (the automatic one where the caller asks for one pass).  Points of a list longer than a
-// tile need neither, but both pay: see points_order.cu.
+// Split-mode point lists longer than one tile: the spatial order's buffers, then the partial images of the pulse split.
 size_t points_order_space(int npts) { return (points_order_bytes(npts) + 255) / 256 * 256; }
-constexpr int kMaxAutoSplit = 8;
 
 size_t points_parts(int npts, int pulse_split) {
     return pulse_split > 1 && npts > 0 ? (size_t)pulse_split * (size_t)npts * sizeof(float2) : 0;
@@ -376,9 +373,10 @@ size_t points_parts(int npts, int pulse_split) {
 }  // namespace
 
 size_t sarbp_backproject_points_workspace(int mode, int npts, int pulse_split) {
-    if (mode != SARBP_SPLIT || npts <= kPointTile) return points_parts(npts, pulse_split);
-    if (pulse_split <= 1) pulse_split = split_points_auto_split(npts, kMaxAutoSplit);
-    return points_order_space(npts) + points_parts(npts, pulse_split);
+    // The automatic split is largest for endlessly many pulses.
+    if (pulse_split == 0) pulse_split = mode == SARBP_SPLIT && npts > 0 ? split_points_auto_split(npts, INT_MAX) : 1;
+    const size_t parts = points_parts(npts, pulse_split);
+    return mode != SARBP_SPLIT || npts <= kPointTile ? parts : points_order_space(npts) + parts;
 }
 
 int sarbp_backproject_points(const float* data, int pulses, int samples, const double* pos, const double* weight,
@@ -389,36 +387,32 @@ int sarbp_backproject_points(const float* data, int pulses, int samples, const d
     if (int st = check_pulses(data, pulses, samples, pos, weight, phase, data_dr, k)) return st;
     if (!xyz || !out) return fail(SARBP_ERR_TYPE, "xyz and out must not be NULL");
     if (npts <= 0) return fail(SARBP_ERR_VALUE, "at least one point is required");
-    if (pulse_split < 1 || pulse_split > pulses) return fail(SARBP_ERR_VALUE, "pulse_split must be in [1, pulses]");
-    if (mode != SARBP_SPLIT && pulse_split != 1) return fail(SARBP_ERR_VALUE, "pulse_split applies to split mode only");
-    size_t need = points_parts(npts, pulse_split);
+    if (pulse_split < 0 || pulse_split > pulses)
+        return fail(SARBP_ERR_VALUE, "pulse_split must be in [1, pulses], or 0 (automatic)");
+    if (mode != SARBP_SPLIT && pulse_split > 1) return fail(SARBP_ERR_VALUE, "pulse_split applies to split mode only");
+    if (pulse_split == 0) pulse_split = mode == SARBP_SPLIT ? split_points_auto_split(npts, pulses) : 1;
+    const size_t need = points_parts(npts, pulse_split);
     if (need && (!workspace || workspace_bytes < need))
         return fail(SARBP_ERR_WORKSPACE, "backproject_points needs %zu workspace bytes", need);
     cudaStream_t s = (cudaStream_t)stream;
     const PulseInputs in = inputs_of(data, pulses, samples, pos, weight, phase, range_start, data_dr, k);
     float2* dst = reinterpret_cast<float2*>(out);
     if (mode != SARBP_SPLIT) return launch_plain_points(mode, in, xyz, npts, 0, dst, s);
-    // With the workspace that the query asks for, the list is taken in spatial order and one pass over the
-    // pulses becomes the split that fills the GPU; with less (partial images only, or none) the list is
-    // taken as it is, in the split that was asked for.
+    // With the workspace that the query asks for, the list is taken in spatial order; with less (partial
+    // images only, or none), as it is.
     const PointOrder* order = nullptr;
     const int* index = nullptr;
     char* ws = static_cast<char*>(workspace);
-    int split = pulse_split;
-    if (npts > kPointTile && workspace && ((uintptr_t)workspace & 255) == 0) {
-        if (pulse_split == 1) split = split_points_auto_split(npts, std::min(pulses, kMaxAutoSplit));
-        if (workspace_bytes >= points_order_space(npts) + points_parts(npts, split)) {
-            if (int st = launch_points_order(xyz, npts, ws, &order, &index, s)) return st;
-            ws += points_order_space(npts);
-        } else {
-            split = pulse_split;
-        }
+    if (npts > kPointTile && workspace && ((uintptr_t)workspace & 255) == 0 &&
+        workspace_bytes >= points_order_space(npts) + need) {
+        if (int st = launch_points_order(xyz, npts, ws, &order, &index, s)) return st;
+        ws += points_order_space(npts);
     }
-    float2* parts = split > 1 ? reinterpret_cast<float2*>(ws) : dst;
+    float2* parts = pulse_split > 1 ? reinterpret_cast<float2*>(ws) : dst;
     const int wb = split_window_bins(kPointRadius, data_dr);
     const int ch = split_chunk_for(wb, 64);
-    int st = launch_split_points(in, xyz, npts, order, index, split, ch, wb, parts, npts, s);
-    if (st == SARBP_OK && split > 1) st = launch_sum_parts(parts, split, npts, npts, dst, s);
+    int st = launch_split_points(in, xyz, npts, order, index, pulse_split, ch, wb, parts, npts, s);
+    if (st == SARBP_OK && pulse_split > 1) st = launch_sum_parts(parts, pulse_split, npts, npts, dst, s);
     return st;
 }
 

@@ -225,7 +225,7 @@ struct PointOrder {
 size_t points_order_bytes(int npts);
 int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder** order, const int** index,
                         cudaStream_t s);
-// The pulse split that fills the GPU for this many points.
+// The pulse split that fills the GPU for this many points; the largest over all pulse counts is INT_MAX's.
 int split_points_auto_split(int npts, int pulses);
 // order: NULL, or the order in which the kernel takes the points (index: point of each place).
 int launch_split_points(const PulseInputs& in, const double* xyz, int npts, const PointOrder* order, const int* index,

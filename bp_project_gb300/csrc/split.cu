@@ -4071,8 +4071,24 @@ int launch_split_lattice(const PulseInputs& in, const sarbp_lattice& lat, int pu
 
 int split_points_auto_split(int npts, int pulses) {
     const size_t smem = dynamic_smem(capacity_for(kMaxChunk, 1 << 20), false);
-    if (prepare(split_points_kernel, smem) != SARBP_OK) return 1;
-    return best_pulse_split(split_points_kernel, kThreads, smem, (npts + kPointTile - 1) / kPointTile, pulses);
+    int dev = 0, sms = 0, per_sm = 0;
+    if (prepare(split_points_kernel, smem) != SARBP_OK || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, split_points_kernel, kThreads, smem) != cudaSuccess ||
+        per_sm <= 0 || sms <= 0) {
+        cudaGetLastError();
+        return 1;
+    }
+    // In pulses of a block: the blocks' work spread over the slots, each with its tile's set-up, which costs as much as
+    // 40 pulses, and one block more at the end (tiles of a list take unevenly long).  Parts also cost memory and a pass
+    // that adds them, hence a twentieth at least.  One pass, best of 2 .. 8 and this choice, us: 8,000 points x 512 pulses 182,
+    // 71 and 71; 192,384 x 1024 900, 610 and 623; 300,000 x 2000 2854, 1688 and 1694; a million x 256 735, 790 and 735.
+    const double waves = (double)((npts + (long long)kPointTile - 1) / kPointTile) / ((double)sms * per_sm);
+    const auto cost = [&](int sp) { return waves * (pulses + 40.0 * sp) + (double)pulses / sp + 40.0; };
+    int best = 1;
+    for (int sp = 2; sp <= 8 && sp <= pulses; ++sp)
+        if (cost(sp) < 0.95 * cost(1) && cost(sp) < cost(best)) best = sp;
+    return best;
 }
 
 int launch_split_points(const PulseInputs& in, const double* xyz, int npts, const PointOrder* order, const int* index,

@@ -154,9 +154,10 @@ int sarbp_direct_polar_static(const float* data, int pulses, int samples, const 
 /* Direct BP at arbitrary points xyz float64 [npts, 3]; out complex64 [npts].
  * Replaces ffbp.backproject_points (fast_bp/ffbp.py:43-55): phase k*r + phase[n],
  * not demodulated.  SPLIT mode groups points into tiles of 512.  With the workspace that the query
- * asks for (256-byte aligned), a list whose tiles would be wide is taken in spatial order and a single
- * pass over the pulses (pulse_split = 1) is split to fill the GPU; with less, consecutive points form the
- * tiles (spatially coherent lists are then the fast ones) and the split is the one asked for. */
+ * asks for (256-byte aligned), a list whose tiles would be wide is taken in spatial order; with less,
+ * consecutive points form the tiles (spatially coherent lists are then the fast ones).  pulse_split as for
+ * lattices: the number of passes over parts of the pulses, or 0 for the number that fills the GPU
+ * (1 where that gains little; 1 in the other modes, which take no other). */
 size_t sarbp_backproject_points_workspace(int mode, int npts, int pulse_split);
 int sarbp_backproject_points(const float* data, int pulses, int samples, const double* pos,
                              const double* weight, const double* phase, const double* xyz, int npts,
