@@ -68,10 +68,13 @@ __global__ void __launch_bounds__(kThreads) pga_targets_kernel(const double2* __
     }
 }
 
-// Order of doubles as signed integers (NaN with the sign bit clear above everything).
+// No number, of either sign (the GPU's own has the sign bit set), by integer operations.
+__device__ __forceinline__ bool no_number(long long bits) { return ((unsigned long long)bits << 1) > 0xffe0000000000000ull; }
+
+// Order of doubles as signed integers, what is no number above everything.
 __device__ __forceinline__ long long order_bits(double v) {
     const long long b = __double_as_longlong(v);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+    return no_number(b) ? 0x7fffffffffffffffll : b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 
 // numpy's median of v[0 .. n) (the two middle values' mean for even n): the values by rank, ties by index.
@@ -265,8 +268,12 @@ __global__ void __launch_bounds__(kTrackThreads) pga_finish_kernel(const double2
                                                                    double* __restrict__ stats) {
     __shared__ double part[33];
     __shared__ long long top[33];
-    // Largest of sizes by their bit patterns (integers; what is no number is above everything).
-    const auto size_bits = [](double v) { return __double_as_longlong(v) & 0x7fffffffffffffffll; };
+    // Largest of sizes by their bit patterns (integers; what is no number is above everything: tested apart, since the
+    // mask may be compiled to an absolute value, which keeps that one's sign).
+    const auto size_bits = [](double v) {
+        const long long b = __double_as_longlong(v);
+        return no_number(b) ? 0x7fffffffffffffffll : b & 0x7fffffffffffffffll;
+    };
     const auto block_max = [&](long long v) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
