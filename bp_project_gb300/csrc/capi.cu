@@ -578,7 +578,7 @@ int sarbp_pga_update(const double* smooth, int targets, int pulses, const double
         return fail(SARBP_ERR_VALUE, "1 to %d targets and at least two pulses are required", pga_max_targets());
     if (window < 1 || window % 2 != 1 || window > pulses)
         return fail(SARBP_ERR_VALUE, "window must be odd and at most the pulse count (got %d)", window);
-    if (!is_finite_value(k) || k == 0.0) return fail(SARBP_ERR_VALUE, "k must be finite and non-zero");
+    if (!is_finite_value(k)) return fail(SARBP_ERR_VALUE, "k must be finite");
     const size_t need = pga_update_workspace(targets, pulses);
     if (!workspace || workspace_bytes < need) return fail(SARBP_ERR_WORKSPACE, "pga_update needs %zu workspace bytes", need);
     return launch_pga_update(reinterpret_cast<const double2*>(smooth), targets, pulses, pos, xyz, k, centre, left, right,

@@ -49,3 +49,10 @@ def test_samples_that_are_no_numbers(monkeypatch, value):
     data, pts = scene(7, 0)
     data[20, :60] = value
     compare(*both(monkeypatch, data, pts))
+
+
+def test_without_a_wavenumber(monkeypatch):
+    """k = 0: gradients have no length, so the corrections are no numbers; the call is taken all the same."""
+    found, want = both(monkeypatch, *scene(5, 0), k=0.0)
+    assert bool(want[0][:, :2].isnan().all())
+    compare(found, want)
