@@ -1619,18 +1619,25 @@ __device__ __forceinline__ void lattice_runs(const SplitParams& P, const Rec* __
     }
 }
 
-// Pulses the fast path cannot stage, every second one from `first`, on the run's pixels: offsets in
-// two-float from FP64 (rare, and out of line so that it costs the fast path no registers).
+// Pulses the fast path cannot stage, every second one from `first`, on the run's pixels, out of line so that it
+// costs the fast path no registers.  The run's first offset in FP64, the others by steps in two-float: in FP64,
+// eight pixels a chunk in both halves of the block, the offsets took as long as the pulses.  256 pulses onto
+// 512 x 512 pixels of 1, 2 and 5 m (wide tiles): 290, 734 and 1557 us so, 268, 607 and 742 now (four pixels
+// per thread, before there were runs: 257, 583 and 908).
 __device__ __noinline__ void lattice_run_slow(const SplitParams& P, const TileShared& S, const sarbp_lattice& L, float di,
                                               float dj, int first, int nslow, int c0, const SlowRec* srec,
                                               float2* more) {
+    FF X, Y, Z;
+    const double i = (double)(di - 3.5f), j = (double)dj;
+    split2(i * L.step_row[0] + j * L.step_col[0], X.h, X.l);
+    split2(i * L.step_row[1] + j * L.step_col[1], Y.h, Y.l);
+    split2(i * L.step_row[2] + j * L.step_col[2], Z.h, Z.l);
 #pragma unroll 1
     for (int k = 0; k < kRun; ++k) {
-        const double i = (double)(di - 3.5f) + (double)k, j = (double)dj;
-        Pix q;
-        pixel_from_offsets(S, i * L.step_row[0] + j * L.step_col[0], i * L.step_row[1] + j * L.step_col[1],
-                           i * L.step_row[2] + j * L.step_col[2], q);
-        more[k] = slow_pixel(P, srec, first, nslow, 2, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, 0.0f);
+        more[k] = slow_pixel(P, srec, first, nslow, 2, c0, X.h, X.l, Y.h, Y.l, Z.h, Z.l, 0.0f);
+        X = ff_add(X, FF{S.sth[0], S.stl[0]});
+        Y = ff_add(Y, FF{S.sth[1], S.stl[1]});
+        Z = ff_add(Z, FF{S.sth[2], S.stl[2]});
     }
 }
 
