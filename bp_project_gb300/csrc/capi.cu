@@ -403,14 +403,14 @@ int sarbp_backproject_points(const float* data, int pulses, int samples, const d
     const PointOrder* order = nullptr;
     const int* index = nullptr;
     char* ws = static_cast<char*>(workspace);
+    const int wb = split_window_bins(kPointRadius, data_dr);
+    const int ch = split_chunk_for(wb, 64);
     if (npts > kPointTile && workspace && ((uintptr_t)workspace & 255) == 0 &&
         workspace_bytes >= points_order_space(npts) + need) {
-        if (int st = launch_points_order(xyz, npts, ws, &order, &index, s)) return st;
+        if (int st = launch_points_order(in, split_points_capacity(ch, wb), xyz, npts, ws, &order, &index, s)) return st;
         ws += points_order_space(npts);
     }
     float2* parts = pulse_split > 1 ? reinterpret_cast<float2*>(ws) : dst;
-    const int wb = split_window_bins(kPointRadius, data_dr);
-    const int ch = split_chunk_for(wb, 64);
     int st = launch_split_points(in, xyz, npts, order, index, pulse_split, ch, wb, parts, npts, s);
     if (st == SARBP_OK && pulse_split > 1) st = launch_sum_parts(parts, pulse_split, npts, npts, dst, s);
     return st;

@@ -1,8 +1,8 @@
 // Spatial order of a point list for split-precision direct BP.
 //
-// The points kernel forms tiles of 512 consecutive points; its fast path needs tiles of at most
-// about 20 m radius, while a raster of terrain points puts a tile on a strip of hundreds of metres
-// and every pulse on the two-float fallback.  These kernels order a list by the Hilbert curve of a 256 x 256
+// The points kernel forms tiles of 512 consecutive points; its fast path needs tiles of a limited
+// radius (points_radius: 22 m at 4 km and 9.6 GHz), while a raster of terrain points puts a tile on a strip of
+// hundreds of metres and every pulse on the two-float fallback.  These kernels order a list by the Hilbert curve of a 256 x 256
 // raster over its bounding square: two stable 8-bit counting passes, so the order (and with it the
 // image) is the same on every run.  Nothing is ordered when no tile is wide: the kernels
 // then return at once, and the points kernel takes the list as it is.
@@ -19,7 +19,6 @@ constexpr int kThreads = 256;
 // ordering instead of 67).
 constexpr int kMaxBlocks = 94;
 constexpr int kTilePoints = kPointTile;  // points per tile of the points kernel
-constexpr float kWideRadius = 16.0f;   // tiles above this radius (m) are worth ordering
 constexpr int kDigits = 256;
 
 // FP32 as an unsigned of the same order.
@@ -31,8 +30,11 @@ __device__ __forceinline__ float unordered(unsigned u) {
     return __uint_as_float(u & 0x80000000u ? u ^ 0x80000000u : ~u);
 }
 
-// Bounds of each tile: the list's bounding box, and whether any tile is wide.  One block per tile.
-__global__ void __launch_bounds__(kThreads) points_extent_kernel(const double* __restrict__ xyz, int npts,
+// Bounds of each tile: the list's bounding box, and whether any tile is wide (above the radius that the fast
+// path takes, seen from the first, middle or last pulse; a tile's own radius is about its points' mean and may be a
+// little larger than its box's).  One block per tile.
+__global__ void __launch_bounds__(kThreads) points_extent_kernel(PulseInputs in, float K, float inv_dr, float cap,
+                                                                 const double* __restrict__ xyz, int npts,
                                                                  PointOrder* __restrict__ h) {
     const float inf = __int_as_float(0x7f800000);
     float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
@@ -65,13 +67,23 @@ __global__ void __launch_bounds__(kThreads) points_extent_kernel(const double* _
             lo[c] = fminf(lo[c], part[w][c]);
             hi[c] = fmaxf(hi[c], part[w][3 + c]);
         }
-    float d2 = 0.0f;
+    float d2 = 0.0f, R2 = inf;
     for (int c = 0; c < 3; ++c) d2 += (hi[c] - lo[c]) * (hi[c] - lo[c]);
+    for (int k = 0; k < 3; ++k) {
+        const double* p = in.pos + 3LL * ((in.pulses - 1) * (long long)k / 2);
+        float r2 = 0.0f;
+        for (int c = 0; c < 3; ++c) {
+            const float d = (float)(p[c] - 0.5 * ((double)lo[c] + (double)hi[c]));
+            r2 = fmaf(d, d, r2);
+        }
+        R2 = fminf(R2, r2);
+    }
+    const float limit = points_radius(K, inv_dr, cap, sqrtf(R2)), radius = 1.1f * 0.5f * sqrtf(d2);
     for (int c = 0; c < 2; ++c) {
         atomicMin(&h->low[c], ordered(lo[c]));
         atomicMin(&h->high[c], ~ordered(hi[c]));
     }
-    atomicMin(&h->narrow, d2 <= 4.0f * kWideRadius * kWideRadius ? 1u : 0u);
+    atomicMin(&h->narrow, radius <= limit ? 1u : 0u);
 }
 
 // Place of cell (x, y) along the Hilbert curve of a 256 x 256 raster: level by level from the top, the
@@ -221,8 +233,8 @@ size_t points_order_bytes(int npts) {
 }
 
 // Orders the list in `ws` (points_order_bytes, 256-byte aligned); *order, *index: what the points kernel takes.
-int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder** order, const int** index,
-                        cudaStream_t s) {
+int launch_points_order(const PulseInputs& in, int cap, const double* xyz, int npts, void* ws, const PointOrder** order,
+                        const int** index, cudaStream_t s) {
     char* p = static_cast<char*>(ws);
     const auto take = [&p](size_t bytes) {
         char* at = p;
@@ -238,7 +250,8 @@ int launch_points_order(const double* xyz, int npts, void* ws, const PointOrder*
     auto* counts = reinterpret_cast<int*>(take(sizeof(int) * (size_t)kDigits * blocks));
     const cudaError_t e = cudaMemsetAsync(h, 0xff, sizeof(PointOrder), s);
     if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "points order: %s", cudaGetErrorString(e));
-    points_extent_kernel<<<(npts + kTilePoints - 1) / kTilePoints, kThreads, 0, s>>>(xyz, npts, h);
+    points_extent_kernel<<<(npts + kTilePoints - 1) / kTilePoints, kThreads, 0, s>>>(
+        in, (float)(in.k * kInvTwoPi), (float)(1.0 / in.data_dr), (float)cap, xyz, npts, h);
     points_count_kernel<true><<<blocks, kThreads, 0, s>>>(xyz, npts, per, h, keys, counts);
     points_scan_kernel<<<1, 1024, 0, s>>>(h, counts, kDigits * blocks);
     points_scatter_kernel<true><<<blocks, kThreads, 0, s>>>(npts, per, h, keys, nullptr, counts, keys1, index1);

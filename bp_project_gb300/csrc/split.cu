@@ -2242,31 +2242,62 @@ __global__ void __launch_bounds__(kThreads, 3) split_points_kernel(SplitParams P
     J.tile_u = 0;
     split_range(0, P.in.pulses, P.pulse_split, blockIdx.y, J.p0, J.p1);
     const int end = min(npts, J.tile_r + kPointTile);
-    // A tile whose list jumps (a spatial order leaves and re-enters the points' outline, targets follow each
-    // other) is formed stretch by stretch: one wide tile on the two-float fallback would take as long as seven
-    // others and hold up the launch's end.  Lists that jump all the time stay whole.
+    // A tile too wide for the fast path whose list jumps (a spatial order leaves and re-enters the points' outline,
+    // targets follow each other) is formed stretch by stretch: whole, on the two-float fallback, it would take as long
+    // as seven others and hold up the launch's end.  Lists that jump all the time stay whole.
     __shared__ unsigned jumps[kPointTile / 32];
-    constexpr float kJump2 = 16.0f * 16.0f;
-#pragma unroll
-    for (int k = 0; k < kPointPX; ++k) {
-        const int at = J.tile_r + threadIdx.x + kThreads * k;
-        bool jump = false;
-        if (at > J.tile_r && at < end) {
-            const double* a = xyz + 3LL * (J.index ? J.index[at] : at);
-            const double* b = xyz + 3LL * (J.index ? J.index[at - 1] : at - 1);
-            const float dx = (float)a[0] - (float)b[0], dy = (float)a[1] - (float)b[1], dz = (float)a[2] - (float)b[2];
-            jump = dx * dx + dy * dy + dz * dz > kJump2;
-        }
-        const unsigned w = __ballot_sync(0xffffffffu, jump);
-        if ((threadIdx.x & 31) == 0) jumps[(threadIdx.x + kThreads * k) >> 5] = w;
-    }
-    __syncthreads();
-    int njumps = 0;
-    for (int w = 0; w < kPointTile / 32; ++w) njumps += __popc(jumps[w]);
+    __shared__ float limit;
     float2* out = P.out + blockIdx.y * P.split_stride;
-    for (J.p_begin = J.tile_r; J.p_begin < end; J.p_begin = J.p_end) {
+    J.p_begin = J.tile_r;
+    J.p_end = end;
+    int njumps = -1;  // not looked for yet
+    while (J.p_begin < end) {
+        PointPix px[kPointPX];
+        setup_points(J, S, px);
+        if (njumps < 0) {
+            if (threadIdx.x < 32) {  // lanes 0 to 2: the range to the tile's first, middle and last pulse
+                const double* p = P.in.pos + 3LL * (J.p0 + (J.p1 - 1 - J.p0) * (long long)min(threadIdx.x, 2) / 2);
+                const float dx = (float)(S.cx - p[0]), dy = (float)(S.cy - p[1]), dz = (float)(S.cz - p[2]);
+                float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                r2 = fminf(r2, fminf(__shfl_sync(0xffffffffu, r2, 1), __shfl_sync(0xffffffffu, r2, 2)));
+                if (threadIdx.x == 0) limit = points_radius(P.Kf, P.inv_drf, (float)P.cap, sqrtf(r2));
+            }
+            __syncthreads();
+            njumps = 0;
+            if ((float)S.rho > limit) {
+                const float far = 0.7f * limit;
+#pragma unroll
+                for (int k = 0; k < kPointPX; ++k) {
+                    const int at = J.tile_r + threadIdx.x + kThreads * k;
+                    bool jump = false;
+                    if (at > J.tile_r && at < end) {
+                        const double* a = xyz + 3LL * (J.index ? J.index[at] : at);
+                        const double* b = xyz + 3LL * (J.index ? J.index[at - 1] : at - 1);
+                        const float dx = (float)a[0] - (float)b[0], dy = (float)a[1] - (float)b[1], dz = (float)a[2] - (float)b[2];
+                        jump = dx * dx + dy * dy + dz * dz > far * far;
+                    }
+                    const unsigned w = __ballot_sync(0xffffffffu, jump);
+                    if ((threadIdx.x & 31) == 0) jumps[(threadIdx.x + kThreads * k) >> 5] = w;
+                }
+                __syncthreads();
+                for (int w = 0; w < kPointTile / 32; ++w) njumps += __popc(jumps[w]);
+                if (njumps > 4) njumps = 0;
+                if (njumps > 0) J.p_end = J.tile_r;  // start over, with the first stretch
+            }
+        }
+        if (J.p_end > J.p_begin) {
+            PointsBody body{P, S, px};
+            chunk_loop(P, J, S, smem, true, body);
+#pragma unroll
+            for (int k = 0; k < kPointPX; ++k) {
+                const int idx = J.tile_r + threadIdx.x + kThreads * k;
+                if (idx >= J.p_begin && idx < J.p_end) out[J.index ? J.index[idx] : idx] = make_float2(px[k].ar, px[k].ai);
+            }
+        }
+        __syncthreads();  // the next stretch's set-up
+        J.p_begin = J.p_end;
         J.p_end = end;
-        if (njumps <= 4)
+        if (njumps > 0)
             for (int w = (J.p_begin + 1 - J.tile_r) >> 5, from = (J.p_begin + 1 - J.tile_r) & 31; w < kPointTile / 32;
                  ++w, from = 0) {
                 const unsigned rest = jumps[w] & (0xffffffffu << from);
@@ -2275,16 +2306,6 @@ __global__ void __launch_bounds__(kThreads, 3) split_points_kernel(SplitParams P
                     break;
                 }
             }
-        PointPix px[kPointPX];
-        setup_points(J, S, px);
-        PointsBody body{P, S, px};
-        chunk_loop(P, J, S, smem, true, body);
-#pragma unroll
-        for (int k = 0; k < kPointPX; ++k) {
-            const int idx = J.tile_r + threadIdx.x + kThreads * k;
-            if (idx >= J.p_begin && idx < J.p_end) out[J.index ? J.index[idx] : idx] = make_float2(px[k].ar, px[k].ai);
-        }
-        __syncthreads();  // the next stretch's set-up
     }
 }
 
@@ -4107,6 +4128,8 @@ int split_points_auto_split(int npts, int pulses) {
         if (cost(sp) < 0.95 * cost(1) && cost(sp) < cost(best)) best = sp;
     return best;
 }
+
+int split_points_capacity(int chunk, int window_bins) { return capacity_for(chunk, window_bins); }
 
 int launch_split_points(const PulseInputs& in, const double* xyz, int npts, const PointOrder* order, const int* index,
                         int pulse_split, int chunk, int window_bins, float2* out, long long split_stride,

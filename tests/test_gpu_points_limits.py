@@ -55,3 +55,19 @@ def test_short_range(lib, rows, cols, step):
 def test_wide_tiles_at_a_long_wavelength(lib):
     """Tiles of 33 km half-width from 360 km, k = 1e-5: the same order is 3e-3 bins of 400 m."""
     assert error(raster(60, 60, 2000.0, 3.0e5), 2.0e5, 100.0, 400.0, 1e-5) <= 1e-5
+
+
+@pytest.mark.parametrize("altitude,x0,step,cols,dr", [(223.0, 200.0, 0.1, 300, 0.2), (3000.0, 3.0e4, 0.5, 120, 0.4164),
+                                                      (3000.0, 3.0e4, 0.25, 300, 0.4164)])
+def test_rasters_at_near_and_far_ranges(lib, altitude, x0, step, cols, dr):
+    """9.6 GHz at 300 m, where tiles may have a radius of 6 m, and at 30 km, where 61 m fit: taken in spatial order or not."""
+    assert error(raster(20, cols, step, x0), altitude, 0.05, dr, 402.0) <= 1e-5
+
+
+@pytest.mark.parametrize("altitude,x0,gap", [(223.0, 200.0, 5.0), (3000.0, 3.0e4, 20.0), (3000.0, 3.0e4, 80.0)])
+def test_patches_at_near_and_far_ranges(lib, altitude, x0, gap):
+    """Patches of 170 points `gap` apart, three to a tile: formed whole where the tile fits, patch by patch where it does not."""
+    n = np.arange(1000)
+    rng = np.random.default_rng(7)
+    xyz = np.column_stack([x0 + gap * (n // 170) + rng.uniform(-0.5, 0.5, 1000), rng.uniform(-0.5, 0.5, 1000), 0.0 * n])
+    assert error(xyz, altitude, 0.05, 0.4, 402.0) <= 1e-5
