@@ -14,10 +14,6 @@ namespace sarbp {
 namespace {
 
 constexpr int kThreads = 256;
-// Blocks of a counting pass, at most, each on a whole number of rounds of kThreads keys.  192,384 points in 0.618 ms
-// all in all; with 188 blocks 0.621, 376 0.633, and 4096 keys per block 0.637 (8,000 points: 30 us of
-// ordering instead of 67).
-constexpr int kMaxBlocks = 94;
 constexpr int kTilePoints = kPointTile;  // points per tile of the points kernel
 constexpr int kDigits = 256;
 
@@ -142,8 +138,8 @@ __global__ void __launch_bounds__(kThreads) points_count_kernel(const double* __
 }
 
 // Exclusive prefix sum of n counts in place (one block, n a multiple of 4, counts 16-byte aligned): rounds of
-// four counts per thread, the next round's load in flight.  48,128 counts: 10 us, with a stretch of them per
-// thread 41.
+// four counts per thread, the next round's load in flight.  (48,128 counts, from 188 blocks: 10 us, with a stretch of
+// them per thread 41.)
 __global__ void __launch_bounds__(1024) points_scan_kernel(const PointOrder* __restrict__ h, int* __restrict__ counts,
                                                            int n) {
     if (h->narrow) return;
@@ -222,8 +218,21 @@ __global__ void __launch_bounds__(kThreads) points_scatter_kernel(int npts, int 
 }
 
 size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
-int keys_per_block(int npts) { return kThreads * ((npts + kThreads * kMaxBlocks - 1) / (kThreads * kMaxBlocks)); }
-int order_blocks(int npts) { return (npts + keys_per_block(npts) - 1) / keys_per_block(npts); }
+
+// Blocks of a counting pass: one per SM at most (the scan of their counts is the cost of more), each on a whole number
+// of rounds of kThreads keys.  192,384 points x 1024 pulses, all in all: 94 blocks 599 us, 152 (one per SM) 598, 188 601,
+// 376 611; six million points x 4 pulses 1131, 974, 935 and 855.
+int keys_per_block(int npts) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        sms <= 0) {
+        cudaGetLastError();
+        sms = 152;
+    }
+    const long long round = (long long)kThreads * sms;
+    return (int)(kThreads * ((npts + round - 1) / round));
+}
+int order_blocks(int npts) { return (int)(((long long)npts + keys_per_block(npts) - 1) / keys_per_block(npts)); }
 
 }  // namespace
 
