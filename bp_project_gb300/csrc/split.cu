@@ -351,9 +351,7 @@ __device__ void polar_tables(const SplitParams& P, const Job& J, TileShared& S, 
     __syncthreads();
 }
 
-__device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T, Pix px[kPX],
-                            bool demodulate) {
-    polar_tables<false>(P, J, S, T, demodulate);
+__device__ __forceinline__ void polar_pixels(const Job& J, const PolarTables& T, Pix px[kPX]) {
     const int tid = threadIdx.x, cols_t = 1 << J.lc;
 #pragma unroll
     for (int k = 0; k < kPX; ++k) {
@@ -372,6 +370,12 @@ __device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, P
         q.ar = q.ai = 0.0f;
     }
     __syncthreads();  // the tables alias the window region
+}
+
+__device__ void setup_polar(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T, Pix px[kPX],
+                            bool demodulate) {
+    polar_tables<false>(P, J, S, T, demodulate);
+    polar_pixels(J, T, px);
 }
 
 // Polar tile set-up from per-node tables of float pairs (FFBP):
@@ -848,12 +852,12 @@ struct SlowRec {
     float4 b;  // w.z hi, w.z lo, phase / 2pi reduced to [-1/2, 1/2], weight
 };
 
-// Sum over pulses c0 + first, c0 + first + step, ... below c0 + n of one pixel's contributions in two-float geometry.  Out of
-// line (and the pixel by value) so that the rarely taken fallback does not add registers
+// (ar, ai) plus the contributions of pulses c0 + first, c0 + first + step, ... below c0 + n to one pixel, in two-float
+// geometry.  Out of line (and the pixel by value) so that the rarely taken fallback does not add registers
 // to the kernels' fast path.
 __device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int first, int n, int step,
                                           int c0, float dxh, float dxl, float dyh, float dyl, float dzh, float dzl,
-                                          float psi);
+                                          float psi, float ar, float ai);
 
 // Dynamic shared memory of the chunk kernels: [records | windows]; the two-float records of
 // a chunk that stages no window live at the start of the window space.
@@ -1101,7 +1105,7 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
 
 __device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* srec, int first, int n, int step,
                                           int c0, float dxh, float dxl, float dyh, float dyl, float dzh, float dzl,
-                                          float psi) {
+                                          float psi, float ar, float ai) {
     Pix q;
     q.dxh = dxh;
     q.dxl = dxl;
@@ -1109,7 +1113,6 @@ __device__ __noinline__ float2 slow_pixel(const SplitParams& P, const SlowRec* s
     q.dyl = dyl;
     q.dzh = dzh;
     q.dzl = dzl;
-    float ar = 0.0f, ai = 0.0f;
     for (int j = first; j < n; j += step) {
         const SlowRec sr = srec[j];
         SlowSample o;
@@ -1506,9 +1509,10 @@ struct PolarBody {
 #pragma unroll
         for (int k = 0; k < kPX; ++k) {
             const Pix& q = px[k];
-            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, q.psi);
-            px[k].ar += v.x;
-            px[k].ai += v.y;
+            // Pulse by pulse onto the pixel's sum, so that the image does not depend on the chunks.
+            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, q.psi, q.ar, q.ai);
+            px[k].ar = v.x;
+            px[k].ai = v.y;
         }
     }
 };
@@ -1526,7 +1530,7 @@ struct PointsBody {
 #pragma unroll
         for (int k = 0; k < kPointPX; ++k) {
             const PointPix& q = px[k];
-            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dx, q.lx, q.dy, q.ly, q.dz, q.lz, 0.0f);
+            const float2 v = slow_pixel(P, srec, 0, nslow, 1, c0, q.dx, q.lx, q.dy, q.ly, q.dz, q.lz, 0.0f, 0.0f, 0.0f);
             px[k].ar += v.x;
             px[k].ai += v.y;
         }
@@ -1644,7 +1648,7 @@ __device__ __noinline__ void lattice_run_slow(const SplitParams& P, const TileSh
     split2(i * L.step_row[2] + j * L.step_col[2], Z.h, Z.l);
 #pragma unroll 1
     for (int k = 0; k < kRun; ++k) {
-        more[k] = slow_pixel(P, srec, first, nslow, 2, c0, X.h, X.l, Y.h, Y.l, Z.h, Z.l, 0.0f);
+        more[k] = slow_pixel(P, srec, first, nslow, 2, c0, X.h, X.l, Y.h, Y.l, Z.h, Z.l, 0.0f, 0.0f, 0.0f);
         X = ff_add(X, FF{S.sth[0], S.stl[0]});
         Y = ff_add(Y, FF{S.sth[1], S.stl[1]});
         Z = ff_add(Z, FF{S.sth[2], S.stl[2]});
@@ -2060,9 +2064,8 @@ struct PolarRun {
     float s1, s2, s3, s4, h;                    // s = side sqrt(1 - u^2): s^(j)(u) du^j / j!; du
 };
 
-__device__ __forceinline__ void setup_polar_runs(const SplitParams& P, const Job& J, TileShared& S, PolarTables& T,
-                                                 int row, int group, PolarRun& q) {
-    polar_tables<true>(P, J, S, T, true);
+__device__ __forceinline__ void polar_run(const Job& J, const TileShared& S, const PolarTables& T, int row, int group,
+                                          PolarRun& q) {
     const int m = kMaxCols + group;
     q.dxh = T.rxh[row] + T.cxh[m];  // exact: both multiples of the quantum
     q.dyh = T.ryh[row] + T.cyh[m];
@@ -2095,12 +2098,8 @@ __device__ __noinline__ void polar_run_slow(const SplitParams& P, const TileShar
         pixel_from_offsets(S, g.ox + (double)g.side * gr * sqrt(fmax(0.0, 1.0 - u * u)) - S.cx, g.oy + gr * u - S.cy, 0.0,
                            q);
         // Pulse by pulse onto the run's sums, so that the image does not depend on the chunks.
-        for (int j = first; j < nslow; j += 2) {
-            const float2 v = slow_pixel(P, srec, j, j + 1, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
-                                        (float)(t - rint(t)));
-            sum[k].x += v.x;
-            sum[k].y += v.y;
-        }
+        sum[k] = slow_pixel(P, srec, first, nslow, 2, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, (float)(t - rint(t)),
+                            sum[k].x, sum[k].y);
     }
 }
 
@@ -2162,6 +2161,36 @@ struct PolarRunBody {
     }
 };
 
+// Whether a polar tile is formed in runs, from 32 pulses spread over its range: they have to fit the fast path
+// and the runs' expansion, and the range has to change by less than kRunSpread bins on average from a run's middle to
+// its ends, so that runs of 32 neighbouring rows mostly stay within a bin.  Fully sampled apertures are at 0.006 (9.6 GHz,
+// 0.83 m bins); coarser angle steps and longer waves go pixel by pixel.  256 pulses onto 720 x 512, rows of 0.72 bins,
+// changes of 0.011, 0.016 and 0.021 bins: runs 181, 204 and 217 us, pixels 200, 212 and 211; rows of a bin: 160 (0.011)
+// and 167 (0.021), pixels 212 and 217.  Tiles too wide for the fast path: runs 1400 to 2050 us, pixels 990 to 1045
+// (890 to 940 in split_polar_kernel, which has their code alone).
+constexpr float kRunSpread = 0.02f;
+__device__ __forceinline__ bool polar_in_runs(const SplitParams& P, const Job& J, TileShared& S) {
+    __shared__ int runs;
+    if (threadIdx.x < 32) {
+        const double* p = P.in.pos + 3LL * (J.p0 + (J.p1 - 1 - J.p0) * (long long)threadIdx.x / 31);
+        const float vx = (float)(S.cx - p[0]), vy = (float)(S.cy - p[1]), vz = (float)(S.cz - p[2]), rho = (float)S.rho;
+        const float ax = S.sth[0] - vx, ay = S.sth[1] - vy, g2 = S.sth[0] * S.sth[0] + S.sth[1] * S.sth[1];
+        const float R = sqrtf(fmaf(vx, vx, fmaf(vy, vy, vz * vz))), iR = 1.0f / R;
+        const float du = (float)fabs(J.g.du), per_m = fabsf(P.inv_drf);
+        float spread = 3.5f * du * per_m * sqrtf(g2) * iR * fabsf(ay - ax * S.sth[1] / S.sth[0]);
+        const float turn = S.sth[3] * (fabsf(ax) + fabsf(ay)), y = turn * iR;
+        const bool fits = fabsf(P.Kf) * rho * rho <= (float)P.envelope * R && rho < 0.25f * R &&
+                          2.0f * rho * per_m + 4.0f <= (float)(kWindowBudget / 32) &&
+                          fabsf(P.Kf) * (fabsf(ax) * S.sth[2] + turn * (y * y) * (y * y)) <= 1e-7f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) spread += __shfl_xor_sync(0xffffffffu, spread, o);
+        const bool all = __all_sync(0xffffffffu, fits);
+        if (threadIdx.x == 0) runs = all && spread <= 32.0f * kRunSpread;
+    }
+    __syncthreads();
+    return runs != 0;
+}
+
 __global__ void __launch_bounds__(kThreads, 3) split_polar_runs_kernel(SplitParams P, PolarDesc g) {
     extern __shared__ __align__(16) char smem[];
     __shared__ TileShared S;
@@ -2170,16 +2199,26 @@ __global__ void __launch_bounds__(kThreads, 3) split_polar_runs_kernel(SplitPara
     J.lc = g.tile_lc;  // 3 to 5: whole runs, and a warp's 32 rows in one run of columns
     tile_of(blockIdx.x, g.win_nu, J.lc, J.tile_r, J.tile_u);
     split_range(g.a, g.b, P.pulse_split, blockIdx.y, J.p0, J.p1);
+    PolarTables& T = *reinterpret_cast<PolarTables*>(smem + window_offset());
+    polar_tables<true>(P, J, S, T, true);
+    float2* out = P.out + blockIdx.y * P.split_stride;
+    if (!polar_in_runs(P, J, S)) {
+        Pix px[kPX];
+        polar_pixels(J, T, px);
+        PolarBody body{P, px};
+        chunk_loop(P, J, S, smem, true, body);
+        store_window(J, g.win_nr, g.win_nu, px, out, P.out_stride);
+        return;
+    }
     const int rows_t = kSplitTilePixels >> J.lc, slot = threadIdx.x & (kRunThreads - 1);
     const int row = slot & (rows_t - 1), col = kColRun * (slot / rows_t);
     PolarRun q;
-    setup_polar_runs(P, J, S, *reinterpret_cast<PolarTables*>(smem + window_offset()), row, col / kColRun, q);
+    polar_run(J, S, T, row, col / kColRun, q);
     float ar[kColRun], ai[kColRun];
 #pragma unroll
     for (int k = 0; k < kColRun; ++k) ar[k] = ai[k] = 0.0f;
     PolarRunBody body{P, S, g, J.p0, q, g.win_r0 + J.tile_r + row, g.win_u0 + J.tile_u + col, ar, ai};
     chunk_loop(P, J, S, smem, true, body);
-    float2* out = P.out + blockIdx.y * P.split_stride;
     add_halves(reinterpret_cast<float2*>(smem + window_offset()), body.group(), slot, ar, ai, [&](int k, float2 v) {
         const int wr = J.tile_r + row, wu = J.tile_u + col + k;
         if (wr < g.win_nr && wu < g.win_nu) out[(long long)wr * P.out_stride + wu] = v;
