@@ -2560,7 +2560,7 @@ struct LeafMid {
     float du;
     float lim;  // half a bin, or below 0: the run's pixels take their own window entries
     int runs;   // the expansion holds for the leaf's pulses
-    int pad;
+    int first;  // floor(Q) of the tile's first row
 };
 
 constexpr int kLeafRun = kColRun;                             // columns per thread
@@ -2638,18 +2638,25 @@ __device__ __forceinline__ LeafMid leaf_mid(const SplitParams& P, const PolarDes
     M.s3 = M.s2 * uf * hc * ic;
     M.s4 = M.s2 * 0.25f * (1.0f + 4.0f * u2) * (hc * ic) * (hc * ic);
     M.du = h;
-    // What the expansion leaves out: the fifth and sixth order of s, and the fifth of the root.
+    // Orders five to seven go into the lower ones: over the run's four |m|, m^5 ~ 15.5 m^3 - 47.3125 m within 26.25,
+    // m^6 ~ 16.396 m^4 - 55.051 m^2 within 52.25 and m^7 ~ 203.44 m^3 - 809.47 m within 544.7 (m^5 itself goes to 525).
+    const float w = hc * ic, d4 = 1.0f / (1.0f + 4.0f * u2), s5 = M.s4 * uf * w * (3.0f + 4.0f * u2) * d4;
+    const float s6 = M.s4 * w * w * 0.5f * (1.0f + 12.0f * u2 + 8.0f * u2 * u2) * d4;
+    const float s7 = M.s4 * uf * w * w * w * 0.5f * (5.0f + 20.0f * u2 + 8.0f * u2 * u2) * d4;
+    M.s1 += fmaf(-47.3125f, s5, -809.46875f * s7);
+    M.s2 = fmaf(-55.050652f, s6, M.s2);
+    M.s3 += fmaf(15.5f, s5, 203.4375f * s7);
+    M.s4 = fmaf(16.395735f, s6, M.s4);
+    // What that leaves, and the fifth order of the root.
     const float m = 0.5f * (kLeafRun - 1), m2 = m * m;
-    const float q5 = fabsf(M.s4 * uf) * (hc * ic) * (3.0f + 4.0f * u2) / (1.0f + 4.0f * u2);
-    const float q6 = fabsf(M.s4) * (hc * ic) * (hc * ic) * 0.5f * (1.0f + 12.0f * u2 + 8.0f * u2 * u2) / (1.0f + 4.0f * u2);
     const float ir = 1.0f / r_min, turn = m * hc * 1.5f * amax, y = turn * ir / fabsf(P.Kf);
-    const float rest = axmax * m2 * m2 * m * (q5 + m * q6) + turn * (y * y) * (y * y);
+    const float rest = axmax * (26.25f * fabsf(s5) + 52.25f * fabsf(s6) + 544.7f * fabsf(s7)) + turn * (y * y) * (y * y);
     M.runs = rest <= 5e-8f && fabsf(P.Kf) > 1e-3f ? 1 : 0;
     // The sample's cubic in m leaves out the square of the quadratic term.
     const float kb = fabsf(P.inv_drf / P.Kf);
     const float x1 = turn * kb, x2 = m2 * (axmax * fabsf(M.s2)) * kb + 0.5f * turn * y * kb;
     M.lim = (3.0f * x1 * x1 + x2) * x2 <= 1e-7f ? 0.5f : -1.0f;
-    M.pad = 0;
+    M.first = 0;
     return M;
 }
 
@@ -2689,7 +2696,7 @@ __device__ __forceinline__ void leaf_runs(int part, const SplitParams& P, const 
 }
 
 // n pulses from c0 on the run's pixels one by one, with the taps from the pulse rows: pulses whose
-// window does not fit, and columns too wide for the expansion (both rare, hence out of line).
+// window does not fit (rare, hence out of line).
 __device__ __noinline__ void leaf_direct(const SplitParams& P, const PolarDesc* __restrict__ node,
                                          const float4* __restrict__ tables, const PulseRec* __restrict__ precs, int i, int j0, int c0, int n,
                                          float2* __restrict__ more) {
@@ -2741,6 +2748,96 @@ __device__ __noinline__ void leaf_direct(const SplitParams& P, const PolarDesc* 
     }
 }
 
+// The n pulses of a chunk onto the run's pixels one by one, in tiles with a run whose expansion does not hold (coarse
+// angle steps at squint): staged windows as in leaf_runs, C and D per column.  A warp's lanes form those of eight
+// columns and some pulses at a time in its part of the columns' shared memory.  n = 0: pulse c0 alone, whose
+// window does not fit (leaf_direct).  Out of line, two columns at a time, which leaves leaf_runs its registers (4096
+// pulses in 256 leaves: with eight at a time the whole image takes 8.05 ms instead of 7.91).  1024 pulses in 64 leaves
+// at 435 MHz and u = 0.5, whole image: 142 us, with the taps from the pulse rows (leaf_direct) 198, a pixel pair per thread,
+// before there were runs, 131; 256 leaves of 4 at 9.6 GHz and u = 0.7: 430, 493 and 417.
+template <int PARTS>
+__device__ __noinline__ void leaf_pixels(const SplitParams& P, const PolarDesc* __restrict__ node,
+                                         const float4* __restrict__ tables, const PulseRec* __restrict__ precs, int i, int j0,
+                                         int c0, int n, float2* __restrict__ sum) {
+    extern __shared__ __align__(16) char smem[];
+    const LeafRec* rec = reinterpret_cast<const LeafRec*>(smem);
+    float4* cols = reinterpret_cast<float4*>(smem + leaf_col_offset());
+    const char* win = smem + leaf_window_offset();
+    const int part = threadIdx.x / kLeafThreads;
+    if (n == 0) {
+        float2 all[kLeafRun];
+        leaf_direct(P, node, tables, precs, i, j0, c0, 1, all);
+#pragma unroll
+        for (int k = 0; k < kLeafRun / PARTS; ++k) {
+            const float2 v = all[PARTS == 1 ? k : run_column<PARTS>(part, k / 2, k % 2)];
+            sum[k].x += v.x;
+            sum[k].y += v.y;
+        }
+        return;
+    }
+    const int I_first = reinterpret_cast<const LeafMid*>(smem + leaf_mid_offset())->first;
+    constexpr int kWarps = kLeafThreads * PARTS / 32, kPulses = kMaxLeafChunk * kLeafGroups * (int)sizeof(LeafCol) /
+                                                                (kWarps * kLeafRun * (int)sizeof(float4));
+    static_assert(kPulses * kLeafRun % 32 == 0, "whole warps of (pulse, column)");
+    const PolarDesc& g = *node;
+    const int lane = threadIdx.x & 31;
+    float4* mine = cols + (threadIdx.x >> 5) * (kPulses * kLeafRun);
+    const LeafRow q = leaf_row(g, tables, i, I_first);
+    const float4 cv = __ldg(tables + g.cols_off + min(j0 + (lane & (kLeafRun - 1)), g.nu - 1));
+    const float side = (float)g.side;
+    for (int b = 0; b < n; b += kPulses) {
+        __syncwarp();
+#pragma unroll 1
+        for (int e = lane; e < kPulses * kLeafRun; e += 32)
+            if (b + e / kLeafRun < n) mine[e] = leaf_col(precs[c0 + b + e / kLeafRun], cv, side);
+        __syncwarp();
+#pragma unroll 1
+        for (int k = 0; k < kLeafRun / PARTS; k += 2) {
+            float ar[2], ai[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                ar[h] = sum[k + h].x;
+                ai[h] = sum[k + h].y;
+            }
+#pragma unroll 1
+            for (int nl = b; nl < min(b + kPulses, n); ++nl) {
+                const float4 ra = rec[nl].p0, rb = rec[nl].p1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float4 cd = mine[(nl - b) * kLeafRun + (PARTS == 1 ? k + h : run_column<PARTS>(part, (k + h) / 2, (k + h) % 2))];
+                    const float L = fmaf(q.a, cd.x, q.b * ra.x);
+                    const float nq2 = fmaf(L, L, ra.y);
+                    const float B = rcp_approx(fmaf(-2.0f, L, q.r2));
+                    const float ne0 = nq2 * B;
+                    const float neps = fmaf(ne0 * ne0, B, ne0);
+                    const float qp = fmaf(-L - neps, P.inv_drf, q.fm);
+                    const float t = qp + kMagic, f = qp - (t - kMagic);
+                    const float4* w = reinterpret_cast<const float4*>(
+                        win + __float_as_int(rb.z) +
+                        min(32u * (unsigned)(__float_as_int(t) + q.o) + (unsigned)__float_as_int(rb.y), (unsigned)__float_as_int(rb.w)));
+                    const float4 c01 = w[0], c23 = w[1];
+                    const float vr = fmaf(fmaf(fmaf(c23.z, f, c23.x), f, c01.z), f, c01.x);
+                    const float vi = fmaf(fmaf(fmaf(c23.w, f, c23.y), f, c01.w), f, c01.y);
+                    const float tb = fmaf(q.ah, cd.y, q.bh * ra.z);
+                    float sm = fmaf(-P.Kf, neps, rb.x);
+                    sm = fmaf(q.ah, cd.z, sm);
+                    sm = fmaf(q.al, cd.w, sm);
+                    sm = fmaf(q.bh, ra.w, sm);
+                    sm = fmaf(q.bl, ra.z + ra.w, sm);
+                    float sn, cs;
+                    __sincosf(((tb - round_magic(tb)) + sm) * kTwoPiF, &sn, &cs);
+                    ar[h] = fmaf(vr, cs, ar[h]);
+                    ar[h] = fmaf(-vi, sn, ar[h]);
+                    ai[h] = fmaf(vr, sn, ai[h]);
+                    ai[h] = fmaf(vi, cs, ai[h]);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) sum[k + h] = make_float2(ar[h], ai[h]);
+        }
+    }
+}
+
 // One leaf tile: the per-item body of the leaf kernels.  precs holds the pulse records of
 // the leaf's scene (indexed by pulse); a node with a destination pointer writes there.  PARTS = 2: two threads
 // per run, for launches of few tiles.
@@ -2778,6 +2875,8 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     if (part == 0 && lane == 0 && row == 0) {
         const float4 pd = precs[g.a].d;
         mids[group] = leaf_mid(P, g, jpix, r_min, pd.z, pd.w);
+        mids[group].first = I_first;
+        if (it.tile_u + kLeafRun * group >= g.win_nu) mids[group].runs = 1;  // past the window: nothing to be exact about
     }
     for (int c0 = g.a; c0 < g.b;) {
         const int want = min(P.chunk, g.b - c0);
@@ -2813,9 +2912,9 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
         __syncthreads();
         const int nfit = s_nfit;
         const int chn = nfit > 0 ? nfit : 1;
-        const LeafMid& M = mids[group];
-        const bool runs = M.runs != 0 && nfit > 0;
-        for (int e = tid; e < nfit * groups; e += kThr) {  // one (pulse, run of columns) each
+        bool runs = true;  // all of the tile's
+        for (int gi = 0; gi < groups; ++gi) runs = runs && mids[gi].runs != 0;
+        for (int e = tid; e < nfit * groups && runs; e += kThr) {  // one (pulse, run of columns) each
             const int nl = e / groups, gi = e - nl * groups;
             const LeafMid& m = mids[gi];
             const PulseRec pr = precs[c0 + nl];
@@ -2830,16 +2929,17 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
                               win + __float_as_int(rec[nl].p1.z) / 16, lane);
         }
         __syncthreads();
-        if (runs) {
-            leaf_runs<PARTS>(part, P, rec, cols + group, reinterpret_cast<const char*>(win), nfit, q, M.lim, ar, ai);
+        if (runs && nfit > 0) {
+            leaf_runs<PARTS>(part, P, rec, cols + group, reinterpret_cast<const char*>(win), nfit, q, mids[group].lim, ar, ai);
         } else {
-            float2 more[kLeafRun];
-            leaf_direct(P, nodes + it.node, tables, precs, ipix, jpix, c0, chn, more);
+            float2 sum[kLeafRun / PARTS];
+#pragma unroll
+            for (int k = 0; k < kLeafRun / PARTS; ++k) sum[k] = make_float2(ar[k], ai[k]);
+            leaf_pixels<PARTS>(P, nodes + it.node, tables, precs, ipix, jpix, c0, nfit, sum);
 #pragma unroll
             for (int k = 0; k < kLeafRun / PARTS; ++k) {
-                const float2 v = more[PARTS == 1 ? k : run_column<PARTS>(part, k / 2, k % 2)];
-                ar[k] += v.x;
-                ai[k] += v.y;
+                ar[k] = sum[k].x;
+                ai[k] = sum[k].y;
             }
         }
         c0 += chn;
