@@ -36,6 +36,13 @@ int check_launch(const char* what) {
     return SARBP_OK;
 }
 
+int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    return sms > 0 ? sms : 152;
+}
+
 int allow_shared(const void* kernel, size_t smem) {
     if (smem <= 40 * 1024) return SARBP_OK;  // 48 KB without the attribute, static shared memory included
     cudaFuncAttributes a;

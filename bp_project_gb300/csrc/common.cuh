@@ -160,6 +160,8 @@ int split_direct_polar(const PulseInputs& in, const sarbp_polar_grid& grid, int 
 // Lets `kernel` be launched with `smem` bytes of dynamic shared memory on the current device.  The limit is the
 // kernel's, not the launch's, and threads share it: it goes to the most that a block can have, and only up.
 int allow_shared(const void* kernel, size_t smem);
+// SMs of the current device (152 where it cannot be asked).
+int sm_count();
 
 // Plain (reference-arithmetic) kernels.
 int launch_plain_polar(int mode, const PulseInputs& in, const PolarDesc& g, int pulse_begin, int pulse_end,

@@ -223,13 +223,7 @@ size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
 // of rounds of kThreads keys.  192,384 points x 1024 pulses, all in all: 94 blocks 599 us, 152 (one per SM) 598, 188 601,
 // 376 611; six million points x 4 pulses 1131, 974, 935 and 855.
 int keys_per_block(int npts) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        sms <= 0) {
-        cudaGetLastError();
-        sms = 152;
-    }
-    const long long round = (long long)kThreads * sms;
+    const long long round = (long long)kThreads * sm_count();
     return (int)(kThreads * ((npts + round - 1) / round));
 }
 int order_blocks(int npts) { return (int)(((long long)npts + keys_per_block(npts) - 1) / keys_per_block(npts)); }

@@ -4350,7 +4350,7 @@ int launch_split_ffbp_leaves(const PulseInputs& in, const PolarDesc* nodes, cons
     // With up to two tiles per SM a sub-partition has only one or two of their warps, and a tile's latency
     // counts: two threads per run (the same image).  32 pulses, 150 tiles: 16.3 us, one thread per run 20.8;
     // 240 tiles 22.3 and 24.4; 160 tiles of 64 pulses 36.6 and 37.3; four threads per run 17.7, 32.6 and 55.0.
-    const bool few = nitems <= 2 * 152;
+    const bool few = nitems <= 2 * sm_count();
     const auto kernel = few ? split_leaf_kernel<2> : split_leaf_kernel<1>;
     if (int st = prepare(kernel, smem)) return st;
     kernel<<<nitems, kLeafThreads * (few ? 2 : 1), smem, s>>>(P, nodes, items, tables,
