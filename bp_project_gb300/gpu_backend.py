@@ -118,7 +118,7 @@ def build_ffbp_plan(position, fc, extent, side=1, leaf_size=128, range_spacing=0
     the sector about its own phase centre with 8-cell guards; leaves hold at
     most ``leaf_size`` pulses and nodes split at ``(a+b)//2``.  The numpy
     operations are the reference's on each value, in its order, so the integer
-    grid sizes and the crop match the reference bit for bit; they run on all
+    grid sizes and the crop match the reference bit for bit; they run on many
     nodes at once (31 nodes: 0.39 ms, one by one 0.81).
     """
     position = np.ascontiguousarray(position, dtype=np.float64)
@@ -166,13 +166,17 @@ def build_ffbp_plan(position, fc, extent, side=1, leaf_size=128, range_spacing=0
             np.minimum(low[left[i]], low[right[i]], out=low[i])
             np.maximum(high[left[i]], high[right[i]], out=high[i])
     span = high - low
-    # The sector boundary seen from every phase centre.
-    dx = bx[None, :] - origins[:, :1]
-    dy = by[None, :] - origins[:, 1:2]
-    gr = np.sqrt(dx * dx + dy * dy)
-    rr = np.sqrt(gr * gr + np.array([[o ** 2] for o in origins[:, 2]]))
-    uu = dy / gr
-    edges = [v.tolist() for v in (rr.min(axis=1), rr.max(axis=1), uu.min(axis=1), uu.max(axis=1))]
+    # The sector boundary seen from every phase centre, 128 nodes at a time: half a megabyte per array, whatever the tree.
+    edges = [[], [], [], []]
+    for at in range(0, count, 128):
+        o = origins[at:at + 128]
+        dx = bx[None, :] - o[:, :1]
+        dy = by[None, :] - o[:, 1:2]
+        gr = np.sqrt(dx * dx + dy * dy)
+        rr = np.sqrt(gr * gr + np.array([[z ** 2] for z in o[:, 2]]))
+        uu = dy / gr
+        for values, v in zip(edges, (rr.min(axis=1), rr.max(axis=1), uu.min(axis=1), uu.max(axis=1))):
+            values += v.tolist()
     counts = {"leaves": 0, "merges": 0, "leaf_pixel_pulse_products": 0, "merged_pixels": 0}
     nodes = []
     for i, (a, b) in enumerate(ranges):
