@@ -90,7 +90,8 @@ struct Rec {
                // middle's place in the window in 2^-28 bins (integers); b = u, 2R; c.y that place, FP32;
                // d = rest of W, rest of u.x / dr; e.w rest of u.y / dr)
     float4 d;  // u.z, W_hi.z, W_lo.z                (polar runs: -2 pi K a.x, -2 pi K a.y with a = pos - origin, the
-               // limit of column_run; lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z)
+               // limit of column_run; lattice adjoint: 2 pi frac(m B_row), u.x, u.y, u.z; lattice forward: the start phases
+               // of even and odd pixels from Phi', radians)
     float4 e;  // lattice adjoint: the pairs (2R, 2R), (frac(Q) - 1/2, frac(Q) - 1/2) of packed-FP32 operands;
                // lattice forward: (-, window bias bits, window offset bits, window count - 1 bits)
 };
@@ -1064,14 +1065,19 @@ __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, 
             r.c = make_float4(fmaf(-21.0625f * P.Kf, e4, t1), 0.0f, 0.0f, 12.5f * e4);
             // The phase step reduced modulo half a turn, which keeps the angles along a run small: the step is
             // spT + N / 2 with |spT| <= 1/4, and pixel k = 2 g - 3.5 + c adds k N / 2 = (g - 2) N + (2 c + 1) N / 4
-            // turns: N / 4 for the even pixels of the run (c = 0) and half of N more for the odd ones.
+            // turns: N / 4 for the even pixels of the run (c = 0) and half of N more for the odd ones.  Half a turn more
+            // is a quarter before and a quarter after a middle phase: the angles stay within 10 rad instead of 12, and the
+            // two starts are one packed operation (192 pulses onto 96 x 128: error 3.01e-7 -> 2.89e-7 on average over 12
+            // scenes, one pixel at a time 2.91e-7; 4096 onto 2048 x 2048: 17.10 -> 16.94 ms).
             const float n2 = rintf(2.0f * sp);
             const float even = 0.25f * (n2 + 2.0f * turns);
             r.c.z = (sp - 0.5f * n2) * kTwoPiF;
             r.c.x += even - rintf(even);
-            const float odd = 0.5f * n2;
-            r.d.x = odd - rintf(odd);
-            r.d.y = r.d.z = r.d.w = 0.0f;
+            const float odd = 0.5f * n2, q = 0.5f * fabsf(odd - rintf(odd));
+            r.c.x += q;
+            r.d.x = -q * kTwoPiF;
+            r.d.y = q * kTwoPiF;
+            r.d.z = r.d.w = 0.0f;
             r.c.x = __int_as_float(wrap(FF{r.c.x, 0.0f}));
         } else {
             r.b = make_float4(Ar, Ac, 2.0f * Rf, Fm);
@@ -1560,7 +1566,7 @@ struct PointsBody {
 // What bounds the loop: the register file feeds two operands a cycle to the FMA pipe (a fused
 // multiply-add of three registers takes 1.5 cycles, a packed one 3), so issue sits at 71% with the
 // FMA pipe, the shared-memory pipe and issue all at 60-70%, and every instruction removed shows in
-// the time.  4096 pulses onto 2048 x 2048: 17.05 ms (1008 Gpixel-pulses/s; 28.9 instructions per
+// the time.  4096 pulses onto 2048 x 2048: 16.94 ms (1014 Gpixel-pulses/s; 28.9 instructions per
 // pixel-pulse), 19.6 ms (876; 31.3) with four pixels per thread and the root-free range chain of the
 // adjoint per pixel.  Measured and not kept: runs of 16 (24 warps per SM instead of 32: 16.7 ms, but a larger
 // error on small scenes), the range to the middle in integers too (18.3; error 0.68e-6 instead of 0.80), even
@@ -1598,7 +1604,7 @@ __device__ __forceinline__ void lattice_runs(const SplitParams& P, const Rec* __
         const float e3 = -a * e2 * iD;
         float P0 = fmaf(P.Kf, eps, (float)turns * 2.3283064365386963e-10f);
         P0 -= round_magic(P0);
-        const float2 p0 = __fmul2_rn(make_float2(P0, P0 + rd.x), pair(kTwoPiF));
+        const float2 p0 = __ffma2_rn(pair(P0), pair(kTwoPiF), rd);
         const float2 p1 = pair(fmaf(kr, e1, rc.z));
         const float2 p2 = pair(kr * e2), p3 = pair(kr * e3);
         const float2 q0 = pair(fmaf(Le, inv_dr, rb.w)), q1 = pair(a * inv_dr), q2k = pair(e2 * inv_dr);
