@@ -225,8 +225,9 @@ class CudaBaseline:
     """Execute BP / FFBP with libsarbp (fast_bp/gpu_backend.py:227-561 surface)."""
 
     kernel_names = (
-        "plain_polar_kernel<fp64|fp32|mixed>", "split_polar_kernel", "split_lattice_kernel", "split_points_kernel",
-        "split_leaf_kernel", "split_merge_kernel", "plain_ffbp_leaf_kernel", "plain_ffbp_merge_kernel",
+        "plain_polar_kernel<fp64|fp32|mixed>", "split_polar_kernel", "split_polar_runs_kernel", "split_lattice_kernel",
+        "split_points_kernel", "split_leaf_kernel", "split_merge_kernel", "split_merge_staged_kernel",
+        "plain_ffbp_leaf_kernel", "plain_ffbp_merge_kernel",
         "plain_regrid_kernel", "plain_merge_kernel", "evaluate_kernel", "target_contrib_kernel", "add_kernel",
         "cast_kernel", "crop_kernel", "sum_parts_kernel",
     )
