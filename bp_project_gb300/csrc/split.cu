@@ -933,7 +933,7 @@ __device__ __noinline__ void slow_record(const SplitParams& P, const TileShared&
 // arithmetic (about 44 bits; GB300's FP64 rate would make these records the barrier-bound
 // part of every chunk).  Returns the number of window entries the pulse needs (cap + 1 if
 // it cannot be staged).
-// MODE 0: per-pixel offsets (polar); 1: lattice tiles; 2: lattice tiles, adjoint; 3: points.
+// MODE 0: per-pixel offsets (polar); 1: lattice tiles; 2: lattice tiles, adjoint; 3: points; 4: polar tiles in runs.
 template <int MODE>
 __device__ __forceinline__ int make_record(const SplitParams& P, TileShared& S, Rec* rec, int lane, int n) {
     const PulseInputs& in = P.in;
@@ -1927,7 +1927,7 @@ struct LatticeAdjointBody {
         const float di = (float)((tid >> lc) + 2 * m - hr);
         const float dj = (float)((tid & (cols_t - 1)) - (cols_t >> 1));
         const float mf = (float)m;
-        // The forward's packed pixel pairs (see lattice_chunk), plus R + (L + eps) as a pair.
+        // Pixel pairs as f32x2 lanes: -L, -q2, -e0 and -eps are carried (negation is exact), plus R + (L + eps).
         const float2 nd2[2] = {make_float2(-d2[0], -d2[1]), make_float2(-d2[2], -d2[3])};
         const float2 kcs[2] = {make_float2(-2.0f, -1.0f), make_float2(0.0f, 1.0f)};
         const float2 ninv = pair(-inv_dr), nkr = pair(-kr), magic = pair(kMagic), nmagic = pair(-kMagic);

@@ -120,7 +120,8 @@ def backproject_points(data, pos, xyz, r_start, dr, k, weight, phase, mode=DEFAU
 
     In split mode a host point list that is an affine lattice in row-major order (the ground
     meshgrids of run.py) is imaged by the lattice kernel, whose row/column terms make it the
-    fastest path; any other point list goes through the points kernel in Morton order."""
+    fastest path; any other host list goes to the points kernel in Morton order (which takes lists whose tiles
+    are still too wide in an order of its own), and a list on the device as it is."""
     keep = _on_device(data, xyz)
     d, p, w, ph = _inputs(data, pos, weight, phase)
     order = None
