@@ -2104,8 +2104,12 @@ __device__ __noinline__ void polar_run_slow(const SplitParams& P, const TileShar
         pixel_from_offsets(S, g.ox + (double)g.side * gr * sqrt(fmax(0.0, 1.0 - u * u)) - S.cx, g.oy + gr * u - S.cy, 0.0,
                            q);
         // Pulse by pulse onto the run's sums, so that the image does not depend on the chunks.
-        sum[k] = slow_pixel(P, srec, first, nslow, 2, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl, (float)(t - rint(t)),
-                            sum[k].x, sum[k].y);
+        for (int j = first; j < nslow; j += 2) {
+            const float2 v = slow_pixel(P, srec, j, j + 1, 1, c0, q.dxh, q.dxl, q.dyh, q.dyl, q.dzh, q.dzl,
+                                        (float)(t - rint(t)), 0.0f, 0.0f);
+            sum[k].x += v.x;
+            sum[k].y += v.y;
+        }
     }
 }
 
@@ -2113,7 +2117,7 @@ __device__ __noinline__ void polar_run_slow(const SplitParams& P, const TileShar
 // lattice tiles' do.  Range, phase and window place are worked out once per run (split arithmetic at its
 // middle, as polar_chunk does per pixel) and expanded along it from the polar geometry (run_phase).
 // What bounds it: instruction issue (77% of the cycles, 248 instructions per warp and pulse) and the last of
-// few waves.  1024 pulses onto 720 x 1600: 1.28 ms, pixel by pixel (polar_chunk) 1.76; with every pixel on its
+// few waves.  1024 pulses onto 720 x 1600: 1.27 ms, pixel by pixel (polar_chunk) 1.76; with every pixel on its
 // own window entry 1.66, with 64 registers and four blocks per SM 1.35, with shuffled staging 1.31.
 struct PolarRunBody {
     static constexpr int kRecMode = 4;
@@ -2172,7 +2176,7 @@ struct PolarRunBody {
 // its ends, so that runs of 32 neighbouring rows mostly stay within a bin.  Fully sampled apertures are at 0.006 (9.6 GHz,
 // 0.83 m bins); coarser angle steps and longer waves go pixel by pixel.  256 pulses onto 720 x 512, rows of 0.72 bins,
 // changes of 0.011, 0.016 and 0.021 bins: runs 181, 204 and 217 us, pixels 200, 212 and 211; rows of a bin: 160 (0.011)
-// and 167 (0.021), pixels 212 and 217.  Tiles too wide for the fast path: runs 1400 to 2050 us, pixels 990 to 1045
+// and 167 (0.021), pixels 212 and 217.  Tiles too wide for the fast path: runs 1400 to 2050 us, pixels 1020 to 1070
 // (890 to 940 in split_polar_kernel, which has their code alone).
 constexpr float kRunSpread = 0.02f;
 __device__ __forceinline__ bool polar_in_runs(const SplitParams& P, const Job& J, TileShared& S) {
