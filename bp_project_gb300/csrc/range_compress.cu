@@ -330,10 +330,16 @@ __device__ __forceinline__ void sum_into(float& s, float& e, float v, float ve) 
     s = t;
 }
 
+// (s + e) / n, rounded once (but for ties); inv: 1 / n.
+__device__ __forceinline__ float mean_of(float s, float e, float n, float inv) {
+    const float q = s * inv;
+    return fmaf(fmaf(-q, n, s) + e, inv, q);
+}
+
 // out[p, k] = sum_m h[m] (x - mean x)[k + taps - 1 - taps / 2 - m]; response: the taps' transform of
-// kBlockFft points divided by kBlockFft.
+// kBlockFft points divided by kBlockFft; inv: 1 / samples.
 __global__ void __launch_bounds__(kBlockThreads, 2) rc_blocks_kernel(const float2* __restrict__ raw, int pulses,
-                                                                     int samples, int taps,
+                                                                     int samples, int taps, float inv,
                                                                      const float2* __restrict__ response,
                                                                      float2* __restrict__ out) {
     extern __shared__ __align__(16) float2 sm[];
@@ -392,7 +398,10 @@ __global__ void __launch_bounds__(kBlockThreads, 2) rc_blocks_kernel(const float
             sum_into(sr, er, v.x, v.y);
             sum_into(si, ei, v.z, v.w);
         }
-        const float mr = (sr + er) / (float)samples, mi = (si + ei) / (float)samples;  // complex64, as the reference
+        // complex64, as the reference: the two-float sums divided with the remainder (a sum rounded first would
+        // put every second mean of a large offset a last bit off).
+        const float count = (float)samples;
+        const float mr = mean_of(sr, er, count, inv), mi = mean_of(si, ei, count, inv);
         for (int b = group; b < nblocks; b += kBlockGroups) {
             const int k0 = b * step, first = k0 - taps / 2;  // the block's first output and input sample
             float2 v[16];
@@ -499,8 +508,8 @@ int launch_rc_blocks(const float2* raw, int pulses, int samples, int taps, const
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rc_blocks_kernel, kBlockThreads, smem);
     if (e != cudaSuccess || per_sm < 1) return fail(SARBP_ERR_CUDA, "rc_blocks: %s", cudaGetErrorString(e));
     const long long slots = (long long)sms * per_sm;
-    rc_blocks_kernel<<<(int)(pulses < slots ? pulses : slots), kBlockThreads, smem, s>>>(raw, pulses, samples, taps,
-                                                                                        response, out);
+    rc_blocks_kernel<<<(int)(pulses < slots ? pulses : slots), kBlockThreads, smem, s>>>(
+        raw, pulses, samples, taps, 1.0f / (float)samples, response, out);
     note_launches(1);
     return check_launch("rc_blocks");
 }
