@@ -128,10 +128,12 @@ __device__ __forceinline__ bool fast_bin(double x, double step, double inv, int 
     const int lo = __double2loint(m);
     i = (__double2hiint(m) & 0x000fffff) - 0x80000;
     s = (float)(lo ^ INT_MIN) * 2.3283064365386963e-10f;
-    const int whole = i + (lo < 0);  // the nearest bin
-    const bool end = (unsigned)lo + 2u <= 4u && (whole == 1 || whole == n - 2);
-    if ((__double2hiint(m) >> 20) == 0x413 && i < 0x7fff0 && !end)
-        return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
+    // Two integer tests on the ordinary path: the exponent and size of the place, and whether it is at a whole bin.
+    if ((__double2hiint(m) >> 20) == 0x413 && i < 0x7fff0) {
+        if ((unsigned)lo + 2u > 4u) return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
+        const int whole = i + (lo < 0);
+        if (whole != 1 && whole != n - 2) return (unsigned)(i - 1) <= (unsigned)(n - 4) && n >= 4;
+    }
     const double q = x / step;
     if (!(q >= 1.0 && q < (double)(n - 2))) return false;  // or no number
     i = (int)floor(q);
