@@ -69,3 +69,23 @@ def test_compact_lists_are_taken_as_they_are(lib, n):
                                         nat.MODE_IDS["split"], 1, core._ptr(plain), None, 0,
                                         core.stream_handle()) == nat.SARBP_OK
     assert torch.equal(out, plain)
+
+
+def test_wide_lists_at_a_far_range_are_ordered(lib):
+    """At 30 km tiles of 33 m radius fit the fast path; ordered, they are compact, and the image is closer to FP64."""
+    from bp_project_gb300 import _native as nat
+    from bp_project_gb300 import core
+    from oracle import reference as ora
+    n = 68 * 266
+    i, j = np.divmod(np.arange(n), 266)
+    xyz = np.column_stack([3.0e4 + 0.25 * i, 0.25 * j, np.zeros(n)])
+    arrays, radar = scene(xyz, 12)
+    data, pos, w, ph = arrays
+    _, ref = ora.backproject_points(data, pos, xyz, *radar, w, ph, c128=True)
+    args = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (*arrays, xyz)]
+    out = core.backproject_points(*args, *radar, pulse_split=1)
+    plain = torch.empty_like(out)
+    assert lib.sarbp_backproject_points(core._ptr(args[0]), *data.shape, *(core._ptr(a) for a in args[1:]), n, *radar,
+                                        nat.MODE_IDS["split"], 1, core._ptr(plain), None, 0,
+                                        core.stream_handle()) == nat.SARBP_OK
+    assert rel_err(ref, out.cpu().numpy()) < rel_err(ref, plain.cpu().numpy()) <= 1e-5
