@@ -95,7 +95,7 @@ int allow_shared(const void* kernel, size_t smem) {
     if (e != cudaSuccess) return fail(SARBP_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (smem > (size_t)limit)
         return fail(SARBP_ERR_CUDA, "%zu bytes of shared memory are more than a block can have", smem);
-    if (slot) {
+    if (slot && id) {
         slot->limit.store((size_t)limit, std::memory_order_relaxed);
         slot->context.store(id, std::memory_order_release);
     }
