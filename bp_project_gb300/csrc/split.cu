@@ -2881,16 +2881,18 @@ __device__ __forceinline__ void leaf_tile(const SplitParams& P, const PolarDesc*
     float4* win = reinterpret_cast<float4*>(smem + leaf_window_offset());
     const PulseInputs& in = P.in;
     const float side = (float)g.side;
-    __syncthreads();  // a persistent block's last tile may still read its runs' middles
-    if (part == 0 && lane == 0 && row == 0) {
-        const float4 pd = precs[g.a].d;
-        mids[group] = leaf_mid(P, g, jpix, r_min, pd.z, pd.w);
-        mids[group].first = I_first;
-        if (it.tile_u + kLeafRun * group >= g.win_nu) mids[group].runs = 1;  // past the window: nothing to be exact about
-    }
     for (int c0 = g.a; c0 < g.b;) {
         const int want = min(P.chunk, g.b - c0);
-        __syncthreads();
+        __syncthreads();  // the last chunk's windows are consumed (and a persistent block's last tile's middles)
+        // The runs' middles, one per lane of the second warp, while the first makes the first chunk's records.
+        if (c0 == g.a && warp == 1 && lane < groups) {
+            const float4 pd = precs[g.a].d;
+            const int j = it.tile_u + kLeafRun * lane;
+            LeafMid M = leaf_mid(P, g, g.win_u0 + j, r_min, pd.z, pd.w);
+            if (j >= g.win_nu) M.runs = 1;  // past the window: nothing to be exact about
+            M.first = I_first;
+            mids[lane] = M;
+        }
         if (warp == 0) {
             int count = 0;
             if (lane < want) {
